@@ -98,7 +98,8 @@ typedef struct pt_stats {
   int bvh_depth;           /* depth of the BVH8 */
   double build_ms;         /* last pt_commit, host wall time */
   double render_ms;        /* last pt_render, device time */
-  uint64_t iterations;     /* wavefront iterations of the last render */
+  uint64_t iterations;     /* wavefront iterations of the last render, the pass over
+                              each chunk's last paths included */
   uint64_t kernel_launches;/* kernels launched by the last render */
   /* device time per stage (enable_timing): generate, trace, shade,
      shadow trace, finish + queue advance */

@@ -237,7 +237,6 @@ PT_API int pt_context_create(const pt_options* opt, pt_context** out) {
   if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_ctr, 2 * sizeof(WaveCounters));
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->evc[0], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->evc[1], cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_ctl, sizeof(WaveCtl));
   if (e != cudaSuccess) {
     int rc = (e == cudaErrorMemoryAllocation) ? PT_ENOMEM : PT_ECUDA;
     delete ctx;
@@ -304,7 +303,6 @@ PT_API int pt_context_destroy(pt_context* ctx) {
   ctx->d_tmp.release();
   ctx->d_tmpu.release();
   if (ctx->h_ctr) cudaFreeHost(ctx->h_ctr);
-  if (ctx->h_ctl) cudaFreeHost(ctx->h_ctl);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -1018,6 +1016,8 @@ PT_API int pt_commit(pt_context* ctx) {
   ctx->lc.refetch = ctx->opt.refetch_lanes ? ctx->opt.refetch_lanes : pth::auto_refetch(n);
   ctx->lc.tex = pth::uses_textures(ctx) ? 1 : 0;
   ctx->lc.motion = pth::has_motion(ctx) ? 1 : 0;
+  ctx->lc.lights = ctx->lights.empty() ? 0 : 1;
+  ctx->lc.env = ctx->env_valid ? 1 : 0;
   auto t1 = std::chrono::steady_clock::now();
   ctx->stats.build_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
   ctx->stats.bvh_nodes = nn;
@@ -1090,9 +1090,10 @@ static int ensure_wave(pt_context* ctx, size_t results_needed) {
 
 static const int kItersPerGraph = 8;
 
-static int run_chunk(pt_context* ctx, const pt_render_params* p, int frame0, int frames) {
-  cudaStream_t st = ctx->stream;
-  WaveCtl& ctl = *ctx->h_ctl;
+// Controls of a chunk of `frames` frames from frame0.
+static WaveCtl chunk_ctl(const pt_context* ctx, const pt_render_params* p, int frame0, int frames) {
+  WaveCtl ctl;
+  memset(&ctl, 0, sizeof(ctl));
   ctl.width = p->width;
   ctl.height = p->height;
   ctl.frame0 = frame0;
@@ -1102,55 +1103,86 @@ static int run_chunk(pt_context* ctx, const pt_render_params* p, int frame0, int
   ctl.mode = p->mode;
   ctl.guide = p->guide;
   ctl.guide_depth = ctx->guide.max_bounces > 0 ? (uint32_t)ctx->guide.max_bounces : 0xffffffffu;
+  ctl.tail_max = pt::tail_paths(ctx->max_stack);
   ctl.chunk_paths = (unsigned long long)p->width * p->height * frames;
   fastdiv_magic((uint32_t)(p->width * p->height), &ctl.wh_m, &ctl.wh_l);
   fastdiv_magic((uint32_t)p->width, &ctl.w_m, &ctl.w_l);
-  CK(cudaMemcpyAsync(ctx->d_ctl.p, &ctl, sizeof(WaveCtl), cudaMemcpyHostToDevice, st));
-  WaveCounters& c = *ctx->h_ctr;
-  memset(&c, 0, sizeof(c));
-  CK(cudaMemcpyAsync(ctx->d_ctr.p, &c, sizeof(WaveCounters), cudaMemcpyHostToDevice, st));
-  bool counters = ctx->opt.enable_counters != 0;
-  bool timing = ctx->opt.enable_timing != 0;
-  if (timing && ctx->tev.empty()) {
-    ctx->tev.resize(2 * 6 * kItersPerGraph);  // a set for each graph instance
-    for (auto& e : ctx->tev) CK(cudaEventCreate(&e));
-  }
-  const bool guide = p->guide != 0;
-  GuideInferArgs gi;
-  if (guide) gi = guide_infer_args(ctx);
-  if (!ctx->graph || ctx->graph_counters != counters || ctx->graph_timing != timing ||
-      ctx->graph_mode != p->mode || ctx->graph_guide != guide ||
-      memcmp(&ctx->graph_W, &ctx->W, sizeof(WaveState)) != 0) {
-    drop_graphs(ctx);
-    // with timing, a second instance records on its own events, so one
-    // launch can run while the host reads the other's times
-    for (int inst = 0; inst < (timing ? 2 : 1); inst++) {
-      cudaGraph_t g;
-      CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      for (int i = 0; i < kItersPerGraph; i++)
-        pt::launch_iteration(ctx->scene, ctx->W, ctx->d_ctl.p, ctx->max_stack, counters, ctx->lc,
-                             st, timing ? &ctx->tev[6 * (kItersPerGraph * inst + i)] : nullptr,
-                             p->mode, nullptr, false, 0, guide ? &gi : nullptr);
-      cudaError_t ce = cudaStreamEndCapture(st, &g);
-      if (ce != cudaSuccess) return cuda_fail(ctx, ce, "cudaStreamEndCapture");
-      cudaError_t e = cudaGraphInstantiate(inst ? &ctx->graph2 : &ctx->graph, g, 0);
-      cudaGraphDestroy(g);
-      if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaGraphInstantiate");
+  return ctl;
+}
+
+// The chunk's iterations as one graph launch: a conditional (while) node whose
+// body is one iteration; k_advance decides on the device whether it goes on
+// (bounded by WaveCtl.max_iter).
+static cudaError_t capture_loop(pt_context* ctx, int mode, bool counters, const GuideInferArgs* gi,
+                                cudaGraphExec_t* out) {
+  cudaStream_t st = ctx->stream;
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaGraphCreate(&g, 0);
+  if (e != cudaSuccess) return e;
+  cudaGraphConditionalHandle h = 0;
+  e = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault);
+  cudaGraphNodeParams np = {};
+  np.type = cudaGraphNodeTypeConditional;
+  np.conditional.handle = h;
+  np.conditional.type = cudaGraphCondTypeWhile;
+  np.conditional.size = 1;
+  cudaGraphNode_t node;
+  if (e == cudaSuccess) e = cudaGraphAddNode(&node, g, nullptr, nullptr, 0, &np);
+  if (e == cudaSuccess) {
+    cudaGraph_t body = np.conditional.phGraph_out[0];
+    e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
+                                      cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      pt::launch_iteration(ctx->scene, ctx->W, ctx->d_ctl.p, ctx->max_stack, counters, ctx->lc, st,
+                           nullptr, mode, nullptr, true, h, gi);
+      e = cudaStreamEndCapture(st, &body);
     }
-    ctx->graph_counters = counters;
-    ctx->graph_timing = timing;
-    ctx->graph_mode = p->mode;
-    ctx->graph_guide = guide;
-    ctx->graph_W = ctx->W;
   }
-  // bounded host loop: a path needs at most max_depth iterations after its
-  // generation, and every iteration generates at least one path while any
-  // remain, so this many iterations always suffice.  The loop keeps one graph
-  // launch queued ahead of the one whose counters it reads (slot 0 / 1:
-  // counters, completion event and, with timing, graph instance and events),
-  // so the GPU does not wait for the host between launches; the launch queued
-  // after the chunk drained runs empty iterations.
-  unsigned long long max_iters = ctl.chunk_paths + (unsigned long long)p->max_depth + 16;
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *out = nullptr;
+  }
+  return e;
+}
+
+// kItersPerGraph iterations and the tail kernel, for the host loop; inst: the
+// events of instance 0 or 1 (timing).
+static cudaError_t capture_iterations(pt_context* ctx, int mode, bool counters, bool timing,
+                                      int inst, const GuideInferArgs* gi, cudaGraphExec_t* out) {
+  cudaStream_t st = ctx->stream;
+  cudaGraph_t g = nullptr;
+  cudaEvent_t* ev = timing ? &ctx->tev[(6 * kItersPerGraph + 1) * inst] : nullptr;
+  cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return e;
+  for (int i = 0; i < kItersPerGraph; i++)
+    pt::launch_iteration(ctx->scene, ctx->W, ctx->d_ctl.p, ctx->max_stack, counters, ctx->lc, st,
+                         ev ? ev + 6 * i : nullptr, mode, nullptr, false, 0, gi);
+  pt::launch_tail(ctx->scene, ctx->W, ctx->d_ctl.p, ctx->max_stack, counters, ctx->lc, mode,
+                  nullptr, true, st);
+  if (ev) cudaEventRecordWithFlags(ev[6 * kItersPerGraph], st, cudaEventRecordExternal);
+  e = cudaStreamEndCapture(st, &g);
+  if (e != cudaSuccess) return e;
+  e = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  return e;
+}
+
+// The host loop of a chunk: a graph of kItersPerGraph iterations and the tail
+// kernel, launched until the counters say that the chunk has drained.  Used
+// with per-stage timing (events cannot sit in a conditional body) and where
+// the runtime refuses conditional nodes.  One graph launch is kept queued
+// ahead of the one whose counters the host reads (slot 0 / 1: counters,
+// completion event and, with timing, graph instance and events), so the GPU
+// does not wait for the host; the launch queued after the chunk drained runs
+// empty iterations.  Bounded: a path needs at most max_depth iterations after
+// its generation, and every iteration generates at least one path while any
+// remain.
+static int host_loop(pt_context* ctx, const WaveCtl& ctl, bool timing, int iter_kernels) {
+  cudaStream_t st = ctx->stream;
+  const unsigned long long max_iters = ctl.chunk_paths + (unsigned long long)ctl.max_depth + 16;
   unsigned long long iters = 0;
   auto launch = [&](int slot) -> cudaError_t {
     cudaError_t e = cudaGraphLaunch(timing && slot ? ctx->graph2 : ctx->graph, st);
@@ -1164,18 +1196,19 @@ static int run_chunk(pt_context* ctx, const pt_render_params* p, int frame0, int
   };
   auto harvest = [&](int slot) -> cudaError_t {
     cudaError_t e = cudaEventSynchronize(ctx->evc[slot]);
-    ctx->stats.iterations += kItersPerGraph;
-    ctx->stats.kernel_launches += 7 * kItersPerGraph;
+    ctx->stats.kernel_launches += iter_kernels * kItersPerGraph + 2;
     if (timing && e == cudaSuccess) {
-      const cudaEvent_t* ev = &ctx->tev[6 * kItersPerGraph * slot];
+      const cudaEvent_t* ev = &ctx->tev[(6 * kItersPerGraph + 1) * slot];
+      auto add = [&](int a, int b, int k) {
+        float ms = 0.f;
+        if (cudaEventElapsedTime(&ms, ev[a], ev[b]) == cudaSuccess)
+          ctx->stats.stage_ms[k] += ms;
+        else
+          cudaGetLastError();  // a missing sample is not an error of the render
+      };
       for (int i = 0; i < kItersPerGraph; i++)
-        for (int k = 0; k < 5; k++) {
-          float ms = 0.f;
-          if (cudaEventElapsedTime(&ms, ev[6 * i + k], ev[6 * i + k + 1]) == cudaSuccess)
-            ctx->stats.stage_ms[k] += ms;
-          else
-            cudaGetLastError();  // a missing sample is not an error of the render
-        }
+        for (int k = 0; k < 5; k++) add(6 * i + k, 6 * i + k + 1, k);
+      add(6 * kItersPerGraph - 1, 6 * kItersPerGraph, 4);  // the tail kernel
     }
     return e;
   };
@@ -1185,14 +1218,9 @@ static int run_chunk(pt_context* ctx, const pt_render_params* p, int frame0, int
     CK(launch(cur ^ 1));
     CK(harvest(cur));
     const WaveCounters& cc = ctx->h_ctr[cur];
-    if (cc.error) {
-      CK(cudaStreamSynchronize(st));
-      return fail(ctx, PT_EQUEUE, "traversal stack overflow");
-    }
-    if (cc.next_path >= ctl.chunk_paths && cc.n_cur == 0) {
+    if (cc.error || (cc.next_path >= ctl.chunk_paths && cc.n_cur == 0)) {
       CK(harvest(cur ^ 1));
-      c = ctx->h_ctr[cur ^ 1];
-      break;
+      return PT_OK;  // render_done looks at the error flags
     }
     if (iters > max_iters) {
       CK(cudaStreamSynchronize(st));
@@ -1200,11 +1228,90 @@ static int run_chunk(pt_context* ctx, const pt_render_params* p, int frame0, int
     }
     cur ^= 1;
   }
+}
+
+// Queues one chunk of frames on the context's stream (with per-stage timing
+// it also waits for them).  first: the render's first chunk.
+static int run_chunk(pt_context* ctx, const pt_render_params* p, int frame0, int frames,
+                     bool first) {
+  cudaStream_t st = ctx->stream;
+  WaveCtl ctl = chunk_ctl(ctx, p, frame0, frames);
+  const unsigned long long slots = (unsigned long long)ctx->slots;
+  ctl.max_iter =
+      ((ctl.chunk_paths + slots - 1) / slots + 2) * (unsigned long long)(p->max_depth + 1) + 16;
+  const bool counters = ctx->opt.enable_counters != 0;
+  const bool timing = ctx->opt.enable_timing != 0;
+  const bool guide = p->guide != 0;
+  const int iter_kernels = pt::iteration_kernels(ctx->lc, p->mode, guide);
+  pt::launch_chunk_begin(ctx->W, ctx->d_ctl.p, ctl, first, st);
   ctx->stats.paths += ctl.chunk_paths;
-  ctx->stats.ext_rays += c.ext_rays;
-  ctx->stats.shadow_rays += c.shadow_rays;
-  ctx->stats.node_fetches += c.node_fetches;
-  ctx->stats.prim_tests += c.prim_tests;
+  ctx->stats.iterations += 1;  // the tail pass; render_done adds the wavefront's
+  ctx->stats.kernel_launches += 1;
+  if (!guide && !timing && ctl.chunk_paths <= ctl.tail_max) {
+    // a chunk this small needs no wavefront
+    pt::launch_tail(ctx->scene, ctx->W, ctx->d_ctl.p, ctx->max_stack, counters, ctx->lc, p->mode,
+                    nullptr, false, st);
+    CK(cudaGetLastError());
+    ctx->stats.kernel_launches += 1;
+    return PT_OK;
+  }
+  if (timing && ctx->tev.empty()) {
+    ctx->tev.resize(2 * (6 * kItersPerGraph + 1));  // a set for each graph instance
+    for (auto& e : ctx->tev) CK(cudaEventCreate(&e));
+  }
+  GuideInferArgs gi;
+  if (guide) gi = guide_infer_args(ctx);
+  const GuideInferArgs* gp = guide ? &gi : nullptr;
+  if (!ctx->graph || ctx->graph_counters != counters || ctx->graph_timing != timing ||
+      ctx->graph_mode != p->mode || ctx->graph_guide != guide ||
+      memcmp(&ctx->graph_W, &ctx->W, sizeof(WaveState)) != 0) {
+    drop_graphs(ctx);
+    ctx->graph_loop = false;
+    if (!timing && ctx->cond_ok) {
+      ctx->graph_loop = capture_loop(ctx, p->mode, counters, gp, &ctx->graph) == cudaSuccess;
+      ctx->cond_ok = ctx->graph_loop;  // else the host loop does the same work
+    }
+    if (!ctx->graph_loop) {
+      CK(capture_iterations(ctx, p->mode, counters, timing, 0, gp, &ctx->graph));
+      // a second instance records on its own events, so one launch can run
+      // while the host reads the other's times
+      if (timing) CK(capture_iterations(ctx, p->mode, counters, timing, 1, gp, &ctx->graph2));
+    }
+    ctx->graph_counters = counters;
+    ctx->graph_timing = timing;
+    ctx->graph_mode = p->mode;
+    ctx->graph_guide = guide;
+    ctx->graph_W = ctx->W;
+  }
+  if (!ctx->graph_loop) return host_loop(ctx, ctl, timing, iter_kernels);
+  CK(cudaGraphLaunch(ctx->graph, st));
+  pt::launch_tail(ctx->scene, ctx->W, ctx->d_ctl.p, ctx->max_stack, counters, ctx->lc, p->mode,
+                  nullptr, false, st);
+  CK(cudaGetLastError());
+  ctx->stats.graph_launches++;
+  ctx->stats.kernel_launches += 1;
+  return PT_OK;
+}
+
+// Queues the read-back of the counters behind the render's chunks.
+static cudaError_t queue_counters(pt_context* ctx) {
+  return cudaMemcpyAsync(ctx->h_ctr, ctx->d_ctr.p, sizeof(WaveCounters), cudaMemcpyDeviceToHost,
+                         ctx->stream);
+}
+
+// After the render's stream is idle: the error flags and the statistics.
+static int render_done(pt_context* ctx, const pt_render_params* p) {
+  const WaveCounters& c = *ctx->h_ctr;
+  if (c.error & 1u) return fail(ctx, PT_EQUEUE, "traversal stack overflow");
+  if (c.error) return fail(ctx, PT_ETIMEOUT, "wavefront did not drain");
+  ctx->stats.ext_rays = c.ext_rays;
+  ctx->stats.shadow_rays = c.shadow_rays;
+  ctx->stats.node_fetches = c.node_fetches;
+  ctx->stats.prim_tests = c.prim_tests;
+  ctx->stats.iterations += c.iters_total;  // beside each chunk's tail pass
+  if (ctx->graph_loop)
+    ctx->stats.kernel_launches +=
+        c.iters_total * (uint64_t)pt::iteration_kernels(ctx->lc, p->mode, p->guide != 0);
   return PT_OK;
 }
 
@@ -1285,7 +1392,7 @@ static int render_device(pt_context* ctx, const pt_render_params* p, void* d_acc
       ctx->W.grec_stride = ctx->guide.rec_stride;
       ctx->W.grec_n = ctx->guide.rec_n;
     }
-    rc = run_chunk(ctx, p, p->frame0 + f, frames);
+    rc = run_chunk(ctx, p, p->frame0 + f, frames, f == 0);
     if (rc) return rc;
     if (p->guide) {
       rc = guide_frame_train(ctx);
@@ -1297,6 +1404,7 @@ static int render_device(pt_context* ctx, const pt_render_params* p, void* d_acc
       pt::launch_accumulate(ctx->d_results.p, (float4*)d_acc, p->width, p->height, frames, st);
     ctx->stats.kernel_launches += 1;
   }
+  CK(queue_counters(ctx));
   if (p->guide) {
     uint32_t fl[4];
     CK(cudaMemcpyAsync(fl, ctx->guide.counters.p, 16, cudaMemcpyDeviceToHost, st));
@@ -1333,10 +1441,14 @@ PT_API int pt_render(pt_context* ctx, const pt_render_params* params, float* acc
   }
   CK(cudaEventRecord(ctx->ev0, st));
   rc = render_device(ctx, params, d_acc);
-  if (rc) return rc;
+  if (rc) {
+    cudaStreamSynchronize(st);  // queued work may still write the accumulator
+    return rc;
+  }
   CK(cudaEventRecord(ctx->ev1, st));
   if (!dev) CK(cudaMemcpyAsync(accum_rgba, d_acc, WH * sizeof(float4), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if ((rc = render_done(ctx, params)) != PT_OK) return rc;
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   ctx->stats.render_ms = ms;
@@ -1369,10 +1481,14 @@ PT_API int pt_render_accum64(pt_context* ctx, const pt_render_params* params,
   }
   CK(cudaEventRecord(ctx->ev0, st));
   rc = render_device(ctx, params, d_acc, true);
-  if (rc) return rc;
+  if (rc) {
+    cudaStreamSynchronize(st);  // queued work may still write the accumulator
+    return rc;
+  }
   CK(cudaEventRecord(ctx->ev1, st));
   if (!dev) CK(cudaMemcpyAsync(accum_rgba, d_acc, WH * 32, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if ((rc = render_done(ctx, params)) != PT_OK) return rc;
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   ctx->stats.render_ms = ms;
@@ -1399,8 +1515,12 @@ PT_API int pt_render_paths(pt_context* ctx, const pt_render_params* params, floa
   rc = ensure_wave(ctx, WH);
   if (rc) return rc;
   p.frame0 = params->frame0;
-  rc = run_chunk(ctx, &p, p.frame0, 1);
-  if (rc) return rc;
+  rc = run_chunk(ctx, &p, p.frame0, 1, true);
+  if (rc) {
+    cudaStreamSynchronize(st);
+    return rc;
+  }
+  CK(queue_counters(ctx));
   int kind = device_ptr_kind(out_rgb, ctx->device);
   if (kind < 0) return fail(ctx, PT_EINVAL, kOtherDevice);
   bool dev = kind > 0;
@@ -1412,7 +1532,7 @@ PT_API int pt_render_paths(pt_context* ctx, const pt_render_params* params, floa
   pt::launch_paths_out(ctx->d_results.p, d_out, (uint32_t)WH, st);
   if (!dev) CK(cudaMemcpyAsync(out_rgb, d_out, 3 * WH * sizeof(float), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  return PT_OK;
+  return render_done(ctx, &p);
 }
 
 PT_API int pt_trace_first_hits(pt_context* ctx, int width, int height, int frame, uint32_t* prim,
@@ -1570,34 +1690,24 @@ extern "C" PT_API int pt_render_noalloc(pt_context* ctx, const pt_render_params*
   float4* acc = (float4*)accum_rgba;
   if (p->frame0 == 0) CK(cudaMemsetAsync(acc, 0, WH * sizeof(float4), st));
   int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)p->spp, kNoAllocMaxPixels / WH));
-  WaveCounters& c = *ctx->h_ctr;
-  WaveCtl& ctl = *ctx->h_ctl;
+  const WaveCounters& c = *ctx->h_ctr;
+  const uint64_t iter_kernels = (uint64_t)pt::iteration_kernels(ctx->lc, p->mode, false);
   for (int f = 0; f < p->spp; f += chunk) {
     int frames = std::min(chunk, p->spp - f);
-    ctl.width = p->width;
-    ctl.height = p->height;
-    ctl.frame0 = p->frame0 + f;
-    ctl.max_depth = p->max_depth;
-    ctl.rr_enable = p->rr_enable;
-    ctl.rr_depth = p->rr_depth;
-    ctl.mode = p->mode;
-    ctl.guide = p->guide;
-    ctl.chunk_paths = (unsigned long long)WH * frames;
-    fastdiv_magic((uint32_t)WH, &ctl.wh_m, &ctl.wh_l);
-    fastdiv_magic((uint32_t)p->width, &ctl.w_m, &ctl.w_l);
-    CK(cudaMemcpyAsync(d_ctl, &ctl, sizeof(WaveCtl), cudaMemcpyHostToDevice, st));
-    memset(&c, 0, sizeof(c));  // no live path; the counters start at zero
-    CK(cudaMemcpyAsync(W.ctr, &c, sizeof(WaveCounters), cudaMemcpyHostToDevice, st));
+    const WaveCtl ctl = chunk_ctl(ctx, p, p->frame0 + f, frames);
+    pt::launch_chunk_begin(W, d_ctl, ctl, f == 0, st);
     unsigned long long max_iters = ctl.chunk_paths + (unsigned long long)p->max_depth + 16;
     unsigned long long iters = 0;
     while (true) {
-      for (int i = 0; i < kItersPerGraph; i++)
+      const int n = ctl.chunk_paths <= ctl.tail_max ? 0 : kItersPerGraph;
+      for (int i = 0; i < n; i++)
         pt::launch_iteration(ctx->scene, W, d_ctl, ctx->max_stack, false, ctx->lc, st, nullptr,
                              p->mode, nullptr, false, 0);
+      pt::launch_tail(ctx->scene, W, d_ctl, ctx->max_stack, false, ctx->lc, p->mode, nullptr, true,
+                      st);
       CK(cudaGetLastError());
       iters += kItersPerGraph;
-      ctx->stats.iterations += kItersPerGraph;
-      ctx->stats.kernel_launches += 7 * kItersPerGraph;
+      ctx->stats.kernel_launches += iter_kernels * n + 2;
       CK(cudaMemcpyAsync(ctx->h_ctr, W.ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
       if (c.error) return fail(ctx, PT_EQUEUE, "traversal stack overflow");
@@ -1605,11 +1715,13 @@ extern "C" PT_API int pt_render_noalloc(pt_context* ctx, const pt_render_params*
       if (iters > max_iters) return fail(ctx, PT_ETIMEOUT, "wavefront did not drain");
     }
     ctx->stats.paths += ctl.chunk_paths;
-    ctx->stats.ext_rays += c.ext_rays;
-    ctx->stats.shadow_rays += c.shadow_rays;
+    ctx->stats.iterations += 1;
     pt::launch_accumulate(W.results, acc, p->width, p->height, frames, st);
-    ctx->stats.kernel_launches += 1;
+    ctx->stats.kernel_launches += 2;
   }
+  ctx->stats.ext_rays = c.ext_rays;
+  ctx->stats.shadow_rays = c.shadow_rays;
+  ctx->stats.iterations += c.iters_total;
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev1, st));
   CK(cudaStreamWaitEvent((cudaStream_t)stream, ctx->ev1, 0));

@@ -13,8 +13,9 @@
  *
  *   while (a chunk is left)             conditional node, set on the device
  *     k_batch_begin                     load the chunk, reset the queues
- *     while (the chunk has paths left)  conditional node, set on the device
+ *     while (the chunk has many paths)  conditional node, set on the device
  *       generate, trace, shade, shadow trace, finish, advance
+ *     k_tail                            the last paths, each to its end
  *     k_accumulate_batch, k_batch_end
  *
  * Both loops are bounded on the device (by the chunk count, and per chunk by
@@ -341,6 +342,8 @@ static cudaError_t capture_loop_graph(pt_batch* b, const BatchRefs& br, bool cou
     if ((r = cudaStreamUpdateCaptureDependencies(st, &n_in, nullptr, 1,
                                                  cudaStreamSetCaptureDependencies)) != cudaSuccess)
       return r;
+    pt::launch_tail(b->merged, b->W, b->d_ctl.p, b->max_stack, counters, b->lc, mode, &br, false,
+                    st);
     pt::launch_batch_end(b->W, b->d_ctl.p, br, true, h_out, st);
     capturing = false;
     if ((r = cudaStreamEndCapture(st, &body_out)) != cudaSuccess) return r;
@@ -368,8 +371,8 @@ static cudaError_t capture_loop_graph(pt_batch* b, const BatchRefs& br, bool cou
   return e;
 }
 
-// The host-loop graph: kItersPerGraph iterations, events between stages
-// when timing.
+// The host-loop graph: kItersPerGraph iterations and the tail kernel, events
+// between stages when timing.
 static cudaError_t capture_iter_graph(pt_batch* b, const BatchRefs& br, bool counters, bool timing,
                                       int mode, cudaGraphExec_t* out) {
   cudaStream_t st = b->stream;
@@ -379,6 +382,8 @@ static cudaError_t capture_iter_graph(pt_batch* b, const BatchRefs& br, bool cou
   for (int i = 0; i < kItersPerGraph; i++)
     pt::launch_iteration(b->merged, b->W, b->d_ctl.p, b->max_stack, counters, b->lc, st,
                          timing ? &b->tev[6 * i] : nullptr, mode, &br, false, 0);
+  pt::launch_tail(b->merged, b->W, b->d_ctl.p, b->max_stack, counters, b->lc, mode, &br, true, st);
+  if (timing) cudaEventRecordWithFlags(b->tev[6 * kItersPerGraph], st, cudaEventRecordExternal);
   e = cudaStreamEndCapture(st, &g);
   if (e != cudaSuccess) return e;
   e = cudaGraphInstantiate(out, g, 0);
@@ -423,10 +428,14 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
     for (const ScenePart& p : b->parts) lc.sort = lc.sort || sort_pays(p.ctx);
   lc.tex = 0;
   lc.motion = 0;
+  lc.lights = lc.env = 0;
   for (const ScenePart& p : b->parts) {
     lc.tex = lc.tex || uses_textures(p.ctx);
     lc.motion = lc.motion || has_motion(p.ctx);
+    lc.lights = lc.lights || p.ctx->scene.num_lights > 0;
+    lc.env = lc.env || p.ctx->scene.env_valid;
   }
+  lc.tail_grid = pt::wave_grid(2, b->max_stack, PT_TAIL_BLOCK);
   lc.refetch = b->tune.refetch_lanes;
   if (lc.refetch == 0) {  // automatic: by the largest scene of the batch
     size_t most = 0;
@@ -559,10 +568,11 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
   WaveCtl hc;
   memset(&hc, 0, sizeof(hc));
   hc.mode = mode;
+  hc.tail_max = pt::tail_paths(b->max_stack);
   BK(cudaMemcpyAsync(b->d_ctl.p, &hc, sizeof(hc), cudaMemcpyHostToDevice, st));
   BatchRefs br{b->d_scenes.p, b->d_segs.p, b->d_roots.p};
   if (timing && b->tev.empty()) {
-    b->tev.resize(6 * kItersPerGraph);
+    b->tev.resize(6 * kItersPerGraph + 1);
     for (auto& e : b->tev) BK(cudaEventCreate(&e));
   }
   GraphSig sig;
@@ -603,18 +613,21 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
       while (true) {
         BK(cudaGraphLaunch(b->exec, st));
         s.graph_launches++;
+        s.kernel_launches += 2;
         iters += kItersPerGraph;
         BK(cudaMemcpyAsync(b->h_ctr, b->d_ctr.p, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st));
         BK(cudaStreamSynchronize(st));
         if (timing) {
+          auto add = [&](int a, int z, int q) {
+            float ms = 0.f;
+            if (cudaEventElapsedTime(&ms, b->tev[a], b->tev[z]) == cudaSuccess)
+              s.stage_ms[q] += ms;
+            else
+              cudaGetLastError();
+          };
           for (int i = 0; i < kItersPerGraph; i++)
-            for (int q = 0; q < 5; q++) {
-              float ms = 0.f;
-              if (cudaEventElapsedTime(&ms, b->tev[6 * i + q], b->tev[6 * i + q + 1]) == cudaSuccess)
-                s.stage_ms[q] += ms;
-              else
-                cudaGetLastError();
-            }
+            for (int q = 0; q < 5; q++) add(6 * i + q, 6 * i + q + 1, q);
+          add(6 * kItersPerGraph - 1, 6 * kItersPerGraph, 4);  // the tail kernel
         }
         if (c.error) break;
         if (c.next_path >= chunks[k].paths && c.n_cur == 0) break;
@@ -646,9 +659,10 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
   s.shadow_rays = c.shadow_rays;
   s.node_fetches = c.node_fetches;
   s.prim_tests = c.prim_tests;
-  s.iterations = c.iters_total;
-  if (sig.device_loop) s.kernel_launches = 7 * c.iters_total + 3 * chunks.size();
-  else s.kernel_launches += 7 * c.iters_total;
+  s.iterations = c.iters_total + chunks.size();  // and each chunk's tail pass
+  const uint64_t iter_kernels = (uint64_t)pt::iteration_kernels(b->lc, mode, false);
+  if (sig.device_loop) s.kernel_launches = iter_kernels * c.iters_total + 4 * chunks.size();
+  else s.kernel_launches += iter_kernels * c.iters_total;
   s.bvh_nodes = b->total_nodes;
   s.bvh_bytes = b->total_nodes * 80 + (size_t)b->merged.num_prims * 48;
   s.bvh_depth = b->max_stack - 1;

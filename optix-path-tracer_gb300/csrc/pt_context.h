@@ -165,16 +165,17 @@ struct pt_context {
   DevBuf<float> d_tmp;
   DevBuf<uint32_t> d_tmpu;
   WaveCounters* h_ctr = nullptr;  // pinned, 2 (the counters after each of two graph launches)
-  WaveCtl* h_ctl = nullptr;       // pinned
   cudaGraphExec_t graph = nullptr;
   cudaGraphExec_t graph2 = nullptr;  // a second instance on its own timing events (timing)
+  bool graph_loop = false;   // graph is the device loop (else iterations for the host loop)
+  bool cond_ok = true;       // conditional graph nodes usable
   cudaEvent_t evc[2] = {nullptr, nullptr};  // the counters of a graph launch have arrived
   bool graph_counters = false;
   bool graph_timing = false;
   int graph_mode = 0;
   WaveState graph_W{};       // the buffers the captured graph refers to
   bool graph_guide = false;
-  std::vector<cudaEvent_t> tev;  // 6 per iteration of the graph (timing)
+  std::vector<cudaEvent_t> tev;  // timing: per graph instance 6 per iteration and 1
   int max_stack = 0;
   LaunchCfg lc{};
   GuideState guide;

@@ -32,6 +32,17 @@
 #define PT_SHADE_G_MINBLOCKS PT_SHADE_MINBLOCKS
 #endif
 
+#define PT_TAIL_BLOCK 128        /* threads per block of the tail kernel */
+/* Paths left in a chunk (live and not generated) that the tail kernel takes
+ * over from the wavefront.  GB300, us per render with 0 (wavefront only) /
+ * 8192 / 16384 / 32768 / 131072: Cornell box 500x500 1121 / 657 / 646 / 665 /
+ * 805, 2.1 M camera paths on the spheres 2941 / 2025 / 2026 / 2014 / 2062,
+ * terrain 1280x720 1481 / 1214 / 1124 / 1126 / 1129, textures (33 frames of
+ * 321x243) 3510 / 3474 / 3524 / 3731 / 4519. */
+#ifndef PT_TAIL_PATHS
+#define PT_TAIL_PATHS 16384
+#endif
+
 /* Path state word st.z: depth (bits 0-15), previous bounce specular (bit 16),
  * scene of a batch (bits 17-31). */
 #define PT_ST_DEPTH_MASK 0xffffu
@@ -48,6 +59,9 @@ struct LaunchCfg {
   int refetch;         /* idle lanes of a trace warp that take new rays together (1..32) */
   int tex;             /* some material takes a texture: the texture variants of shading */
   int motion;          /* some sphere moves: the trace variants that carry ray times */
+  int tail_grid;       /* blocks of the tail kernel: those resident at once */
+  int lights;          /* some scene has lights */
+  int env;             /* some scene has an importance-sampled environment */
 };
 
 struct Ray3 {
@@ -70,6 +84,8 @@ struct WaveCounters {
   uint32_t n_chunks;     /* chunks of the batch (set by the host) */
   uint32_t ray_next[2];  /* rays taken by trace warps this iteration (extension, shadow) */
   uint32_t guide_rows;   /* positions listed for guide inference this iteration */
+  uint32_t drained;      /* iterations since the chunk's last path was generated, that one
+                            included: every live path has bounced this often */
 };
 
 /* Per-chunk render controls, in device memory (kernels read them, so one
@@ -83,6 +99,7 @@ struct WaveCtl {
   /* batch: segments [seg_begin, seg_end) make up this chunk, `pixels` pixels */
   uint32_t seg_begin, seg_end, pixels;
   uint32_t guide_depth;           /* guided bounces: depth < guide_depth */
+  uint32_t tail_max;              /* most paths left that the tail kernel takes over */
   unsigned long long max_iter;    /* device-side iteration bound of this chunk */
 };
 
@@ -192,15 +209,32 @@ int trace_blocks_per_sm(int block, size_t smem);
 void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W,
                   const WaveCtl* ctl, int max_stack, const BatchRefs* br, const LaunchCfg& lc,
                   cudaStream_t st);
-/* Resident blocks per SM x SMs for a trace (kind 0) or shade (kind 1)
- * kernel of `block` threads. */
+/* WaveCtl.tail_max for a BVH of this stack depth: PT_TAIL_PATHS, or 0 where
+ * the tail kernel's stacks would not fit in shared memory. */
+uint32_t tail_paths(int max_stack);
+/* Resident tail blocks per SM (pt_tail.cu). */
+int tail_blocks_per_sm(int max_stack);
+/* The chunk's last paths, each to its end, when at most tail_max are left
+ * (pt_tail.cu); mark: the counters then say that the chunk has drained. */
+void launch_tail(const DevScene& S, const WaveState& W, const WaveCtl* ctl, int max_stack,
+                 bool counters, const LaunchCfg& lc, int mode, const BatchRefs* br, bool mark,
+                 cudaStream_t st);
+/* Starts a chunk: *ctl = v, empty queues; first: the totals start at zero
+ * too (else they go on, with the error flags). */
+void launch_chunk_begin(const WaveState& W, WaveCtl* ctl, const WaveCtl& v, bool first,
+                        cudaStream_t st);
+/* Kernels of one iteration in `mode` (without a light or environment to
+ * sample there are no shadow rays to trace or finish). */
+int iteration_kernels(const LaunchCfg& lc, int mode, bool guide);
+/* Resident blocks per SM x SMs for a trace (kind 0), shade (kind 1) or tail
+ * (kind 2, blocks of PT_TAIL_BLOCK) kernel of `block` threads. */
 int wave_grid(int kind, int max_stack, int block);
 /* Raises the dynamic shared memory limit of the trace kernels to the
  * device maximum (once per device). */
 cudaError_t set_trace_smem();
 /* Default launch shape for a BVH of the given stack depth. */
 LaunchCfg default_launch(int max_stack);
-/* One wavefront iteration (7 kernels).  ev, if not null, holds 6 events
+/* One wavefront iteration (iteration_kernels launches).  ev, if not null, holds 6 events
  * recorded between the stages.  br: batch tables, or null for one scene.
  * use_cond: the queue-advance kernel sets graph conditional `cond` to
  * whether the chunk has work left (device-side iteration loop).  gi: the

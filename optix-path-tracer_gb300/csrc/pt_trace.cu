@@ -11,7 +11,7 @@
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include "pt_device.cuh"
+#include "pt_bvh.cuh"
 #include "pt_internal.h"
 #include "pt_wave.cuh"
 
@@ -53,69 +53,6 @@ struct WarpShared {
   uint32_t pair_prim[PT_PAIR_CAP];
   uint8_t pair_owner[PT_PAIR_CAP];
 };
-
-__device__ __forceinline__ uint32_t byte_of(uint32_t w, int i) { return (w >> (8 * i)) & 0xffu; }
-
-// Three-input max / min (one instruction each on sm_100+) and the paired
-// FP32 fused multiply-add: a node step evaluates 8 children x 3 axes of
-// (near, far) slab distances, so pairs share one instruction.
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-__device__ __forceinline__ float min3f(float a, float b, float c) {
-  float r;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-// (a.x * s + t, a.y * s + t), each rounded once.
-__device__ __forceinline__ float2 fma2s(float ax, float ay, float s, float t) {
-  unsigned long long a, b, c, d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(ax), "f"(ay));
-  asm("mov.b64 %0, {%1, %1};" : "=l"(b) : "f"(s));
-  asm("mov.b64 %0, {%1, %1};" : "=l"(c) : "f"(t));
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
-  return r;
-}
-
-__device__ __forceinline__ WtRay wt_unpack(float4 w) {
-  WtRay r;
-  uint32_t k = __float_as_uint(w.w);
-  r.kx = (int)(k & 3u);
-  r.ky = (int)((k >> 2) & 3u);
-  r.kz = (int)((k >> 4) & 3u);
-  r.Sx = w.x;
-  r.Sy = w.y;
-  r.Sz = w.z;
-  return r;
-}
-
-// Candidate of one primitive for a world-space ray (object space inside);
-// MOTION: spheres may move (at the ray's `time`), else every sphere is static.
-template <bool MOTION>
-__device__ __forceinline__ bool prim_test(const DevScene& S, const PrimRec& p, V3 o, V3 d,
-                                          const WtRay& wt, float tmin, float tmax, float& t,
-                                          float& bu, float& bv, float time) {
-  bu = bv = 0.f;
-  if (S.tri_only) return tri_candidate(p, o, wt, tmin, tmax, t, bu, bv);
-  int type = prim_type(p);
-  if (type == PT_PRIM_TRIANGLE) return tri_candidate(p, o, wt, tmin, tmax, t, bu, bv);
-  V3 oo = o, dd = d;
-  int xf = prim_xform(p);
-  if (xf >= 0) {
-    const float4* I = S.xforms + 6 * xf + 3;
-    oo = xpoint(I, o);
-    dd = xvector(I, d);
-  }
-  if (type == PT_PRIM_SPHERE)
-    return sphere_candidate_at(p, MOTION ? sphere_center(p, time) : v3(p.r0.x, p.r0.y, p.r0.z), oo,
-                               dd, tmin, tmax, t);
-  if (type == PT_PRIM_RECT) return rect_candidate(p, oo, dd, tmin, tmax, t);
-  return box_candidate(p, oo, dd, tmin, tmax, t);
-}
 
 struct FirstHitOut {
   uint32_t* prim;
@@ -168,9 +105,13 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
   // warp's shared copy, ws.rd[lane]: the node tests need only o, tmin and
   // the reciprocal direction)
   const uint32_t parity = MODE == TRACE_EXT ? c.parity : 0u;
-  V3 o = v3(0.f);
-  float tmin = 0.f, ix = 0.f, iy = 0.f, iz = 0.f, tbest = 0.f;
-  bool negx = false, negy = false, negz = false;
+  BoxRay ray;
+  V3& o = ray.o;
+  float& tmin = ray.tmin;
+  o = v3(0.f);
+  tmin = ray.ix = ray.iy = ray.iz = 0.f;
+  ray.negx = ray.negy = ray.negz = false;
+  float tbest = 0.f;
   uint32_t cur = 0, best_id = PT_NO_HIT;
   int sp = 0;
   bool active = false;
@@ -259,9 +200,7 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
     V3 d;
     float tmax;
     load_ray(d, tmax);
-    bool nan = !(o.x == o.x && o.y == o.y && o.z == o.z && d.x == d.x && d.y == d.y &&
-                 d.z == d.z);
-    if (nan || S.num_prims == 0) {
+    if (nan_ray(o, d) || S.num_prims == 0) {
       best_id = PT_NO_HIT;
       tbest = tmax;
       finish(d, tmax);
@@ -270,16 +209,7 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
       return;
     }
     active = true;
-    const float eps = 1e-18f;
-    float dx = fabsf(d.x) < eps ? copysignf(eps, d.x) : d.x;
-    float dy = fabsf(d.y) < eps ? copysignf(eps, d.y) : d.y;
-    float dz = fabsf(d.z) < eps ? copysignf(eps, d.z) : d.z;
-    ix = 1.0f / dx;
-    iy = 1.0f / dy;
-    iz = 1.0f / dz;
-    negx = ix < 0.f;
-    negy = iy < 0.f;
-    negz = iz < 0.f;
+    ray.set_direction(d);
     WtRay w = wt_setup(d);
     ws.ro[lane] = make_float4(o.x, o.y, o.z, tmin);
     ws.rd[lane] = make_float4(d.x, d.y, d.z, tmax);
@@ -334,69 +264,21 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
       }
     }
     if (!busy) break;
-    // ---- node step: the eight child boxes of each active lane's node.
-    // Internal children fill the low slots, slot == offset of the child node
-    // from child_base; leaf children follow.
-    uint32_t ihit = 0, leafmask = 0, pbase = 0, mlo = 0, mhi = 0, child_base = 0;
-    // the two nearest hit internal children: entry distance (tn >= 0, so its
-    // bits order like the value) with the slot in the low 3 bits
-    uint32_t k1 = 0xffffffffu, k2 = 0xffffffffu;
+    // ---- node step: the eight child boxes of each active lane's node
+    NodeHits hits;
+    hits.ihit = hits.leafmask = hits.pbase = hits.mlo = hits.mhi = hits.child_base = 0;
+    hits.k1 = hits.k2 = 0xffffffffu;
     if (active) {
-      const uint4* nptr = S.nodes + 5 * (size_t)cur;
-      uint4 n0 = __ldg(nptr), n1 = __ldg(nptr + 1), n2 = __ldg(nptr + 2), n3 = __ldg(nptr + 3),
-            n4 = __ldg(nptr + 4);
       if (COUNT) nn++;
-      child_base = n1.x;
-      pbase = n1.y;
-      mlo = n1.z;
-      mhi = n1.w;
-      const uint32_t im = n0.w >> 24;
-      // child bound q (8 bits) is read as the float f = 1 + q * 2^-15 built by
-      // one byte permute; t = q*a + b = f*A + B with A = 2^15 a, B = b - A
-      float sx = __uint_as_float((n0.w & 0xffu) << 23);
-      float sy = __uint_as_float(((n0.w >> 8) & 0xffu) << 23);
-      float sz = __uint_as_float(((n0.w >> 16) & 0xffu) << 23);
-      float Ax = 32768.0f * (sx * ix), Ay = 32768.0f * (sy * iy), Az = 32768.0f * (sz * iz);
-      float Bx = (__uint_as_float(n0.x) - o.x) * ix - Ax;
-      float By = (__uint_as_float(n0.y) - o.y) * iy - Ay;
-      float Bz = (__uint_as_float(n0.z) - o.z) * iz - Az;
-      uint32_t nx0 = negx ? n3.z : n2.x, nx1 = negx ? n3.w : n2.y;
-      uint32_t fx0 = negx ? n2.x : n3.z, fx1 = negx ? n2.y : n3.w;
-      uint32_t ny0 = negy ? n4.x : n2.z, ny1 = negy ? n4.y : n2.w;
-      uint32_t fy0 = negy ? n2.z : n4.x, fy1 = negy ? n2.w : n4.y;
-      uint32_t nz0 = negz ? n4.z : n3.x, nz1 = negz ? n4.w : n3.y;
-      uint32_t fz0 = negz ? n3.x : n4.z, fz1 = negz ? n3.y : n4.w;
-      float tlim = tbest * 1.0000005f;
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const uint32_t sel = 0x7604u | ((uint32_t)(k & 3) << 4);
-        float2 tx = fma2s(__uint_as_float(__byte_perm(k < 4 ? nx0 : nx1, 0x3F800000u, sel)),
-                          __uint_as_float(__byte_perm(k < 4 ? fx0 : fx1, 0x3F800000u, sel)), Ax, Bx);
-        float2 ty = fma2s(__uint_as_float(__byte_perm(k < 4 ? ny0 : ny1, 0x3F800000u, sel)),
-                          __uint_as_float(__byte_perm(k < 4 ? fy0 : fy1, 0x3F800000u, sel)), Ay, By);
-        float2 tz = fma2s(__uint_as_float(__byte_perm(k < 4 ? nz0 : nz1, 0x3F800000u, sel)),
-                          __uint_as_float(__byte_perm(k < 4 ? fz0 : fz1, 0x3F800000u, sel)), Az, Bz);
-        float tn = max3f(tx.x, ty.x, fmaxf(tz.x, tmin));
-        float tf = min3f(tx.y, ty.y, fminf(tz.y, tlim));
-        // an empty slot (meta 0) has an inverted box and fails here; were it
-        // to pass (infinite slab distances), it is a leaf of no primitives.
-        if (tn <= tf) {
-          if ((im >> k) & 1u) {
-            const uint32_t key = (__float_as_uint(tn) & 0xfffffff8u) | (uint32_t)k;
-            k2 = min(k2, max(k1, key));
-            k1 = min(k1, key);
-            ihit |= 1u << k;
-          } else {
-            leafmask |= 1u << k;
-          }
-        }
-      }
+      node_step(S.nodes + 5 * (size_t)cur, ray, tbest * 1.0000005f, hits);
     }
     // ---- next node, chosen before the primitive tests: the nearest hit
     // internal child, the others pushed as one group (closest hit: in
     // near-to-far order with the distance of the nearest; occlusion: as a
     // mask).  With no internal child hit, a closest-hit ray pops after the
     // tests, which may shorten it and so drop groups beyond the new hit.
+    const uint32_t ihit = hits.ihit, child_base = hits.child_base, pbase = hits.pbase;
+    const uint32_t k1 = hits.k1, k2 = hits.k2;
     const int nint = __popc(ihit);
     bool pop = false;
     float tnext = 0.f;
@@ -451,16 +333,7 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
     // whose ray ended above: its leaves of this node still count).  pm: the
     // lane's primitives as bits over the node's range, bit j = record
     // pbase + j (a node's leaves hold at most 24 primitives).
-    uint32_t pm = 0;
-    {
-      uint32_t m = leafmask;
-      while (m) {
-        const int k = __ffs(m) - 1;
-        m &= m - 1;
-        const uint32_t meta = (k < 4 ? mlo : mhi) >> (8 * (k & 3));
-        pm |= ((1u << ((meta >> 5) & 7u)) - 1u) << (meta & 31u);
-      }
-    }
+    const uint32_t pm = leaf_prims(hits);
     if (__any_sync(0xffffffffu, pm != 0)) {
       const uint32_t cnt = __popc(pm);
       const uint32_t total = __reduce_add_sync(0xffffffffu, cnt);

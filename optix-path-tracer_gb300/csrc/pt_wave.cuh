@@ -15,6 +15,14 @@ __device__ __forceinline__ uint32_t gen_count(const WaveCounters& c, const WaveC
   return (uint32_t)min((unsigned long long)(slots - c.n_cur), left);
 }
 
+// Whether the tail kernel takes the chunk's remaining paths: few are left and,
+// with the guide, all of them are past the guided bounces.
+__device__ __forceinline__ bool tail_ready(const WaveCounters& c, const WaveCtl& ctl) {
+  const unsigned long long left = ctl.chunk_paths - c.next_path;
+  if (c.error || left + c.n_cur > ctl.tail_max) return false;
+  return !ctl.guide || (left == 0 && c.drained >= ctl.guide_depth);
+}
+
 __device__ __forceinline__ Ray3 camera_ray(const GpuCamera& cam, uint32_t x, uint32_t y,
                                            uint32_t Wd, uint32_t Hd, uint32_t& seed) {
   float u = float((float)x + rnd(seed)) / (float)Wd;
