@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <algorithm>
 #include "pt_device.cuh"
 #include "pt_internal.h"
 #include "pt_shade.cuh"
@@ -110,6 +111,9 @@ __global__ void k_generate(DevScene S0, WaveState W, const WaveCtl* __restrict__
 #define PT_SHADE_TILE_GRID 1
 #endif
 #define PT_SORT_KEYS (PT_NUM_MAT_TYPES + 2)
+#ifndef PT_SORT_FILL
+#define PT_SORT_FILL 1024u  // tiles that keep the GPU busy
+#endif
 
 struct SortTile {
   uint16_t perm[PT_SHADE_BLOCK * PT_SORT_ITEMS];  // tile position in sorted order
@@ -128,13 +132,14 @@ __device__ __forceinline__ uint32_t shade_key(const DevScene& S0, const float4* 
 
 __device__ __forceinline__ void sort_tile(SortTile& t, const DevScene& S0,
                                           const float4* __restrict__ hit, uint32_t base,
-                                          uint32_t n) {
+                                          uint32_t n, int items) {
   const uint32_t bd = blockDim.x;
   if (threadIdx.x < PT_SORT_KEYS) t.cnt[threadIdx.x] = 0;
   __syncthreads();
   uint32_t key[PT_SORT_ITEMS], rank[PT_SORT_ITEMS];
 #pragma unroll
   for (int it = 0; it < PT_SORT_ITEMS; it++) {
+    if (it >= items) break;
     key[it] = shade_key(S0, hit, base + it * bd + threadIdx.x, n);
     rank[it] = atomicAdd(&t.cnt[key[it]], 1u);
   }
@@ -148,9 +153,20 @@ __device__ __forceinline__ void sort_tile(SortTile& t, const DevScene& S0,
   }
   __syncthreads();
 #pragma unroll
-  for (int it = 0; it < PT_SORT_ITEMS; it++)
+  for (int it = 0; it < PT_SORT_ITEMS; it++) {
+    if (it >= items) break;
     t.perm[t.start[key[it]] + rank[it]] = (uint16_t)(it * bd + threadIdx.x);
+  }
   __syncthreads();
+}
+
+// Paths per thread of a tile: larger tiles sort better, but a launch of fewer
+// than PT_SORT_FILL tiles leaves SMs idle, and a block takes its paths one
+// after the other, so small launches use smaller tiles.  GB300: 33 frames of
+// 321 x 243 with textures 3467 -> 3346 us (every launch with 1024-path tiles,
+// then this rule); launches that fill the GPU keep 1024.
+__device__ __forceinline__ int sort_items(uint32_t n) {
+  return (int)min((uint32_t)PT_SORT_ITEMS, 1u + n / (PT_SORT_FILL * blockDim.x));
 }
 
 // Loop of a shade kernel over its paths: material-sorted tiles (SORT) or a
@@ -158,10 +174,11 @@ __device__ __forceinline__ void sort_tile(SortTile& t, const DevScene& S0,
 // appends inside are warp-aggregated).
 #define SHADE_LOOP(CALL)                                                           \
   if (SORT) {                                                                      \
-    const uint32_t tile_n = blockDim.x * PT_SORT_ITEMS;                            \
+    const int items = sort_items(n);                                               \
+    const uint32_t tile_n = blockDim.x * items;                                    \
     for (uint32_t base = blockIdx.x * tile_n; base < n; base += gridDim.x * tile_n) { \
-      sort_tile(tile, S0, W.hit, base, n);                                         \
-      for (int it = 0; it < PT_SORT_ITEMS; it++) {                                 \
+      sort_tile(tile, S0, W.hit, base, n, items);                                  \
+      for (int it = 0; it < items; it++) {                                         \
         uint32_t i = base + tile.perm[it * blockDim.x + threadIdx.x];              \
         CALL;                                                                      \
       }                                                                            \
@@ -746,6 +763,14 @@ void launch_chunk_begin(const WaveState& W, WaveCtl* ctl, const WaveCtl& v, bool
   k_chunk_begin<<<1, 1, 0, st>>>(W, ctl, v, first ? 1 : 0);
 }
 
+// Blocks of a sorted shading launch: one per tile of a full buffer, or as many
+// as its smaller tiles need when it is not full (sort_items).
+static int sort_grid(int slots, int block) {
+  const long long full = ((long long)slots + block * PT_SORT_ITEMS - 1) / (block * PT_SORT_ITEMS);
+  const long long fine = ((long long)slots + block - 1) / block;
+  return (int)std::max<long long>(1, std::max(full, std::min<long long>(fine, PT_SORT_FILL)));
+}
+
 template <bool BATCH>
 static void launch_iteration_t(const DevScene& S, const WaveState& W, const WaveCtl* ctl,
                                int max_stack, bool counters, const LaunchCfg& lc, cudaStream_t st,
@@ -755,9 +780,8 @@ static void launch_iteration_t(const DevScene& S, const WaveState& W, const Wave
   const BatchRefs* brp = BATCH ? &br : nullptr;
   // sorted shading: one block per tile of the buffer (blocks past the live
   // paths return at once), so the block scheduler balances uneven tiles
-  const int tile = sb * PT_SORT_ITEMS;
 #if PT_SHADE_TILE_GRID
-  const int tgs = W.slots > 0 ? (W.slots + tile - 1) / tile : 1;
+  const int tgs = sort_grid(W.slots, sb);
 #else
   const int tgs = sg;
 #endif
