@@ -274,6 +274,8 @@ PT_API int pt_context_destroy(pt_context* ctx) {
   ctx->d_env_rows.release();
   ctx->d_env_pre.release();
   ctx->d_env_valid.release();
+  ctx->d_env_row.release();
+  ctx->d_env_idx.release();
   ctx->d_slot_f4.release();
   ctx->d_slot_u4.release();
   ctx->d_ctr.release();
@@ -937,9 +939,24 @@ static cudaError_t upload_tables(pt_context* ctx, size_t* bytes) {
     if (e == cudaSuccess) e = ctx->d_env_rows.ensure((size_t)h);
     if (e == cudaSuccess) e = ctx->d_env_pre.ensure((size_t)w * h);
     if (e == cudaSuccess) e = ctx->d_env_valid.ensure(1);
+    if (e == cudaSuccess) e = ctx->d_env_row.ensure((size_t)h);
+    // search tables about as fine as the CDFs; their entries are 16-bit
+    const bool idx = w <= 65535 && h <= 65535;
+    auto bits = [](int n) {
+      int b = 0;
+      while (b < 16 && (1 << b) < n) b++;
+      return b;
+    };
+    const int mb = bits(h), cb = bits(w);
+    const size_t nm = ((size_t)1 << mb) + 1, nc = ((size_t)1 << cb) + 1;
+    if (idx && e == cudaSuccess) e = ctx->d_env_idx.ensure(nm + nc * h);
+    ctx->env_marg_bits = mb;
+    ctx->env_cond_bits = cb;
     if (e == cudaSuccess) {
+      uint16_t* mi = idx ? ctx->d_env_idx.p : nullptr;
       pt::launch_env_cdf(ctx->d_env.p, w, h, ctx->d_env_marg.p, ctx->d_env_cond.p,
-                         ctx->d_env_rows.p, ctx->d_env_pre.p, ctx->d_env_valid.p, st);
+                         ctx->d_env_rows.p, ctx->d_env_pre.p, ctx->d_env_valid.p,
+                         ctx->d_env_row.p, mi, mb, idx ? mi + nm : nullptr, cb, st);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess)
@@ -1003,7 +1020,15 @@ PT_API int pt_commit(pt_context* ctx) {
   S.cam = ctx->cam;
   S.env_marg = ctx->d_env_marg.p;
   S.env_cond = ctx->d_env_cond.p;
-  S.env_valid = ctx->env_valid;
+  S.env_valid = ctx->env_valid ? 1 : 0;
+  S.env_row = ctx->d_env_row.p;
+  S.env_marg_bits = ctx->env_marg_bits;
+  S.env_cond_bits = ctx->env_cond_bits;
+  // a total that is not finite makes CDFs that are not sorted: searched whole
+  if (ctx->env_valid == 3 && ctx->miss.w <= 65535 && ctx->miss.h <= 65535) {
+    S.env_marg_idx = ctx->d_env_idx.p;
+    S.env_cond_idx = ctx->d_env_idx.p + ((size_t)1 << ctx->env_marg_bits) + 1;
+  }
   ctx->bvh_depth = depth;
   ctx->bvh_nodes = nn;
   ctx->bvh_width = width;

@@ -146,6 +146,9 @@ struct pt_context {
   DevBuf<double> d_env_rows;
   DevBuf<double> d_env_pre;   // per texel: weights, then row prefix sums
   DevBuf<int> d_env_valid;
+  DevBuf<float2> d_env_row;
+  DevBuf<uint16_t> d_env_idx; // search tables: marginal, then conditional
+  int env_marg_bits = 0, env_cond_bits = 0;
   int env_valid = 0;
   DevScene scene{};
   int bvh_depth = 0;

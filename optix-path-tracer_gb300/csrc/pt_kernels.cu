@@ -662,7 +662,8 @@ __global__ void k_env_cond(const double* __restrict__ pre, const double* __restr
 
 // Marginal CDF over the row totals: the sums by one thread in the oracle's
 // order (rows[] becomes the running sums), the divisions by the block.
-__global__ void k_env_marg(double* rows, int h, float* marg, int* valid) {
+// *valid: bit 0 the environment can be sampled, bit 1 its total is finite.
+__global__ void k_env_marg(double* rows, int h, float* marg, float2* row, int* valid) {
   __shared__ double tot_s;
   if (blockIdx.x != 0) return;
   if (threadIdx.x == 0) {
@@ -674,7 +675,7 @@ __global__ void k_env_marg(double* rows, int h, float* marg, int* valid) {
       rows[r] = mp;
     }
     tot_s = tot;
-    *valid = tot > 0.0 ? 1 : 0;
+    *valid = tot > 0.0 ? (isfinite(tot) ? 3 : 1) : 0;
   }
   __syncthreads();
   const double tot = tot_s;
@@ -683,6 +684,28 @@ __global__ void k_env_marg(double* rows, int h, float* marg, int* valid) {
   if (threadIdx.x == 0) marg[0] = 0.f;
   __syncthreads();
   if (threadIdx.x == 0) marg[h] = 1.f;
+  __syncthreads();
+  for (int r = threadIdx.x; r < h; r += blockDim.x)
+    row[r] = make_float2(marg[r + 1] - marg[r], pt_sinf(PI_F * (((float)r + 0.5f) / (float)h)));
+}
+
+// Where the searches of cdf_find_from start: row -1 the marginal CDF, rows
+// 0..h-1 the conditional ones (a 2048 x 1024 sky: 2 M searches, 4 MB).
+__global__ void k_env_index(const float* __restrict__ marg, const float* __restrict__ cond, int w,
+                            int h, int marg_bits, int cond_bits, uint16_t* marg_idx,
+                            uint16_t* cond_idx) {
+  const size_t nm = ((size_t)1 << marg_bits) + 1, nc = ((size_t)1 << cond_bits) + 1;
+  const size_t n = nm + nc * h;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    if (i < nm) {
+      marg_idx[i] = (uint16_t)cdf_find(marg, h, (float)i / (float)(1 << marg_bits));
+    } else {
+      const size_t r = (i - nm) / nc, k = (i - nm) - r * nc;
+      cond_idx[i - nm] =
+          (uint16_t)cdf_find(cond + r * (w + 1), w, (float)k / (float)(1 << cond_bits));
+    }
+  }
 }
 
 // ------------------------------------------------------- host launchers ---
@@ -861,12 +884,15 @@ void launch_paths_out(const float4* results, float* out, uint32_t n, cudaStream_
 }
 
 void launch_env_cdf(const float4* env, int w, int h, float* marg, float* cond, double* rows,
-                    double* pre, int* valid, cudaStream_t st) {
+                    double* pre, int* valid, float2* row, uint16_t* marg_idx, int marg_bits,
+                    uint16_t* cond_idx, int cond_bits, cudaStream_t st) {
   const int g = num_sms() * 8;
   k_env_weights<<<g, 256, 0, st>>>(env, w, h, pre);
   k_env_prefix<<<(h + 31) / 32, 32, 0, st>>>(pre, w, h, rows);
   k_env_cond<<<g, 256, 0, st>>>(pre, rows, w, h, cond);
-  k_env_marg<<<1, 256, 0, st>>>(rows, h, marg, valid);
+  k_env_marg<<<1, 256, 0, st>>>(rows, h, marg, row, valid);
+  if (marg_idx)
+    k_env_index<<<g, 256, 0, st>>>(marg, cond, w, h, marg_bits, cond_bits, marg_idx, cond_idx);
 }
 
 void launch_resolve(const float4* acc, uchar4* out, int n, int frame, cudaStream_t st) {

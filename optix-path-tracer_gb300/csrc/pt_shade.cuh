@@ -264,11 +264,7 @@ __device__ __forceinline__ V3 miss_color(const GpuMiss& ms, V3 d) {
   }
   float u, v;
   if (ms.spherical) {
-    float r = length(d);
-    float lon = pt_atan2f(d.z, d.x);
-    float lat = pt_acosf(d.y / r);
-    u = lon * (1.f / (PI_F * 2.f));
-    v = lat * (1.f / PI_F);
+    env_uv(d, u, v);
   } else {
     float theta = pt_atan2f(d.x, d.z);
     theta = theta < 0.f ? theta + (2.f * PI_F) : theta;
@@ -409,6 +405,16 @@ __device__ __forceinline__ void finish_step(const DevScene& S, uint4& st, V3& th
   after_nee(m, st.x, n.P, n.Wo, n.N, direct, thr, rad, tl);
 }
 
+// Radiance and sampling density of an importance-sampled environment (then the
+// miss program is the spherical HDR map) in direction d, from one set of
+// coordinates.
+__device__ __forceinline__ void env_eval(const DevScene& S, V3 d, V3& Le, float& pdf) {
+  float u, v;
+  env_uv(d, u, v);
+  pdf = env_pdf_uv(S, u, v);
+  Le = 2.f * env_lookup(S.miss, u, v);
+}
+
 // Sum over the lights of their sampling pdf for direction d from P (per
 // light selection), the MIS partner of BSDF sampling at emitter hits.
 __device__ __forceinline__ float lights_pdf_c(const DevScene& S, V3 P, V3 d, int n_sel) {
@@ -478,9 +484,15 @@ __device__ __forceinline__ void shade_step_c(const DevScene& S, const PathCtl& p
   float pdf_prev = __uint_as_float(st.w);
   uint32_t leaf = __float_as_uint(hit.w);
   if (leaf == PT_NO_HIT) {
-    V3 Le = miss_color(S.miss, d);
+    V3 Le;
     float w = 1.f;
-    if (!prev_spec && S.env_valid) w = power_mis(pdf_prev, env_pdf_dir(S, d) / (float)n_sel);
+    if (!prev_spec && S.env_valid) {
+      float pe;
+      env_eval(S, d, Le, pe);
+      w = power_mis(pdf_prev, pe / (float)n_sel);
+    } else {
+      Le = miss_color(S.miss, d);
+    }
     rad += thr * Le * w;
     ended = true;
   } else {
@@ -555,16 +567,16 @@ __device__ __forceinline__ void shade_step_c(const DevScene& S, const PathCtl& p
           float u1 = rnd(st.x);
           float u2 = rnd(st.x);
           Wi = env_sample_dir(S, u1, u2);
-          pl = env_pdf_dir(S, Wi);
-          Le = miss_color(S.miss, Wi);
+          env_eval(S, Wi, Le, pl);
         }
         V3 wi_n = normalize(Wi);
         float cs = dot(wi_n, N);
         float pls = pl / (float)n_sel;
         if (cs > 0.f && pls > 0.f && tmax > 1e-3f) {
           V3 wi_l = fr.to_local(wi_n);
-          V3 f = bsdf_f_c(m, wo_l, wi_l);
-          float pbs = bsdf_pdf_c(m, wo_l, wi_l);
+          V3 f;
+          float pbs;
+          bsdf_eval_c(m, wo_l, wi_l, f, pbs);
           if (guided)
             pbs = G_alpha * guide_pdf_packed(G, wi_n.x, wi_n.y, wi_n.z) + (1.f - G_alpha) * pbs;
           V3 cv = f * Le * (cs * power_mis(pls, pbs) / pls);
@@ -585,10 +597,11 @@ __device__ __forceinline__ void shade_step_c(const DevScene& S, const PathCtl& p
         wi_l = bsdf_sample_c(m, wo_l, st.x);
         wdir = fr.to_world(wi_l);
       }
-      float pbs = bsdf_pdf_c(m, wo_l, wi_l);
+      V3 f;
+      float pbs;
+      bsdf_eval_c(m, wo_l, wi_l, f, pbs);
       float q = pbs;
       if (guided) q = G_alpha * guide_pdf_packed(G, wdir.x, wdir.y, wdir.z) + (1.f - G_alpha) * pbs;
-      V3 f = bsdf_f_c(m, wo_l, wi_l);
       if (!(q > 0.f) || isNull(f) || !(wi_l.y > 0.f)) {
         ended = true;
       } else {

@@ -31,6 +31,7 @@
 #define PT_TYPES_H
 
 #include <stdint.h>
+#include <vector_types.h>
 
 #define PT_PRIM_TRIANGLE 0
 #define PT_PRIM_SPHERE 1
@@ -121,6 +122,11 @@ struct DevScene {
   const uint32_t* leaf_of_id; /* primitive id -> position in the leaf-ordered records */
   const float* env_marg;    /* environment sampling: marginal CDF over rows (h+1) */
   const float* env_cond;    /* conditional CDFs, h rows of w+1 */
+  const float2* env_row;    /* per row: its marginal probability, sin of its polar angle */
+  /* where a CDF search starts: for each of 2^bits + 1 equally spaced u, the
+     entry found (marginal; conditional per row); null: search the whole CDF */
+  const uint16_t *env_marg_idx, *env_cond_idx;
+  int env_marg_bits, env_cond_bits;
   int env_valid;            /* 1 if the environment can be importance sampled */
   int num_lights;
   int num_prims;
