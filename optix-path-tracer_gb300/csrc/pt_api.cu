@@ -1076,6 +1076,11 @@ void pth::carve_wave(WaveState& W, float4* f, uint4* u, size_t s) {
   W.sh.rad = f + 14 * s;
   W.sh.C = f + 15 * s;
   W.sh.st = u + 2 * s;
+  for (int k = 0; k < 2; k++) {
+    W.nee[k].Wi = k ? W.sh.P : W.sh.Wi;
+    W.nee[k].C = k ? W.sh.N : W.sh.C;
+    W.nee[k].queue = (uint32_t*)(u + 2 * s) + k * s;
+  }
   W.slots = (int)s;
 }
 
@@ -1263,7 +1268,7 @@ static int run_chunk(pt_context* ctx, const pt_render_params* p, int frame0, int
   WaveCtl ctl = chunk_ctl(ctx, p, frame0, frames);
   const unsigned long long slots = (unsigned long long)ctx->slots;
   ctl.max_iter =
-      ((ctl.chunk_paths + slots - 1) / slots + 2) * (unsigned long long)(p->max_depth + 1) + 16;
+      ((ctl.chunk_paths + slots - 1) / slots + 2) * (unsigned long long)(p->max_depth + 2) + 16;
   const bool counters = ctx->opt.enable_counters != 0;
   const bool timing = ctx->opt.enable_timing != 0;
   const bool guide = p->guide != 0;

@@ -19,8 +19,8 @@
  *     k_accumulate_batch, k_batch_end
  *
  * Both loops are bounded on the device (by the chunk count, and per chunk by
- * (ceil(paths / slots) + 2) * (max depth + 1) + 16 iterations: every path
- * ends within max depth iterations of its generation, and generation keeps
+ * (ceil(paths / slots) + 2) * (max depth + 2) + 16 iterations: every path
+ * ends within max depth + 1 iterations of its generation, and generation keeps
  * the slots full while paths remain) and end on any error flag.  With
  * per-stage timing, or where the runtime refuses conditional nodes, the same
  * kernels run under a host loop.
@@ -507,7 +507,7 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
   auto close = [&]() {
     if (!cur.paths) return;
     cur.seg_end = (uint32_t)segs.size();
-    cur.max_iter = ((cur.paths + slots - 1) / slots + 2) * (unsigned long long)(cur_depth + 1) + 16;
+    cur.max_iter = ((cur.paths + slots - 1) / slots + 2) * (unsigned long long)(cur_depth + 2) + 16;
     max_chunk = std::max<size_t>(max_chunk, cur.paths);
     chunks.push_back(cur);
     cur = BatchChunk{};

@@ -72,7 +72,10 @@ struct Ray3 {
 struct WaveCounters {
   uint32_t n_cur;        /* live paths at the start of the current buffer (before generation) */
   uint32_t n_next;       /* paths written to the next buffer */
-  uint32_t n_shadow;     /* paths parked at a shadow ray this iteration */
+  uint32_t n_shadow;     /* shadow rays queued this iteration */
+  uint32_t n_occ;        /* consistent mode: occlusion rays of the current buffer's paths */
+  uint32_t n_wait, n_wait_next; /* paths of the current / next buffer that have ended but
+                            for their NEE term */
   uint32_t parity;       /* which path buffer is current */
   uint32_t error;        /* bit 0: traversal stack overflow, bit 1: iteration bound reached */
   uint32_t iter;         /* iterations of the current chunk */
@@ -162,14 +165,26 @@ struct PathBuf {
   uint4* st;                  /* seed, path id, depth|prevSpecular<<16 */
 };
 
-/* Paths parked at a shadow ray (Direct_Light context), in shadow-queue
- * order. */
+/* Reference mode: paths parked at a shadow ray (Direct_Light context: the
+ * random stream after it depends on it), in shadow-queue order. */
 struct ShadowBuf {
   float4 *P, *N, *Wo, *Wi;    /* P+light pdf, N+light index, Wo+material, Wi+occluded */
-  float4* C;                  /* consistent mode: NEE term + shadow tmax */
+  float4* C;                  /* texture colour */
   float4 *thr, *rad;
   uint4* st;
 };
+
+/* Consistent mode: NEE terms of the paths of a buffer, by position.  The
+ * continuation does not depend on the occlusion ray, so a path goes on at
+ * once and adds its term when it is next shaded, after both its rays were
+ * traced in one launch; a path that has ended waits one iteration for it
+ * (ray_d.w = 0: no extension ray). */
+struct NeeBuf {
+  float4* Wi;                 /* direction + occluded */
+  float4* C;                  /* term + tmax */
+  uint32_t* queue;            /* positions of the paths with an occlusion ray */
+};
+#define PT_CODE_PENDING 8     /* rad.w of such a path: this + its guide-record word */
 
 struct GuidePacked;
 struct GuideSample;
@@ -178,7 +193,8 @@ struct GuideInferArgs;
 struct WaveState {
   PathBuf path[2];            /* ping-pong: path[parity] is current */
   float4* hit;                /* t, u, v, leaf index: by position in the current buffer */
-  ShadowBuf sh;
+  ShadowBuf sh;               /* reference mode */
+  NeeBuf nee[2];              /* consistent mode, beside path[]; shares sh's memory */
   WaveCounters* ctr;
   float4* results;            /* per path of the chunk: colour */
   int slots;                  /* capacity of each buffer */
@@ -196,15 +212,16 @@ struct WaveState {
 
 /* Ray kinds of the trace kernels: closest hit of extension rays; closest
  * hit of a shadow ray (reference mode: the light must be the first thing
- * hit); first-hit queries; any hit before tmax (consistent-mode occlusion). */
-enum { TRACE_EXT = 0, TRACE_SHADOW = 1, TRACE_FIRST = 2, TRACE_OCCLUDED = 3 };
+ * hit); first-hit queries; any hit before tmax (consistent-mode occlusion);
+ * extension rays, then occlusion rays. */
+enum { TRACE_EXT = 0, TRACE_SHADOW = 1, TRACE_FIRST = 2, TRACE_OCCLUDED = 3, TRACE_BOTH = 4 };
 
 namespace pt {
 /* Dynamic shared memory of a trace block (pt_trace.cu). */
 size_t trace_smem(int max_stack, int block);
 /* Resident trace blocks per SM (0 if the shape does not fit). */
 int trace_blocks_per_sm(int block, size_t smem);
-/* One trace launch of `mode` (TRACE_EXT, TRACE_SHADOW or TRACE_OCCLUDED)
+/* One trace launch of `mode` (TRACE_EXT, TRACE_SHADOW or TRACE_BOTH)
  * over the wavefront's rays, with the launch shape of lc. */
 void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W,
                   const WaveCtl* ctl, int max_stack, const BatchRefs* br, const LaunchCfg& lc,

@@ -14,9 +14,11 @@
  *   k_trace_t<SHADOW> shadow rays (programs/hit.cu:16-24, closest-hit rule)
  *   k_finish        rest of Direct_Light (MIS), BSDF continuation
  *   k_advance       counter bookkeeping (one thread)
- * The consistent mode (NEE over lights and the environment with MIS) uses
- * k_shade_c, k_trace_t<OCCLUDED> (any hit before the light ends the ray) and
- * k_finish_c in the same places.  Trace warps take rays from a per-launch
+ * The consistent mode (NEE over lights and the environment with MIS) samples
+ * the continuation before the occlusion test is known, so k_shade_c passes
+ * the path on with its NEE term pending, and the next iteration traces both
+ * rays in one launch (k_trace_t<BOTH>: extension rays, then occlusion rays,
+ * which any hit before the light ends) and adds the term.  Trace warps take rays from a per-launch
  * counter (ray_next), so no warp sits idle while others still have rays.
  * Without lights (or a sampled environment) the shadow stages are not
  * launched.  The iterations of a chunk run in a conditional graph node that
@@ -287,25 +289,8 @@ __global__ void __launch_bounds__(PT_SHADE_BLOCK) k_finish(DevScene S0, WaveStat
 
 // ------------------------------------------------- consistent-mode stages --
 
-// Appends a continuing path (consistent mode) to the next buffer; tm is the
-// path's time (in the throughput's w), rad_w the guide-record word carried
-// in the radiance's w (0 without the guide).
-__device__ __forceinline__ void path_push(const WaveState& W, const WaveCounters& c, uint4 st,
-                                          V3 thr, V3 rad, V3 o, V3 d, bool cont, float tm,
-                                          float rad_w = 0.f) {
-  uint32_t pos = warp_push(&W.ctr->n_next, cont);
-  if (cont) {
-    const PathBuf& nb = W.path[c.parity ^ 1u];
-    nb.ray_o[pos] = make_float4(o.x, o.y, o.z, 1e-3f);
-    nb.ray_d[pos] = make_float4(d.x, d.y, d.z, PT_RAY_TMAX);
-    nb.thr[pos] = make_float4(thr.x, thr.y, thr.z, tm);
-    nb.rad[pos] = make_float4(rad.x, rad.y, rad.z, rad_w);
-    nb.st[pos] = st;
-  }
-}
-
-
-// One path of k_shade_c (see shade_path).
+// One path of k_shade_c (see shade_path): adds the NEE term of the previous
+// bounce, then shades this one.
 template <bool BATCH, bool GUIDE, bool TEX>
 __device__ __forceinline__ void shade_c_path(const DevScene& S0, const WaveState& W,
                                            const WaveCounters& c, const WaveCtl& ctl,
@@ -320,34 +305,46 @@ __device__ __forceinline__ void shade_c_path(const DevScene& S0, const WaveState
   if (active) st = pb.st[i];
   const DevScene& S = path_scene<BATCH>(S0, br, st.z);
   if (active) {
-    const float4 t4 = pb.thr[i], r4 = pb.rad[i];
+    const float4 t4 = pb.thr[i], r4 = pb.rad[i], d4 = pb.ray_d[i];
     thr = f4xyz(t4);
     tm = t4.w;
     rad = f4xyz(r4);
-    b.code = GUIDE ? r4.w : 0.f;
-    shade_step_c<GUIDE, TEX>(S, path_ctl<BATCH>(ctl, br, st.z), W, ctl.guide_depth, i, W.hit[i],
-                             f4xyz(pb.ray_o[i]), f4xyz(pb.ray_d[i]), tm, st, thr, rad, b);
+    const int word = (int)r4.w;
+    if (word & PT_CODE_PENDING) nee_arrived(W, W.nee[c.parity].Wi[i].w, W.nee[c.parity].C[i], st.y, word, rad);
+    b.code = GUIDE ? (float)(word & 6) : 0.f;
+    if (d4.w == 0.f)
+      b.ended = true;
+    else
+      shade_step_c<GUIDE, TEX>(S, path_ctl<BATCH>(ctl, br, st.z), W, ctl.guide_depth, i, W.hit[i],
+                               f4xyz(pb.ray_o[i]), f4xyz(d4), tm, st, thr, rad, b);
   }
-  const V3 P = b.P, Wi = b.Wi, C = b.C, dcont = b.dcont;
-  const bool ended = b.ended, shadow = b.shadow;
-  const float tmax = b.tmax, code = b.code;
-  uint32_t spos = warp_push(&W.ctr->n_shadow, shadow);
-  if (shadow) {
-    W.sh.P[spos] = make_float4(P.x, P.y, P.z, 0.f);
-    W.sh.Wi[spos] = make_float4(Wi.x, Wi.y, Wi.z, 0.f);
-    W.sh.C[spos] = make_float4(C.x, C.y, C.z, tmax);
-    W.sh.Wo[spos] = make_float4(dcont.x, dcont.y, dcont.z, ended ? 1.f : 0.f);
-    W.sh.thr[spos] = make_float4(thr.x, thr.y, thr.z, tm);
-    W.sh.rad[spos] = make_float4(rad.x, rad.y, rad.z, code);
-    W.sh.st[spos] = st;
-  }
-  if (active && !shadow && ended) {
+  if (active && !b.shadow && b.ended) {
     finalize_path(W, st.y, rad);
-    if (GUIDE) guide_end(W, st.y, code, rad);
+    if (GUIDE) guide_end(W, st.y, b.code, rad);
   }
-  // the next vertex starts without a pending record of its own
-  float cw = GUIDE ? (float)(((int)code >> 1) * 2) : 0.f;
-  path_push(W, c, st, thr, rad, P, dcont, active && !shadow && !ended, tm, cw);
+  // a path with an occlusion ray goes on (or, ended, waits) with its NEE term
+  // pending; else the next vertex starts without a pending record of its own
+  const bool push = active && (b.shadow || !b.ended);
+  const uint32_t pos = warp_push(&W.ctr->n_next, push);
+  if (push) {
+    const PathBuf& nb = W.path[c.parity ^ 1u];
+    const int word = GUIDE ? (int)b.code : 0;
+    nb.ray_o[pos] = make_float4(b.P.x, b.P.y, b.P.z, 1e-3f);
+    nb.ray_d[pos] = make_float4(b.dcont.x, b.dcont.y, b.dcont.z, b.ended ? 0.f : PT_RAY_TMAX);
+    nb.thr[pos] = make_float4(thr.x, thr.y, thr.z, tm);
+    nb.rad[pos] = make_float4(rad.x, rad.y, rad.z,
+                              (float)(b.shadow ? word + PT_CODE_PENDING : word & 6));
+    nb.st[pos] = st;
+  }
+  const uint32_t q = warp_push(&W.ctr->n_shadow, b.shadow);
+  if (b.shadow) {
+    const NeeBuf& ne = W.nee[c.parity ^ 1u];
+    ne.queue[q] = pos;
+    ne.Wi[pos] = make_float4(b.Wi.x, b.Wi.y, b.Wi.z, 0.f);
+    ne.C[pos] = make_float4(b.C.x, b.C.y, b.C.z, b.tmax);
+  }
+  const uint32_t waits = __ballot_sync(0xffffffffu, b.shadow && b.ended);
+  if (waits && (threadIdx.x & 31) == 0) atomicAdd(&W.ctr->n_wait_next, (uint32_t)__popc(waits));
 }
 
 template <bool BATCH, bool SORT, bool GUIDE, bool TEX>
@@ -361,50 +358,6 @@ __global__ void __launch_bounds__(PT_SHADE_BLOCK, GUIDE ? PT_SHADE_G_MINBLOCKS :
   SHADE_LOOP((shade_c_path<BATCH, GUIDE, TEX>(S0, W, c, ctl, br, i, i < n)))
 }
 
-__global__ void __launch_bounds__(PT_SHADE_BLOCK) k_finish_c(DevScene S, WaveState W,
-                                                             const WaveCtl* __restrict__ ctlp) {
-  (void)S;
-  (void)ctlp;
-  WaveCounters c = *W.ctr;
-  uint32_t n = c.n_shadow;
-  uint32_t stride = gridDim.x * blockDim.x;
-  uint32_t iters = (n + stride - 1) / stride;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  for (uint32_t it = 0; it < iters; it++, i += stride) {
-    bool active = i < n;
-    uint4 st = make_uint4(0, 0, 0, 0);
-    V3 thr = v3(0.f), rad = v3(0.f), P = v3(0.f), dcont = v3(0.f);
-    bool ended = false;
-    float code = 0.f, tm = 0.f;
-    if (active) {
-      st = W.sh.st[i];
-      const float4 t4 = W.sh.thr[i];
-      thr = f4xyz(t4);
-      tm = t4.w;
-      float4 r4 = W.sh.rad[i];
-      rad = f4xyz(r4);
-      code = r4.w;
-      float4 Wi4 = W.sh.Wi[i], C4 = W.sh.C[i], Wo4 = W.sh.Wo[i];
-      P = f4xyz(W.sh.P[i]);
-      if (Wi4.w == 0.f) {  // unoccluded
-        rad += f4xyz(C4);
-        // the vertex that just recorded a guide sample: its NEE light did
-        // not come along the recorded direction
-        int ci = (int)code;
-        if (ci & 1) W.grec[2u * (st.y / W.grec_stride) + (uint32_t)(ci >> 1) - 1u].pad[0] +=
-            lum3(f4xyz(C4));
-      }
-      dcont = f4xyz(Wo4);
-      ended = Wo4.w != 0.f;
-      if (ended) {
-        finalize_path(W, st.y, rad);
-        if (code != 0.f) guide_end(W, st.y, code, rad);
-      }
-    }
-    path_push(W, c, st, thr, rad, P, dcont, active && !ended, tm, (float)(((int)code >> 1) * 2));
-  }
-}
-
 // Queue bookkeeping after an iteration.  With use_cond (the iteration loop
 // is a graph conditional node) it also decides whether the loop goes on:
 // not once the chunk has drained, an error was flagged, or the chunk's
@@ -415,12 +368,15 @@ __global__ void k_advance(WaveState W, const WaveCtl* __restrict__ ctlp, int use
   WaveCounters& c = *W.ctr;
   const WaveCtl& ctl = *ctlp;
   uint32_t n_gen = gen_count(c, ctl, (uint32_t)W.slots);
-  c.ext_rays += c.n_cur + n_gen;
+  c.ext_rays += c.n_cur + n_gen - c.n_wait;
   c.shadow_rays += c.n_shadow;
   c.next_path += n_gen;
   c.drained = n_gen ? 1u : c.drained + 1u;
   c.n_cur = c.n_next;
   c.n_next = 0;
+  c.n_wait = c.n_wait_next;
+  c.n_wait_next = 0;
+  c.n_occ = c.n_shadow;
   c.n_shadow = 0;
   c.ray_next[0] = 0;
   c.ray_next[1] = 0;
@@ -466,7 +422,8 @@ __global__ void k_batch_begin(WaveState W, WaveCtl* ctl, const BatchChunk* __res
   ctl->pixels = ch.pixels;
   c.n_cur = 0;
   c.n_next = 0;
-  c.n_shadow = 0;
+  c.n_shadow = c.n_occ = 0;
+  c.n_wait = c.n_wait_next = 0;
   c.parity = 0;
   c.iter = 0;
   c.next_path = 0;
@@ -778,7 +735,7 @@ static bool shadow_rays(const LaunchCfg& lc, int mode) {
 }
 
 int iteration_kernels(const LaunchCfg& lc, int mode, bool guide) {
-  return 4 + (shadow_rays(lc, mode) ? 2 : 0) + (mode == 1 && guide ? 2 : 0);
+  return 4 + (mode != 1 && shadow_rays(lc, mode) ? 2 : 0) + (mode == 1 && guide ? 2 : 0);
 }
 
 void launch_chunk_begin(const WaveState& W, WaveCtl* ctl, const WaveCtl& v, bool first,
@@ -811,23 +768,19 @@ static void launch_iteration_t(const DevScene& S, const WaveState& W, const Wave
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
   k_generate<BATCH><<<sg, sb, 0, st>>>(S, W, ctl, br);
   if (ev) cudaEventRecordWithFlags(ev[1], st, cudaEventRecordExternal);
-  launch_trace(TRACE_EXT, counters, S, W, ctl, max_stack, brp, lc, st);
+  const bool nee = shadow_rays(lc, mode);
+  launch_trace(mode == 1 && nee ? TRACE_BOTH : TRACE_EXT, counters, S, W, ctl, max_stack, brp, lc,
+               st);
   if (ev) cudaEventRecordWithFlags(ev[2], st, cudaEventRecordExternal);
   if (mode == 1 && gi) launch_guide_infer(S, W, ctl, *gi, 2 * num_sms(), st);
   if (lc.tex)
     launch_shade<BATCH, true>(S, W, ctl, br, mode, gi != nullptr, lc.sort, tgs, sg, sb, st);
   else
     launch_shade<BATCH, false>(S, W, ctl, br, mode, gi != nullptr, lc.sort, tgs, sg, sb, st);
-  const bool nee = shadow_rays(lc, mode);
   if (ev) cudaEventRecordWithFlags(ev[3], st, cudaEventRecordExternal);
-  if (nee)
-    launch_trace(mode == 1 ? TRACE_OCCLUDED : TRACE_SHADOW, counters, S, W, ctl, max_stack, brp,
-                 lc, st);
+  if (nee && mode != 1) launch_trace(TRACE_SHADOW, counters, S, W, ctl, max_stack, brp, lc, st);
   if (ev) cudaEventRecordWithFlags(ev[4], st, cudaEventRecordExternal);
-  if (nee && mode == 1)
-    k_finish_c<<<sg, sb, 0, st>>>(S, W, ctl);
-  else if (nee)
-    k_finish<BATCH><<<sg, sb, 0, st>>>(S, W, ctl, br);
+  if (nee && mode != 1) k_finish<BATCH><<<sg, sb, 0, st>>>(S, W, ctl, br);
   k_advance<<<1, 1, 0, st>>>(W, ctl, use_cond ? 1 : 0, (cudaGraphConditionalHandle)cond);
   if (ev) cudaEventRecordWithFlags(ev[5], st, cudaEventRecordExternal);
 }

@@ -451,6 +451,17 @@ __device__ __forceinline__ void guide_end(const WaveState& W, uint32_t pid, floa
   }
 }
 
+// The occlusion ray of a path's NEE term has been traced: adds the term if
+// nothing was hit.  A vertex that just recorded a guide sample: its NEE light
+// did not come along the recorded direction.
+__device__ __forceinline__ void nee_arrived(const WaveState& W, float occluded, float4 C,
+                                            uint32_t pid, int word, V3& rad) {
+  if (occluded != 0.f) return;
+  rad += f4xyz(C);
+  if (word & 1)
+    W.grec[2u * (pid / W.grec_stride) + (uint32_t)((word & 6) >> 1) - 1u].pad[0] += lum3(f4xyz(C));
+}
+
 // ------------------------------------------------- consistent mode --------
 // What a bounce of the consistent integrator leaves: its shadow ray (P, Wi,
 // tmax) with the NEE term C that an unoccluded ray adds to the radiance, and
@@ -463,8 +474,8 @@ struct BounceC {
 
 // One bounce of the consistent integrator (the oracle's color_c): emission
 // with MIS at hits and misses, NEE over lights + environment, BSDF
-// continuation, Russian roulette.  The NEE term waits for its shadow ray in
-// the shadow buffer together with the already-sampled continuation.  With
+// continuation, Russian roulette.  The NEE term waits for its shadow ray while
+// the path goes on.  With
 // GUIDE the continuation is drawn from alpha * guide + (1 - alpha) * BSDF
 // (the guide of this position from k_guide_infer) and that mixture density is
 // the MIS partner of NEE and of emitter hits at the next vertex.  i: the path's

@@ -158,17 +158,24 @@ __device__ __forceinline__ void run_path(const DevScene& S0, const WaveState& W,
   finalize_path(W, st.y, col);
 }
 
-// Consistent mode: the same; code is the guide-record word (its bounces are
-// past the guided depth).
+// Consistent mode: the same; word holds the guide-record word (the bounces left
+// are past the guided depth) and whether the NEE term nee_c of the previous
+// bounce still waits for its occlusion ray (nee_wi).  tmax 0: it is all that
+// the path waits for.
 template <bool BATCH>
 __device__ __forceinline__ void run_path_c(const DevScene& S0, const WaveState& W,
                                            const WaveCtl& ctl, const BatchRefs& br, V3 o, V3 d,
-                                           float tmin, float tmax, V3 thr, V3 rad, float code,
-                                           float tm, uint4 st, LaneTrace& lt, uint32_t& ext,
-                                           uint32_t& shadow) {
+                                           float tmin, float tmax, V3 thr, V3 rad, int word,
+                                           float4 nee_wi, float4 nee_c, float tm, uint4 st,
+                                           LaneTrace& lt, uint32_t& ext, uint32_t& shadow) {
   const DevScene& S = path_scene<BATCH>(S0, br, st.z);
   const PathCtl pc = path_ctl<BATCH>(ctl, br, st.z);
-  while (true) {
+  if (word & PT_CODE_PENDING) {
+    const bool hit =
+        (uint32_t)lane_trace<true>(S, o, f4xyz(nee_wi), 1e-3f, nee_c.w, tm, lt) != PT_NO_HIT;
+    nee_arrived(W, hit ? 1.f : 0.f, nee_c, st.y, word, rad);
+  }
+  while (tmax != 0.f) {
     ext++;
     const float4 hit = lane_hit(S, o, d, tmin, tmax, tm, lt);
     BounceC b;
@@ -186,7 +193,7 @@ __device__ __forceinline__ void run_path_c(const DevScene& S0, const WaveState& 
     tmax = PT_RAY_TMAX;
   }
   finalize_path(W, st.y, rad);
-  guide_end(W, st.y, code, rad);
+  guide_end(W, st.y, (float)(word & 6), rad);
 }
 
 template <int MODE, bool BATCH>
@@ -214,7 +221,9 @@ __global__ void __launch_bounds__(PT_TAIL_BLOCK)
     const uint32_t j = base + (uint32_t)lane;
     if ((uint32_t)lane < lanes && j < total) {
       V3 o, d, thr = v3(1.f), rad = v3(0.f);
-      float tmin = 1e-6f, tmax = PT_RAY_TMAX, tm, code = 0.f;
+      float tmin = 1e-6f, tmax = PT_RAY_TMAX, tm;
+      int word = 0;
+      float4 nee_wi = make_float4(0.f, 0.f, 0.f, 0.f), nee_c = nee_wi;
       uint4 st;
       if (j < c.n_cur) {
         const float4 o4 = pb.ray_o[j], d4 = pb.ray_d[j], t4 = pb.thr[j], r4 = pb.rad[j];
@@ -225,7 +234,11 @@ __global__ void __launch_bounds__(PT_TAIL_BLOCK)
         thr = f4xyz(t4);
         tm = t4.w;
         rad = f4xyz(r4);
-        code = r4.w;
+        word = (int)r4.w;
+        if (MODE == 1 && (word & PT_CODE_PENDING)) {
+          nee_wi = W.nee[c.parity].Wi[j];
+          nee_c = W.nee[c.parity].C[j];
+        }
         st = pb.st[j];
       } else {
         const NewPath np =
@@ -236,8 +249,8 @@ __global__ void __launch_bounds__(PT_TAIL_BLOCK)
         st = np.st;
       }
       if (MODE == 1)
-        run_path_c<BATCH>(S0, W, ctl, br, o, d, tmin, tmax, thr, rad, code, tm, st, lt, ext,
-                          shadow);
+        run_path_c<BATCH>(S0, W, ctl, br, o, d, tmin, tmax, thr, rad, word, nee_wi, nee_c, tm, st,
+                          lt, ext, shadow);
       else
         run_path<BATCH>(S0, W, ctl, br, o, d, tmin, tmax, thr, rad, tm, st, lt, ext, shadow);
     }
@@ -261,7 +274,7 @@ __global__ void k_tail_end(WaveState W, const WaveCtl* __restrict__ ctlp) {
   WaveCounters& c = *W.ctr;
   if (!tail_ready(c, *ctlp)) return;
   c.next_path = ctlp->chunk_paths;
-  c.n_cur = 0;
+  c.n_cur = c.n_wait = c.n_occ = 0;
 }
 
 constexpr int kMaxSmem = 200 * 1024;  // the same for every context: a function attribute is shared

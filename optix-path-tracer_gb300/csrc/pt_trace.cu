@@ -2,7 +2,8 @@
  * pt_trace.cu - BVH8 traversal kernels for sm_103a: the closest hit of
  * extension rays (replaces rtTrace into the scene's top object), the shadow
  * ray of Direct_Light (programs/hit.cu:16-24 under the closest-hit rule), the
- * occlusion rays of the consistent mode and first-hit queries.
+ * occlusion rays of the consistent mode (in one launch with the extension
+ * rays) and first-hit queries.
  *
  * The BVH8 (csrc/bvh_gpu.cu, csrc/bvh_host.cpp) stores 80-byte nodes with
  * 8-bit quantised child boxes and 48-byte primitive records; rays come from
@@ -70,9 +71,10 @@ struct FirstHitOut {
 // scene index is in the path state word st.z).  MOTION: the scene has moving
 // spheres, so each ray carries its path's time (other scenes do without).
 template <int MODE, bool COUNT, bool BATCH, bool MOTION>
-__global__ void __maxnreg__(PT_TRACE_MAXREG)
-    k_trace_t(DevScene S, WaveState W, const WaveCtl* __restrict__ ctlp, int max_stack,
-              FirstHitOut fo, BatchRefs br, int refetch) {
+__device__ __forceinline__ void trace_rays(const DevScene& S, const WaveState& W,
+                                           const WaveCtl* __restrict__ ctlp, int max_stack,
+                                           const FirstHitOut& fo, const BatchRefs& br,
+                                           int refetch) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   WarpShared& ws = ((WarpShared*)smem)[threadIdx.x >> 5];
@@ -83,13 +85,15 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
 
   uint32_t n;
   WaveCounters c;
+  if (MODE != TRACE_FIRST) c = *W.ctr;
   constexpr bool consistent = MODE == TRACE_OCCLUDED;
   constexpr bool SHADOWRAY = MODE == TRACE_SHADOW || MODE == TRACE_OCCLUDED;
   if (MODE == TRACE_EXT) {
-    c = *W.ctr;
     n = c.n_cur + gen_count(c, *ctlp, (uint32_t)W.slots);
-  } else if (SHADOWRAY) {
-    n = W.ctr->n_shadow;
+  } else if (MODE == TRACE_OCCLUDED) {
+    n = c.n_occ;
+  } else if (MODE == TRACE_SHADOW) {
+    n = c.n_shadow;
   } else {
     n = (uint32_t)fo.width * (uint32_t)fo.height;
   }
@@ -104,7 +108,7 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
   // per-lane ray state (the direction and tmax of a lane's ray live in the
   // warp's shared copy, ws.rd[lane]: the node tests need only o, tmin and
   // the reciprocal direction)
-  const uint32_t parity = MODE == TRACE_EXT ? c.parity : 0u;
+  const uint32_t parity = MODE == TRACE_EXT || MODE == TRACE_OCCLUDED ? c.parity : 0u;
   BoxRay ray;
   V3& o = ray.o;
   float& tmin = ray.tmin;
@@ -124,11 +128,17 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
       d = f4xyz(rdv);
       tmin = ro.w;
       tmax = rdv.w;
-    } else if (SHADOWRAY) {
+    } else if (MODE == TRACE_OCCLUDED) {
+      // from the point where its path goes on (i: the path's position)
+      o = f4xyz(W.path[parity].ray_o[i]);
+      d = f4xyz(W.nee[parity].Wi[i]);
+      tmin = 1e-3f;
+      tmax = W.nee[parity].C[i].w;
+    } else if (MODE == TRACE_SHADOW) {
       o = f4xyz(W.sh.P[i]);
       d = f4xyz(W.sh.Wi[i]);
       tmin = 1e-3f;
-      tmax = consistent ? W.sh.C[i].w : PT_RAY_TMAX;
+      tmax = PT_RAY_TMAX;
     } else {
       uint32_t x = i % (uint32_t)fo.width, y = i / (uint32_t)fo.width;
       uint32_t seed = tea64((uint32_t)fo.width * y + x, (uint32_t)fo.frame);
@@ -153,11 +163,12 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
         h = make_float4(tbest, bu, bv, __uint_as_float(leaf));
       }
       W.hit[i] = h;
-    } else if (SHADOWRAY) {
+    } else if (MODE == TRACE_OCCLUDED) {
+      // anything before the light
+      W.nee[parity].Wi[i].w = best_id != PT_NO_HIT ? 1.f : 0.f;
+    } else if (MODE == TRACE_SHADOW) {
       bool occluded = true;
-      if (consistent) {
-        occluded = best_id != PT_NO_HIT;  // anything before the light
-      } else if (best_id != PT_NO_HIT) {
+      if (best_id != PT_NO_HIT) {
         PrimRec p = load_prim(S.prims, __ldg(S.leaf_of_id + best_id));
         bool is_light = S.mats[prim_material(p)].type == PT_MAT_DIFFUSE_LIGHT;
         occluded = !(is_light && dot(f4xyz(W.sh.N[i]), d) > 0.f);
@@ -195,12 +206,14 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
   auto fetch = [&]() {
     // a ray with a NaN in its origin or direction hits nothing (every
     // primitive test fails or yields a NaN distance, which never wins the
-    // closest-hit minimum), and neither does any ray of an empty scene: both
-    // end here, without a traversal (a NaN ray would pass every box test)
+    // closest-hit minimum), and neither does any ray of an empty scene: both end
+    // here, without a traversal (a NaN ray would pass every box test)
     V3 d;
     float tmax;
     load_ray(d, tmax);
-    if (nan_ray(o, d) || S.num_prims == 0) {
+    // here, and so does an extension ray whose path has ended (tmax 0: it only
+    // waits for its NEE term)
+    if (nan_ray(o, d) || S.num_prims == 0 || (MODE == TRACE_EXT && tmax == 0.f)) {
       best_id = PT_NO_HIT;
       tbest = tmax;
       finish(d, tmax);
@@ -220,10 +233,10 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
     best_id = PT_NO_HIT;
     ws.best[lane] = ((unsigned long long)__float_as_uint(tmax) << 32) | 0xffffffffull;
     if (MOTION && MODE != TRACE_FIRST)  // the path's time rides in throughput.w
-      ws.tm[lane] = MODE == TRACE_EXT ? W.path[parity].thr[i].w : W.sh.thr[i].w;
+      ws.tm[lane] = MODE == TRACE_SHADOW ? W.sh.thr[i].w : W.path[parity].thr[i].w;
     cur = S.root;
     if (BATCH) {
-      uint32_t z = MODE == TRACE_EXT ? W.path[parity].st[i].z : W.sh.st[i].z;
+      uint32_t z = MODE == TRACE_SHADOW ? W.sh.st[i].z : W.path[parity].st[i].z;
       cur = __ldg(br.roots + (z >> PT_ST_SCENE_SHIFT));
     }
     sp = 0;
@@ -255,7 +268,10 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
       }
       if (idle) {
         idle = false;
-        if (i < n) fetch();
+        if (i < n) {
+          if (MODE == TRACE_OCCLUDED) i = W.nee[parity].queue[i];
+          fetch();
+        }
       }
       busy = __ballot_sync(0xffffffffu, active);
       if (!busy) {
@@ -444,6 +460,24 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
   }
 }
 
+template <int MODE, bool COUNT, bool BATCH, bool MOTION>
+__global__ void __maxnreg__(PT_TRACE_MAXREG)
+    k_trace_t(DevScene S, WaveState W, const WaveCtl* __restrict__ ctlp, int max_stack,
+              FirstHitOut fo, BatchRefs br, int refetch) {
+  if (MODE == TRACE_BOTH) {
+    // a warp that finds no extension ray left goes on to the occlusion rays, so
+    // the one kind fills the SMs while the longest rays of the other end.  Two
+    // launches, with a finishing kernel behind the second, took 1052 us per
+    // 1280x720 terrain frame and 80.0 ms per 64 frames at 1920x1080; this one,
+    // with the path state passed on once instead of parked, 973 us and 76.9 ms
+    // (GB300)
+    trace_rays<TRACE_EXT, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch);
+    __syncwarp();
+    trace_rays<TRACE_OCCLUDED, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch);
+  } else {
+    trace_rays<MODE, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch);
+  }
+}
 
 // ------------------------------------------------------- host launchers ---
 namespace pt {
@@ -498,10 +532,10 @@ cudaError_t set_trace_smem() {
     return e;
   if ((e = smem_attr_mode<TRACE_EXT, false>(optin)) != cudaSuccess) return e;
   if ((e = smem_attr_mode<TRACE_SHADOW, false>(optin)) != cudaSuccess) return e;
-  if ((e = smem_attr_mode<TRACE_OCCLUDED, false>(optin)) != cudaSuccess) return e;
+  if ((e = smem_attr_mode<TRACE_BOTH, false>(optin)) != cudaSuccess) return e;
   if ((e = smem_attr_mode<TRACE_EXT, true>(optin)) != cudaSuccess) return e;
   if ((e = smem_attr_mode<TRACE_SHADOW, true>(optin)) != cudaSuccess) return e;
-  if ((e = smem_attr_mode<TRACE_OCCLUDED, true>(optin)) != cudaSuccess) return e;
+  if ((e = smem_attr_mode<TRACE_BOTH, true>(optin)) != cudaSuccess) return e;
   if ((e = smem_attr(k_trace_t<TRACE_FIRST, false, false, false>, optin)) != cudaSuccess) return e;
   if ((e = smem_attr(k_trace_t<TRACE_FIRST, false, false, true>, optin)) != cudaSuccess) return e;
   if (dev >= 0 && dev < kMaxDev) g_smem_set[dev] = true;
@@ -530,7 +564,7 @@ static void launch_kind(int mode, bool counters, const DevScene& S, const WaveSt
   else if (mode == TRACE_SHADOW)
     launch_mode<TRACE_SHADOW, BATCH, MOTION>(counters, S, W, ctl, max_stack, br, lc, smem, st);
   else
-    launch_mode<TRACE_OCCLUDED, BATCH, MOTION>(counters, S, W, ctl, max_stack, br, lc, smem, st);
+    launch_mode<TRACE_BOTH, BATCH, MOTION>(counters, S, W, ctl, max_stack, br, lc, smem, st);
 }
 
 void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W,
