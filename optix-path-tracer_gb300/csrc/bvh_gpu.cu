@@ -6,21 +6,25 @@
  *  2. k_morton      30-bit Morton code of the centroid (10 bits per axis, one
  *                   scale for all axes: the centroid box's longest side)
  *  3. radix sort    CUB DeviceRadixSort over (code, primitive) pairs
- *  4. k_karras      binary radix tree, Karras, "Maximizing Parallelism in the
- *                   Construction of BVHs, Octrees, and k-d Trees", HPG 2012
- *  5. k_bottom_up   bounds and SAH cost bottom-up (atomic arrival counters);
- *                   at every node with >= 7 primitives below it the treelet of
- *                   up to 7 leaves is rebuilt optimally for SAH by dynamic
- *                   programming over leaf subsets (Karras & Aila, "Fast
- *                   Parallel Construction of High-Quality BVHs", HPG 2013),
- *                   one warp per treelet; a first pass without restructuring,
- *                   then one per treelet round
- *  6. k_collapse    one launch per level: each binary node becomes a wide
- *                   node by expanding its largest child until 8 children
- *                   (or the requested width);
+ *  4. k_ploc        (triangle meshes) binary tree by locally-ordered clustering
+ *                   and the cost of every subtree as slots of wide nodes, in
+ *                   one launch (H-PLOC, HPG 2024)
+ *     k_karras      (other scenes) binary radix tree, Karras, "Maximizing
+ *                   Parallelism in the Construction of BVHs, Octrees, and k-d
+ *                   Trees", HPG 2012; then k_bottom_up: bounds and SAH cost
+ *                   bottom-up (atomic arrival counters); at every node with
+ *                   >= 7 primitives below it the treelet of up to 7 leaves is
+ *                   rebuilt optimally for SAH by dynamic programming over leaf
+ *                   subsets (Karras & Aila, "Fast Parallel Construction of
+ *                   High-Quality BVHs", HPG 2013), one warp per treelet; a
+ *                   first pass without restructuring, then one per treelet
+ *                   round
+ *  5. k_collapse    one launch per level: each binary node becomes a wide
+ *                   node, cut by the costs of k_ploc, or by expanding its
+ *                   largest child until 8 children (or the requested width);
  *                   subtrees of <= 3 primitives become leaf slots; child
  *                   boxes are quantised to 8 bits (node format: pt_types.h)
- *  7. k_check_*     structural check of the finished tree before any
+ *  6. k_check_*     structural check of the finished tree before any
  *                   traversal runs on it (check_node8 on every node, every
  *                   leaf position covered once, leaf_of_id a permutation)
  * The result is order independent for rendering (closest hit is the minimum
@@ -35,9 +39,14 @@
 #include "pt_device.cuh"
 #include "pt_internal.h"
 
+#ifndef PT_TREELET_ROUNDS
+#define PT_TREELET_ROUNDS 2  /* SAH treelet restructuring passes */
+#endif
+
 namespace {
 
 constexpr uint32_t LEAF_BIT = 0x80000000u;
+constexpr uint32_t NONE = 0xffffffffu;
 constexpr float C_INNER = 1.2f, C_TRI = 1.0f;
 
 struct GBox {
@@ -69,7 +78,7 @@ __device__ __forceinline__ GBox box_load(const float4* lo, const float4* hi, uin
   return r;
 }
 // Loads of tree data that other threads write during the same kernel
-// (k_bottom_up): L2 only (ld.global.cg), so no stale L1 line is read.
+// (k_ploc, k_bottom_up): L2 only (ld.global.cg), so no stale L1 line is read.
 __device__ __forceinline__ GBox box_load_cg(const float4* lo, const float4* hi, uint32_t i) {
   float4 a = __ldcg(lo + i), b = __ldcg(hi + i);
   GBox r;
@@ -82,13 +91,12 @@ __device__ __forceinline__ GBox box_load_cg(const float4* lo, const float4* hi, 
 __global__ void k_bounds(const float4* __restrict__ rec, const float4* __restrict__ xforms,
                          uint32_t n, float cam_t0, float cam_t1, float4* lo, float4* hi,
                          unsigned int* cbox) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   GBox c;
   for (int k = 0; k < 3; k++) {
     c.lo[k] = 3.0e38f;
     c.hi[k] = -3.0e38f;
   }
-  if (i < n) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float4 r0 = rec[3 * i], r1 = rec[3 * i + 1], r2 = rec[3 * i + 2];
     uint32_t tag = __float_as_uint(r0.w);
     int type = tag & 3, axis = (tag >> 2) & 3, xf = (int)(tag >> 8) - 1;
@@ -146,9 +154,15 @@ __global__ void k_bounds(const float4* __restrict__ rec, const float4* __restric
     }
     lo[i] = make_float4(b.lo[0], b.lo[1], b.lo[2], 0.f);
     hi[i] = make_float4(b.hi[0], b.hi[1], b.hi[2], 0.f);
-    for (int a = 0; a < 3; a++) c.lo[a] = c.hi[a] = 0.5f * (b.lo[a] + b.hi[a]);
+    for (int a = 0; a < 3; a++) {
+      const float m = 0.5f * (b.lo[a] + b.hi[a]);
+      c.lo[a] = fminf(c.lo[a], m);
+      c.hi[a] = fmaxf(c.hi[a], m);
+    }
   }
-  // centroid bounds: block reduction, then ordered-int atomics
+  // centroid bounds: warp reductions, then ordered-int atomics (the grid is a
+  // few blocks per SM: an atomic per warp of all primitives took 0.28 ms for
+  // 2.1 M)
   for (int a = 0; a < 3; a++) {
     for (int o = 16; o > 0; o >>= 1) {
       c.lo[a] = fminf(c.lo[a], __shfl_xor_sync(0xffffffffu, c.lo[a], o));
@@ -203,6 +217,259 @@ __global__ void k_morton(const float4* __restrict__ lo, const float4* __restrict
   vals[i] = i;
 }
 
+// ---------------------------------------------------------- binary tree ----
+// Internal nodes 0..n-2; references with LEAF_BIT are leaves in Morton order.
+struct Tree {
+  uint32_t *left, *right;
+  uint32_t *parent_int, *parent_leaf, *flags;  // treelet builder
+  float4 *ilo, *ihi;        // internal bounds; ilo.w = SAH cost (treelet builder),
+                            // ihi.w = primitive count
+  const float4 *llo, *lhi;  // leaf bounds (sorted order)
+  float4* cost;             // 2 per node, of nodes that are clusters between merges: WideCost
+  uint32_t* plan;           // per node: how it is cut into wide nodes (wide_cost); null: by area
+  uint32_t root;
+};
+
+// Cost of a subtree as at most i + 1 slots of a wide node, by dynamic
+// programming over the binary tree (Ylitie, Karras & Laine, HPG 2017, sec. 3):
+// one slot holds a leaf of up to 3 primitives or a wide node of its own, more
+// slots are shared between the two children.
+#ifndef PT_COST_NODE
+#define PT_COST_NODE 1.0f
+#endif
+#ifndef PT_COST_PRIM
+#define PT_COST_PRIM 0.3f
+#endif
+struct WideCost {
+  float c[7];
+};
+
+// The costs of a node from its children's and its plan: bits 3j..3j+2 (j =
+// 0..6): the left child's slots when the node has j + 2 (0: it takes fewer);
+// bit 21: as one slot it is a leaf.
+__device__ __forceinline__ WideCost wide_cost(const WideCost& l, const WideCost& r, float area,
+                                              float count, int width, uint32_t& plan) {
+  WideCost o;
+  float dist[7];
+  plan = 0;
+#pragma unroll
+  for (int j = 2; j <= 8; j++) {
+    float best = 3.0e38f;
+    uint32_t k = 1;
+#pragma unroll
+    for (int i = 1; i < j; i++) {
+      if (j - i > 7 || i > 7) continue;
+      const float v = l.c[i - 1] + r.c[j - i - 1];
+      if (v < best) {
+        best = v;
+        k = (uint32_t)i;
+      }
+    }
+    dist[j - 2] = best;
+    plan |= k << (3 * (j - 2));
+  }
+  float whole = dist[6];
+#pragma unroll
+  for (int j = 2; j < 8; j++)
+    if (j == width) whole = dist[j - 2];
+  o.c[0] = PT_COST_NODE * area + whole;
+  if (count <= 3.f && PT_COST_PRIM * area * count <= o.c[0]) {
+    o.c[0] = PT_COST_PRIM * area * count;
+    plan |= 1u << 21;
+  }
+#pragma unroll
+  for (int j = 2; j <= 7; j++) {
+    o.c[j - 1] = dist[j - 2];
+    if (j == width) continue;  // a full node is always shared out
+    if (o.c[j - 2] <= o.c[j - 1]) {
+      o.c[j - 1] = o.c[j - 2];
+      plan &= ~(7u << (3 * (j - 2)));
+    }
+  }
+  return o;
+}
+
+__device__ __forceinline__ GBox ref_box(const Tree& T, uint32_t r) {
+  return (r & LEAF_BIT) ? box_load(T.llo, T.lhi, r & ~LEAF_BIT) : box_load(T.ilo, T.ihi, r);
+}
+__device__ __forceinline__ float ref_count(const Tree& T, uint32_t r) {
+  return (r & LEAF_BIT) ? 1.f : T.ihi[r].w;
+}
+
+// Where the Morton codes of positions i and i + 1 differ (equal codes: where
+// the positions do); smaller = closer.
+__device__ __forceinline__ unsigned long long code_gap(const uint32_t* __restrict__ keys, uint32_t i) {
+  const unsigned long long a = ((unsigned long long)keys[i] << 32) | i;
+  const unsigned long long b = ((unsigned long long)keys[i + 1] << 32) | (i + 1);
+  return a ^ b;
+}
+
+// Clusters kept per code range, and places searched on each side.  The radius
+// is small: with 1 / 2 / 3 / 4 / 8 / 16 a 2.1 M-triangle terrain took 7.28 /
+// 7.30 / 7.26 / 7.43 / 7.48 / - node fetches per ray, one of 0.5 M 6.60 /
+// 6.59 / 6.79 / 6.86 / 7.16 / - (greedy collapse, 8 / 16: 7.66 / 8.03 and
+// 7.45 / 7.54): on regular meshes the Morton order already is the good tree.
+constexpr uint32_t PLOC_KEEP = 16, PLOC_RADIUS = 2;
+
+// A lane's cluster while a warp merges.
+struct Cluster {
+  uint32_t ref;
+  GBox box;
+  float count;
+  WideCost w;
+};
+
+__device__ __forceinline__ Cluster shfl_cluster(const Cluster& c, int src) {
+  Cluster r;
+  r.ref = __shfl_sync(0xffffffffu, c.ref, src);
+  for (int a = 0; a < 3; a++) {
+    r.box.lo[a] = __shfl_sync(0xffffffffu, c.box.lo[a], src);
+    r.box.hi[a] = __shfl_sync(0xffffffffu, c.box.hi[a], src);
+  }
+  r.count = __shfl_sync(0xffffffffu, c.count, src);
+  for (int k = 0; k < 7; k++) r.w.c[k] = __shfl_sync(0xffffffffu, c.w.c[k], src);
+  return r;
+}
+
+// Merges the clusters of the code ranges [L, split) and [split, R] (at most
+// PLOC_KEEP each, at the front of their range's entries of `cluster`) until at
+// most PLOC_KEEP are left (one at the root): each cluster finds the neighbour
+// within PLOC_RADIUS places whose union with it has the least area, and
+// mutual nearest neighbours become one node.  All lanes call it together.
+__device__ void ploc_merge(const Tree& T, uint32_t* cluster, uint32_t* counter, uint32_t L,
+                           uint32_t split, uint32_t R, bool top, int width, uint8_t* map, int lane) {
+  const uint32_t nl = min(PLOC_KEEP, split - L), nr = min(PLOC_KEEP, R + 1 - split);
+  Cluster c;
+  c.ref = NONE;
+  if ((uint32_t)lane < nl) c.ref = __ldcg(cluster + L + lane);
+  if ((uint32_t)lane >= PLOC_KEEP && (uint32_t)lane - PLOC_KEEP < nr)
+    c.ref = __ldcg(cluster + split + (lane - PLOC_KEEP));
+  const uint32_t valid = __ballot_sync(0xffffffffu, c.ref != NONE);
+  const int cl = __popc(valid & ((1u << PLOC_KEEP) - 1u));
+  int num = __popc(valid);
+  c.ref = __shfl_sync(0xffffffffu, c.ref, lane < cl ? lane : (lane - cl + (int)PLOC_KEEP) & 31);
+  if (lane >= num) c.ref = NONE;
+  c.count = 1.f;
+  for (int a = 0; a < 3; a++) c.box.lo[a] = c.box.hi[a] = 0.f;
+  for (int k = 0; k < 7; k++) c.w.c[k] = 0.f;
+  if (c.ref != NONE) {
+    if (c.ref & LEAF_BIT) {
+      c.box = box_load(T.llo, T.lhi, c.ref & ~LEAF_BIT);
+      for (int k = 0; k < 7; k++) c.w.c[k] = PT_COST_PRIM * box_area(c.box);
+    } else {
+      c.box = box_load_cg(T.ilo, T.ihi, c.ref);
+      const float4 w0 = __ldcg(T.cost + 2 * (size_t)c.ref), w1 = __ldcg(T.cost + 2 * (size_t)c.ref + 1);
+      c.w.c[0] = w0.x; c.w.c[1] = w0.y; c.w.c[2] = w0.z; c.w.c[3] = w0.w;
+      c.w.c[4] = w1.x; c.w.c[5] = w1.y; c.w.c[6] = w1.z;
+      c.count = w1.w;
+    }
+  }
+  const int goal = top ? 1 : (int)PLOC_KEEP;
+  for (int it = 0; it < 32 && num > goal; it++) {  // each step merges a pair at least
+    // nearest neighbour: the area's bits (it is not negative) with the lane in
+    // the low 5; the pair of least (area, lanes) is always mutual
+    uint32_t best = NONE;
+#pragma unroll
+    for (int r = 1; r <= (int)PLOC_RADIUS; r++) {
+      GBox o;
+      for (int a = 0; a < 3; a++) {
+        o.lo[a] = __shfl_down_sync(0xffffffffu, c.box.lo[a], r);
+        o.hi[a] = __shfl_down_sync(0xffffffffu, c.box.hi[a], r);
+      }
+      uint32_t d = NONE;
+      if (lane + r < num) {
+        d = __float_as_uint(fmaxf(box_area(box_union(c.box, o)), 0.f)) & ~31u;
+        best = min(best, d | (uint32_t)(lane + r));
+      }
+      const uint32_t up = __shfl_up_sync(0xffffffffu, d, r);
+      if (lane >= r && lane < num) best = min(best, up | (uint32_t)(lane - r));
+    }
+    const int nn = lane < num ? (int)(best & 31u) : lane;
+    const int back = __shfl_sync(0xffffffffu, nn, nn);  // every lane takes part
+    const bool mutual = lane < num && back == lane;
+    const bool merges = mutual && lane < nn;
+    const uint32_t mm = __ballot_sync(0xffffffffu, merges);
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(counter, (uint32_t)__popc(mm));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const Cluster o = shfl_cluster(c, nn);
+    if (merges) {
+      const uint32_t node = base + (uint32_t)__popc(mm & ((1u << lane) - 1u));
+      T.left[node] = c.ref;
+      T.right[node] = o.ref;
+      c.box = box_union(c.box, o.box);
+      c.count += o.count;
+      box_store(T.ilo, T.ihi, node, c.box, 0.f, c.count);
+      uint32_t plan;
+      c.w = wide_cost(c.w, o.w, box_area(c.box), c.count, width, plan);
+      T.plan[node] = plan;
+      c.ref = node;
+    }
+    const bool keep = lane < num && !(mutual && lane > nn);
+    const uint32_t km = __ballot_sync(0xffffffffu, keep);
+    if (keep) map[__popc(km & ((1u << lane) - 1u))] = (uint8_t)lane;
+    __syncwarp();
+    num = __popc(km);
+    c = shfl_cluster(c, lane < num ? map[lane] : lane);
+    __syncwarp();
+    if (lane >= num) c.ref = NONE;
+  }
+  if ((uint32_t)lane < PLOC_KEEP && L + lane <= R) {
+    cluster[L + lane] = c.ref;
+    if (!(c.ref & LEAF_BIT)) {  // NONE has the bit too
+      T.cost[2 * (size_t)c.ref] = make_float4(c.w.c[0], c.w.c[1], c.w.c[2], c.w.c[3]);
+      T.cost[2 * (size_t)c.ref + 1] = make_float4(c.w.c[4], c.w.c[5], c.w.c[6], c.count);
+    }
+  }
+  __threadfence();  // nodes and entries before any lane of this warp reports the range upward
+  __syncwarp();
+}
+
+// Bottom-up over the Morton order (H-PLOC: Benthin, Meister, Barczak, Mehalwal,
+// Tsakok & Kensler, "H-PLOC: Hierarchical Parallel Locally-Ordered Clustering
+// for Bounding Volume Hierarchy Construction", HPG 2024): a thread's code
+// range joins its sibling's (the second to arrive goes on), and ranges of more
+// than PLOC_KEEP primitives are merged to PLOC_KEEP clusters by the whole
+// warp.  ends: per gap between codes, the outer end of the range that arrived
+// first (NONE before).  Launched with 256 threads.
+__global__ void __launch_bounds__(256) k_ploc(Tree T, const uint32_t* __restrict__ keys, uint32_t n,
+                                              uint32_t* cluster, uint32_t* ends,
+                                              uint32_t* counter, int width) {
+  __shared__ uint8_t maps[8][32];
+  const int lane = threadIdx.x & 31;
+  uint32_t L = blockIdx.x * blockDim.x + threadIdx.x, R = L, split = L;
+  bool alive = L < n;
+  while (__any_sync(0xffffffffu, alive)) {
+    if (alive) {
+      // the parent range: towards the smaller gap
+      const bool right = L == 0 || (R != n - 1 && code_gap(keys, R) < code_gap(keys, L - 1));
+      __threadfence();
+      const uint32_t other = atomicExch(&ends[right ? R : L - 1], right ? L : R);
+      if (other == NONE) {
+        alive = false;  // the sibling range is not done: its thread continues
+      } else if (right) {
+        split = R + 1;
+        R = other;
+      } else {
+        split = L;
+        L = other;
+      }
+      __threadfence();
+    }
+    const bool top = alive && L == 0 && R == n - 1;
+    uint32_t m = __ballot_sync(0xffffffffu, alive && (R - L + 1 > PLOC_KEEP || top));
+    while (m) {
+      const int src = __ffs(m) - 1;
+      m &= m - 1;
+      ploc_merge(T, cluster, counter, __shfl_sync(0xffffffffu, L, src),
+                 __shfl_sync(0xffffffffu, split, src), __shfl_sync(0xffffffffu, R, src),
+                 __shfl_sync(0xffffffffu, top ? 1 : 0, src) != 0, width, maps[threadIdx.x >> 5], lane);
+    }
+    if (top) alive = false;
+  }
+}
+
+// ------------------------------------------------------ treelet builder ----
 __device__ __forceinline__ int delta(const uint32_t* keys, int n, int i, int j) {
   if (j < 0 || j >= n) return -1;
   uint32_t a = keys[i], b = keys[j];
@@ -243,24 +510,17 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, int n, uint32_t* lef
   if (i == 0) parent_int[0] = 0xffffffffu;
 }
 
-struct Tree {
-  uint32_t *left, *right, *parent_int, *parent_leaf;
-  float4 *ilo, *ihi;        // internal bounds; ilo.w = SAH cost, ihi.w = primitive count
-  const float4 *llo, *lhi;  // leaf bounds (sorted order)
-  uint32_t* flags;
-};
-
 // Internal-node data (boxes, costs, counts, links) is written by other
 // threads of k_bottom_up while it runs, so it is read through L2 only; leaf
 // boxes come from an earlier kernel.
-__device__ __forceinline__ GBox ref_box(const Tree& T, uint32_t r) {
+__device__ __forceinline__ GBox ref_box_cg(const Tree& T, uint32_t r) {
   return (r & LEAF_BIT) ? box_load(T.llo, T.lhi, r & ~LEAF_BIT) : box_load_cg(T.ilo, T.ihi, r);
 }
 __device__ __forceinline__ float ref_cost(const Tree& T, uint32_t r) {
   return (r & LEAF_BIT) ? C_TRI * box_area(box_load(T.llo, T.lhi, r & ~LEAF_BIT))
                         : __ldcg(&T.ilo[r].w);
 }
-__device__ __forceinline__ float ref_count(const Tree& T, uint32_t r) {
+__device__ __forceinline__ float ref_count_cg(const Tree& T, uint32_t r) {
   return (r & LEAF_BIT) ? 1.f : __ldcg(&T.ihi[r].w);
 }
 __device__ __forceinline__ uint32_t left_of(const Tree& T, uint32_t x) { return __ldcg(T.left + x); }
@@ -308,7 +568,7 @@ __device__ void optimize_treelet(const Tree& T, uint32_t root, TreeletDP& dp, in
   if (nl < 3) return;  // the same for every lane
   const int full = (1 << nl) - 1;
   if (lane < nl) {
-    GBox b = ref_box(T, leaves[lane]);
+    GBox b = ref_box_cg(T, leaves[lane]);
     const int S = 1 << lane;
     for (int a = 0; a < 3; a++) {
       dp.box[a][S] = b.lo[a];
@@ -377,7 +637,7 @@ __device__ void optimize_treelet(const Tree& T, uint32_t root, TreeletDP& dp, in
       float cnt = 0.f;
       // count = sum of leaf counts in S
       for (int k = 0; k < nl; k++)
-        if (it.S & (1 << k)) cnt += ref_count(T, leaves[k]);
+        if (it.S & (1 << k)) cnt += ref_count_cg(T, leaves[k]);
       GBox b;
       for (int a = 0; a < 3; a++) {
         b.lo[a] = dp.box[a][it.S];
@@ -412,8 +672,8 @@ __global__ void __launch_bounds__(256) k_bottom_up(Tree T, int n, int optimize) 
         } else {
           __threadfence();
           uint32_t l = left_of(T, node), r = right_of(T, node);
-          GBox b = box_union(ref_box(T, l), ref_box(T, r));
-          float cnt = ref_count(T, l) + ref_count(T, r);
+          GBox b = box_union(ref_box_cg(T, l), ref_box_cg(T, r));
+          float cnt = ref_count_cg(T, l) + ref_count_cg(T, r);
           float cost = C_INNER * box_area(b) + ref_cost(T, l) + ref_cost(T, r);
           box_store(T.ilo, T.ihi, node, b, cost, cnt);
           need = optimize && cnt >= 7.f;
@@ -437,7 +697,7 @@ struct CollapseOut {
   uint4* nodes;           // 5 per node
   float4* rec_out;        // leaf-ordered primitive records
   uint32_t* leaf_of_id;
-  uint32_t* counters;     // [0] nodes, [1] primitives, [2] next-level queue length, [3] error
+  uint32_t* counters;     // [0] nodes, [1] primitives, [2] error
   uint32_t n;             // primitives = capacity of nodes, records and queues
 };
 
@@ -461,21 +721,21 @@ __device__ __forceinline__ int gather_small(const Tree& T, const uint32_t* sorte
   return cnt;
 }
 
-__global__ void k_collapse(Tree T, const uint32_t* __restrict__ sorted_prim,
-                           const float4* __restrict__ rec_in, const uint2* __restrict__ qin,
-                           uint32_t nq, uint2* qout, CollapseOut out, int width) {
-  uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nq) return;
-  uint2 it = qin[t];
+// One wide node: it.x the binary subtree, it.y its index.
+__device__ __forceinline__ void collapse_node(const Tree& T, const uint32_t* __restrict__ sorted_prim,
+                                              const float4* __restrict__ rec_in, uint2 it,
+                                              uint2* qout, uint32_t* qout_len,
+                                              const CollapseOut& out, int width) {
   uint32_t kids[8];
+  uint32_t slots = 0;  // 4 bits per kid: the slots its subtree may take (0: it is one slot)
   int nk = 0;
   if (it.x & LEAF_BIT) {  // a single-primitive scene
     kids[nk++] = it.x;
-  } else {
+  } else if (!T.plan) {
     kids[nk++] = T.left[it.x];
     kids[nk++] = T.right[it.x];
-    // at most 6 expansions (2 -> 8 children); a fixed trip count keeps the
-    // per-thread arrays in registers
+    // the child of largest area is expanded, at most 6 times (2 -> 8 children);
+    // a fixed trip count keeps the per-thread arrays in registers
 #pragma unroll
     for (int ex = 0; ex < 6; ex++) {
       if (nk >= width) break;
@@ -494,6 +754,39 @@ __global__ void k_collapse(Tree T, const uint32_t* __restrict__ sorted_prim,
       kids[best] = T.left[x];
       kids[nk++] = T.right[x];
     }
+  } else {
+    // the node's children, then every child with slots to share out in turn:
+    // at most 6 more; a fixed trip count keeps the arrays in registers
+    const uint32_t k = (__ldg(T.plan + it.x) >> (3 * (width - 2))) & 7u;
+    kids[0] = T.left[it.x];
+    kids[1] = T.right[it.x];
+    slots = k | (((uint32_t)width - k) << 4);
+    nk = 2;
+#pragma unroll
+    for (int ex = 0; ex < 6; ex++) {
+      int at = -1;
+      uint32_t share = 0, have = 0;
+      for (int q = 0; q < nk; q++) {
+        if (at >= 0) break;
+        uint32_t j = (slots >> (4 * q)) & 15u;
+        if (j < 2 || (kids[q] & LEAF_BIT)) continue;
+        const uint32_t plan = __ldg(T.plan + kids[q]);
+        while (j >= 2 && !((plan >> (3 * (j - 2))) & 7u)) j--;
+        if (j < 2) {
+          slots &= ~(15u << (4 * q));
+          continue;
+        }
+        at = q;
+        have = j;
+        share = (plan >> (3 * (j - 2))) & 7u;
+      }
+      if (at < 0) break;
+      const uint32_t x = kids[at];
+      kids[at] = T.left[x];
+      kids[nk] = T.right[x];
+      slots = (slots & ~(15u << (4 * at))) | (share << (4 * at)) | ((have - share) << (4 * nk));
+      nk++;
+    }
   }
   // classify and allocate
   int n_int = 0;
@@ -501,23 +794,23 @@ __global__ void k_collapse(Tree T, const uint32_t* __restrict__ sorted_prim,
   uint32_t cnts[8];
   for (int k = 0; k < nk; k++) {
     float c = ref_count(T, kids[k]);
-    if (!(kids[k] & LEAF_BIT) && c > 3.f) {
+    if (!(kids[k] & LEAF_BIT) && (T.plan ? !((__ldg(T.plan + kids[k]) >> 21) & 1u) : c > 3.f)) {
       n_int++;
       cnts[k] = 0;
     } else if (c >= 1.f && c <= 3.f) {
       cnts[k] = (uint32_t)c;
       nprim += cnts[k];
     } else {  // a count a valid tree cannot have: flag it, write nothing
-      atomicOr(&out.counters[3], 1u);
+      atomicOr(&out.counters[2], 1u);
       return;
     }
   }
   uint32_t child_base = n_int ? atomicAdd(&out.counters[0], (uint32_t)n_int) : 0;
   uint32_t prim_base = nprim ? atomicAdd(&out.counters[1], nprim) : 0;
-  uint32_t qbase = n_int ? atomicAdd(&out.counters[2], (uint32_t)n_int) : 0;
+  uint32_t qbase = n_int ? atomicAdd(qout_len, (uint32_t)n_int) : 0;
   if (it.y >= out.n || child_base + (uint32_t)n_int > out.n || prim_base + nprim > out.n ||
       qbase + (uint32_t)n_int > out.n) {
-    atomicOr(&out.counters[3], 2u);  // would overrun the buffers: the host rejects the tree
+    atomicOr(&out.counters[2], 2u);  // would overrun the buffers: the host rejects the tree
     return;
   }
   pt::WideChild wc[8];
@@ -546,7 +839,7 @@ __global__ void k_collapse(Tree T, const uint32_t* __restrict__ sorted_prim,
       wc[k].prim_off = off;
       uint32_t pr[3];
       if (gather_small(T, sorted_prim, kids[k], pr) != (int)cnts[k]) {
-        atomicOr(&out.counters[3], 4u);
+        atomicOr(&out.counters[2], 4u);
         return;
       }
       for (uint32_t q = 0; q < cnts[k]; q++) {
@@ -565,20 +858,38 @@ __global__ void k_collapse(Tree T, const uint32_t* __restrict__ sorted_prim,
     pb.hi[a] = parent.hi[a];
   }
   uint32_t words[20];
-  pt::encode_node_dev(pb, wc, nk, child_base, prim_base, words);
+  pt::encode_node_dev(pb, wc, nk, child_base, prim_base, words, T.plan != nullptr);
   uint4* dst = out.nodes + 5 * (size_t)it.y;
   for (int w = 0; w < 5; w++)
     dst[w] = make_uint4(words[4 * w], words[4 * w + 1], words[4 * w + 2], words[4 * w + 3]);
 }
 
-// leaf boxes in sorted (Morton) order
+// One level of the wide tree; its length and the next level's are on the device.
+__global__ void k_collapse(Tree T, const uint32_t* __restrict__ sorted_prim,
+                           const float4* __restrict__ rec_in, const uint2* __restrict__ qin,
+                           const uint32_t* __restrict__ qlen, uint2* qout, uint32_t* qout_len,
+                           CollapseOut out, int width) {
+  // an earlier level met an inconsistency, or the binary tree is incomplete: the
+  // queue is not to be trusted
+  const uint32_t err = __ldcg(out.counters + 2), made = __ldcg(out.counters + 3);
+  if (err || (T.plan && out.n > 1 && made != out.n - 1)) return;
+  const uint32_t nq = min(*qlen, out.n);
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nq; t += gridDim.x * blockDim.x)
+    collapse_node(T, sorted_prim, rec_in, qin[t], qout, qout_len, out, width);
+}
+
+// Leaf boxes in sorted (Morton) order, every leaf a cluster of its own, and
+// the first entry of the collapse queue.
 __global__ void k_gather_boxes(const float4* lo, const float4* hi, const uint32_t* order, uint32_t n,
-                               float4* slo, float4* shi) {
+                               float4* slo, float4* shi, uint32_t* cluster, uint2* queue,
+                               uint32_t root) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t p = order[i];
   slo[i] = lo[p];
   shi[i] = hi[p];
+  if (cluster) cluster[i] = i | LEAF_BIT;
+  if (i == 0) queue[0] = make_uint2(root, 0u);
 }
 
 // Carves the builder's scratch arrays out of one device arena that persists
@@ -643,24 +954,33 @@ namespace pt {
 // n records, n ids).  Returns the number of nodes and the depth (depth < 0:
 // the collapse met an inconsistent tree and stopped before overrunning a
 // buffer; -depth: 1 bad count, 2 capacity, 4 leaf gather mismatch; 8: the
-// finished tree broke a structural rule).
+// finished tree broke a structural rule; 16: incomplete or too deep).
+// triangles: every primitive is one; then the tree is clustered, else rebuilt
+// in treelets.  GB300, 2.1 M-triangle terrain: pt_commit 16.0 -> 4.3 ms (the
+// treelet passes took 12.6), 64 frames at 1920x1080 76.9 -> 76.3 ms, a batch of
+// eight terrains 72.0 -> 71.1 ms.  Scenes with other shapes keep the treelet
+// tree and with it their images: see encode_node_dev on node boundaries.
 cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t n,
                            uint4* d_nodes, float4* d_rec_out, uint32_t* d_leaf_of_id,
-                           uint32_t* out_nodes, int* out_depth, int treelet_rounds, int width,
+                           uint32_t* out_nodes, int* out_depth, int width, bool triangles,
                            float cam_t0, float cam_t1, BuildArena* arena, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   if (width < 2 || width > 8) width = 8;
   float4 *lo = nullptr, *hi = nullptr, *ilo = nullptr, *ihi = nullptr, *slo = nullptr,
-         *shi = nullptr;
+         *shi = nullptr, *cost = nullptr;
+  uint32_t* plan = nullptr;
   uint32_t *keys = nullptr, *vals = nullptr, *keys2 = nullptr, *vals2 = nullptr, *left = nullptr,
-           *right = nullptr, *pint = nullptr, *pleaf = nullptr, *flags = nullptr, *counters = nullptr;
+           *right = nullptr, *cluster = nullptr, *ends = nullptr, *counters = nullptr;
+  uint32_t *pint = nullptr, *pleaf = nullptr, *flags = nullptr;
   unsigned int* cbox = nullptr;
   uint2 *qa = nullptr, *qb = nullptr;
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
   uint32_t ni = n > 1 ? n - 1 : 1;
   int depth = 0;
-  uint32_t h_cnt[4] = {1, 0, 0, 0};
+  // nodes, primitives, error, tree nodes; then the queue length of each level
+  constexpr int kLevels = 252;
+  uint32_t h_cnt[4 + kLevels] = {1, 0, 0, 0, 1};
   unsigned int h_cbox[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
 #define BV(x)                         \
   do {                                \
@@ -686,10 +1006,17 @@ cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t
       cv.take(&vals2, n);
       cv.take(&left, ni);
       cv.take(&right, ni);
-      cv.take(&pint, ni);
-      cv.take(&pleaf, n);
-      cv.take(&flags, ni);
-      cv.take(&counters, 4);
+      if (triangles) {
+        cv.take(&cluster, n);
+        cv.take(&ends, n);
+        cv.take(&cost, 2 * (size_t)ni);
+        cv.take(&plan, ni);
+      } else {
+        cv.take(&pint, ni);
+        cv.take(&pleaf, n);
+        cv.take(&flags, ni);
+      }
+      cv.take(&counters, 4 + kLevels);
       cv.take(&cbox, 6);
       cv.take(&qa, n);
       cv.take(&qb, n);
@@ -709,65 +1036,78 @@ cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t
   BV(cudaMemcpyAsync(cbox, h_cbox, sizeof(h_cbox), cudaMemcpyHostToDevice, st));
   {
     uint32_t g = (n + 255) / 256;
-    k_bounds<<<g, 256, 0, st>>>(d_rec, d_xforms, n, cam_t0, cam_t1, lo, hi, cbox);
+    k_bounds<<<g < 608u ? g : 608u, 256, 0, st>>>(d_rec, d_xforms, n, cam_t0, cam_t1, lo, hi, cbox);
     k_morton<<<g, 256, 0, st>>>(lo, hi, n, cbox, keys, vals);
     BV(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, vals, vals2, (int)n, 0, 30, st));
     // leaf bounds in sorted order
-    BV(cudaMemsetAsync(pint, 0xff, ni * 4, st));
-    BV(cudaMemsetAsync(pleaf, 0xff, (size_t)n * 4, st));
     Tree T;
     T.left = left;
     T.right = right;
-    T.parent_int = pint;
-    T.parent_leaf = pleaf;
     T.ilo = ilo;
     T.ihi = ihi;
     T.llo = slo;
     T.lhi = shi;
+    T.cost = cost;
+    T.plan = plan;
+    T.parent_int = pint;
+    T.parent_leaf = pleaf;
     T.flags = flags;
-    k_gather_boxes<<<g, 256, 0, st>>>(lo, hi, vals2, n, slo, shi);
-    if (n > 1) {
+    T.root = n == 1 ? (0u | LEAF_BIT) : (triangles ? n - 2 : 0u);
+    BV(cudaMemcpyAsync(counters, h_cnt, sizeof(h_cnt), cudaMemcpyHostToDevice, st));
+    k_gather_boxes<<<g, 256, 0, st>>>(lo, hi, vals2, n, slo, shi, cluster, qa, T.root);
+    if (n > 1 && triangles) {
+      BV(cudaMemsetAsync(ends, 0xff, (size_t)n * 4, st));
+      k_ploc<<<g, 256, 0, st>>>(T, keys2, n, cluster, ends, counters + 3, width);
+    } else if (n > 1) {
+      BV(cudaMemsetAsync(pint, 0xff, ni * 4, st));
+      BV(cudaMemsetAsync(pleaf, 0xff, (size_t)n * 4, st));
       k_karras<<<(ni + 255) / 256, 256, 0, st>>>(keys2, (int)n, left, right, pint, pleaf);
-      for (int round = 0; round <= treelet_rounds; round++) {
+      for (int round = 0; round <= PT_TREELET_ROUNDS; round++) {
         BV(cudaMemsetAsync(flags, 0, ni * 4, st));
         k_bottom_up<<<g, 256, 0, st>>>(T, (int)n, round > 0 ? 1 : 0);
       }
     }
-    // collapse, level by level
-    BV(cudaMemcpyAsync(counters, h_cnt, sizeof(h_cnt), cudaMemcpyHostToDevice, st));
-    uint2 root = make_uint2(n > 1 ? 0u : (0u | LEAF_BIT), 0u);
-    BV(cudaMemcpyAsync(qa, &root, sizeof(root), cudaMemcpyHostToDevice, st));
-    uint32_t nq = 1;
+    // collapse level by level; the host looks every few levels whether one is left
     CollapseOut co{d_nodes, d_rec_out, d_leaf_of_id, counters, n};
-    while (nq) {
-      depth++;
-      BV(cudaMemsetAsync(counters + 2, 0, 4, st));
-      k_collapse<<<(nq + 127) / 128, 128, 0, st>>>(T, vals2, d_rec, qa, nq, qb, co, width);
+    const uint32_t cg = g < 2048u ? g : 2048u;
+    while (true) {
+      const int last = depth + 6 < kLevels - 1 ? depth + 6 : kLevels - 1;
+      for (; depth < last; depth++) {
+        k_collapse<<<cg, 128, 0, st>>>(T, vals2, d_rec, qa, counters + 4 + depth, qb,
+                                       counters + 5 + depth, co, width);
+        uint2* tq = qa;
+        qa = qb;
+        qb = tq;
+      }
       BV(cudaMemcpyAsync(h_cnt, counters, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
       BV(cudaStreamSynchronize(st));
-      nq = h_cnt[3] ? 0u : h_cnt[2];
-      uint2* tq = qa;
-      qa = qb;
-      qb = tq;
+      if (h_cnt[2] || !h_cnt[4 + depth]) break;
+      if (depth == kLevels - 1) {
+        h_cnt[2] = 16;
+        break;
+      }
     }
+    depth = 0;
+    while (depth < kLevels && h_cnt[4 + depth]) depth++;
+    if (triangles && n > 1 && !h_cnt[2] && h_cnt[3] != n - 1) h_cnt[2] = 16;
     // structural check of the result (keys and vals are free by now)
-    if (!h_cnt[3] && n > 0) {
+    if (!h_cnt[2] && n > 0) {
       const uint32_t nn = h_cnt[0];
       if (nn == 0 || nn > n) {
-        h_cnt[3] = 8;
+        h_cnt[2] = 8;
       } else {
         BV(cudaMemsetAsync(keys, 0, (size_t)n * 4, st));
         BV(cudaMemsetAsync(vals, 0, (size_t)n * 4, st));
-        k_check_nodes<<<(nn + 255) / 256, 256, 0, st>>>(d_nodes, nn, n, keys, counters + 3);
-        k_check_ids<<<g, 256, 0, st>>>(d_leaf_of_id, n, vals, counters + 3);
-        k_check_cover<<<g, 256, 0, st>>>(keys, vals, n, counters + 3);
-        BV(cudaMemcpyAsync(&h_cnt[3], counters + 3, 4, cudaMemcpyDeviceToHost, st));
+        k_check_nodes<<<(nn + 255) / 256, 256, 0, st>>>(d_nodes, nn, n, keys, counters + 2);
+        k_check_ids<<<g, 256, 0, st>>>(d_leaf_of_id, n, vals, counters + 2);
+        k_check_cover<<<g, 256, 0, st>>>(keys, vals, n, counters + 2);
+        BV(cudaMemcpyAsync(&h_cnt[2], counters + 2, 4, cudaMemcpyDeviceToHost, st));
         BV(cudaStreamSynchronize(st));
       }
     }
     BV(cudaGetLastError());
-    *out_nodes = h_cnt[3] ? 0u : h_cnt[0];
-    *out_depth = h_cnt[3] ? -(int)h_cnt[3] : depth;  // < 0: the collapse found an inconsistent tree
+    *out_nodes = h_cnt[2] ? 0u : h_cnt[0];
+    *out_depth = h_cnt[2] ? -(int)h_cnt[2] : depth;  // < 0: the collapse found an inconsistent tree
   }
 done:
 #undef BV

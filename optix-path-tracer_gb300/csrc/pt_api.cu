@@ -31,17 +31,13 @@
 namespace pt {
 cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t n,
                            uint4* d_nodes, float4* d_rec_out, uint32_t* d_leaf_of_id,
-                           uint32_t* out_nodes, int* out_depth, int treelet_rounds, int width,
+                           uint32_t* out_nodes, int* out_depth, int width, bool triangles,
                            float cam_t0, float cam_t1, BuildArena* arena, cudaStream_t st);
 }
 
 namespace {
 const float PI_F = 3.141592654f;
 }  // namespace
-
-#ifndef PT_TREELET_ROUNDS
-#define PT_TREELET_ROUNDS 2  /* SAH treelet restructuring passes of the GPU builder */
-#endif
 
 using namespace pth;
 
@@ -878,7 +874,8 @@ int pth::build_bvh(pt_context* ctx, int width, DevBuf<uint4>& d_nodes, DevBuf<fl
     uint32_t nodes = 0;
     int depth = 0;
     CK(pt::build_bvh8_gpu(ctx->d_rec_in.p, ctx->d_xforms.p, (uint32_t)n, d_nodes.p,
-                          d_prims.p, d_leaf_of_id.p, &nodes, &depth, PT_TREELET_ROUNDS, width,
+                          d_prims.p, d_leaf_of_id.p, &nodes, &depth, width,
+                          all_triangles(ctx),
                           ctx->cam.time0, ctx->cam.time1, &ctx->build_arena, st));
     if (depth < 0)
       return fail(ctx, PT_EINVAL,
