@@ -69,7 +69,7 @@ typedef struct pt_options {
   int enable_timing;   /* per-stage device times (CUDA events in the graph) */
   int bvh_builder;     /* 0 automatic, 1 host (binned SAH), 2 GPU (LBVH + treelets) */
   int bvh_width;       /* most children per BVH node, 2..8; 0 = 8 */
-  int shade_order;     /* 0 automatic (material-sorted tiles when the scene uses
+  int shade_order;     /* 0 automatic (material order when the scene uses
                           Oren-Nayar, Torrance-Sparrow or Ashikhmin-Shirley), 1 sorted,
                           2 path order */
   int refetch_lanes;   /* idle lanes of a trace warp that take new rays together, 1..32;
@@ -321,7 +321,7 @@ PT_API int pt_get_stats(pt_context* ctx, pt_stats* out);
 /* pt_render for callers that cannot allocate device memory while rendering
  * (a strict memory pool, or an application that allocates only at start-up).
  * No counterpart in the reference.  It calls no cudaMalloc/cudaFree: its
- * wavefront scratch is a fixed 8.75 MiB device array inside libpt.so that
+ * wavefront scratch is a fixed 9.25 MiB device array inside libpt.so that
  * every GPU loading the library holds until exit.  Same results as
  * pt_render.  accum_rgba must be device memory; images of at most 262144
  * pixels (PT_EINVAL beyond); fewer paths in flight, so slower.  All calls
@@ -427,8 +427,8 @@ PT_API const char* pt_batch_last_error(pt_batch* b);
 PT_API int pt_batch_render(pt_batch* b, const pt_batch_item* items, int n, void* stream);
 /* Times short renders of a sample of the items (every item at low spp, into
  * scratch accumulators; the items' accumulators are not touched) over path
- * slots, trace and shade block sizes, BVH node width and shade order (material-
- * sorted tiles or path order), keeps the fastest
+ * slots, trace and shade block sizes, BVH node width and shade order (material
+ * order or path order), keeps the fastest
  * configuration for later pt_batch_render calls and returns it in *best. */
 PT_API int pt_batch_autotune(pt_batch* b, const pt_batch_item* items, int n, pt_tune* best);
 PT_API int pt_batch_set_tune(pt_batch* b, const pt_tune* t);

@@ -1065,6 +1065,7 @@ void pth::carve_wave(WaveState& W, float4* f, uint4* u, size_t s) {
     b.st = u + k * s;
   }
   W.hit = f + 8 * s;
+  W.lists = (uint32_t*)(u + 3 * s);
   W.sh.P = f + 9 * s;
   W.sh.N = f + 10 * s;
   W.sh.Wo = f + 11 * s;

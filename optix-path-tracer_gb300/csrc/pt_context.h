@@ -205,7 +205,7 @@ bool uses_textures(const pt_context* ctx);
 bool all_triangles(const pt_context* ctx);
 /* Whether some sphere of the scene moves. */
 bool has_motion(const pt_context* ctx);
-/* Whether shading in material-sorted tiles pays for this scene: it does when
+/* Whether shading in material order pays for this scene: it does when
  * one of the costly BRDFs (Oren-Nayar, Torrance-Sparrow, Ashikhmin-Shirley)
  * is present, whose code paths diverge most in a mixed warp. */
 bool sort_pays(const pt_context* ctx);

@@ -16,22 +16,14 @@
 #define PT_TRACE_MAXREG 72       /* registers per trace thread: 7 blocks of 128 per SM */
 #endif
 #define PT_SHADE_BLOCK 256       /* default and largest shade block */
+/* Shading: 4 resident blocks of 256 threads (64 registers).  Consistent mode on
+ * the 2.1 M-triangle terrain, 64 frames, with 2 / 3 / 4 / 5 / 6 / 7: 71.4 / 66.8 /
+ * 64.9 / 65.6 / 66.0 / 67.6 ms (fewer registers spill, fewer blocks hide less
+ * latency); guided 20.3 / 19.9 / 19.6 / 19.6 / 19.6 / 19.6 ms; reference mode is
+ * 10 % slower at 5 on random spheres. */
 #ifndef PT_SHADE_MINBLOCKS
-#define PT_SHADE_MINBLOCKS 4     /* of 256 threads: <= 64 registers, 1024 resident threads per SM */
+#define PT_SHADE_MINBLOCKS 4
 #endif
-/* consistent-mode shading: more resident blocks of fewer registers (the
- * spills go to L1) hide more of its dependent loads: 7 blocks of 256 (<= 36
- * registers) gave 1150 -> 1210 M paths/s on the 2.1 M-triangle heightfield
- * (5: 1167, 6: 1182, 8: 1210); reference-mode shading (k_shade) is faster
- * at 4 (5 blocks: 10 % slower on random spheres), and so is guided shading
- * (7 blocks: 256 guided frames of the lit box 3 % slower) */
-#ifndef PT_SHADE_C_MINBLOCKS
-#define PT_SHADE_C_MINBLOCKS 7
-#endif
-#ifndef PT_SHADE_G_MINBLOCKS
-#define PT_SHADE_G_MINBLOCKS PT_SHADE_MINBLOCKS
-#endif
-
 #define PT_TAIL_BLOCK 128        /* threads per block of the tail kernel */
 /* Paths left in a chunk (live and not generated) that the tail kernel takes
  * over from the wavefront.  GB300, us per render with 0 (wavefront only) /
@@ -55,7 +47,7 @@
 struct LaunchCfg {
   int trace_block, trace_grid;
   int shade_block, shade_grid;
-  int sort;            /* shade in material-sorted tiles */
+  int sort;            /* shade in material order (by lists that the trace fills) */
   int refetch;         /* idle lanes of a trace warp that take new rays together (1..32) */
   int tex;             /* some material takes a texture: the texture variants of shading */
   int motion;          /* some sphere moves: the trace variants that carry ray times */
@@ -85,6 +77,7 @@ struct WaveCounters {
   unsigned long long iters_total; /* iterations over all chunks (batch) */
   uint32_t chunk;        /* current chunk of a batch */
   uint32_t n_chunks;     /* chunks of the batch (set by the host) */
+  uint32_t listed[8];    /* positions in each shading list (PT_SHADE_KEYS of them) */
   uint32_t ray_next[2];  /* rays taken by trace warps this iteration (extension, shadow) */
   uint32_t guide_rows;   /* positions listed for guide inference this iteration */
   uint32_t drained;      /* iterations since the chunk's last path was generated, that one
@@ -193,6 +186,7 @@ struct GuideInferArgs;
 struct WaveState {
   PathBuf path[2];            /* ping-pong: path[parity] is current */
   float4* hit;                /* t, u, v, leaf index: by position in the current buffer */
+  uint32_t* lists;            /* sorted shading: `slots` positions for each shading key */
   ShadowBuf sh;               /* reference mode */
   NeeBuf nee[2];              /* consistent mode, beside path[]; shares sh's memory */
   WaveCounters* ctr;
@@ -206,9 +200,11 @@ struct WaveState {
 };
 
 /* float4 arrays per slot: 2 x 4 (path buffers) + 1 (hit) + 7 (shadow), and
- * 3 uint4 state arrays. */
+ * uint4 entries: 3 states and an entry in each of the 8 shading lists. */
 #define PT_SLOT_F4 16
-#define PT_SLOT_U4 3
+#define PT_SLOT_U4 5
+/* Shading key of a hit: 0 none, 1 + material type. */
+#define PT_SHADE_KEYS (PT_NUM_MAT_TYPES + 1)
 
 /* Ray kinds of the trace kernels: closest hit of extension rays; closest
  * hit of a shadow ray (reference mode: the light must be the first thing
@@ -221,6 +217,7 @@ namespace pt {
 size_t trace_smem(int max_stack, int block);
 /* Resident trace blocks per SM (0 if the shape does not fit). */
 int trace_blocks_per_sm(int block, size_t smem);
+static_assert(PT_SHADE_KEYS == 8, "WaveCounters::listed, WaveState::lists");
 /* One trace launch of `mode` (TRACE_EXT, TRACE_SHADOW or TRACE_BOTH)
  * over the wavefront's rays, with the launch shape of lc. */
 void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W,

@@ -98,93 +98,51 @@ __global__ void k_generate(DevScene S0, WaveState W, const WaveCtl* __restrict__
   }
 }
 
-// ------------------------------------------------ material-sorted tiles --
-// The shade kernels take the live paths in tiles of blockDim x
-// PT_SORT_ITEMS consecutive positions and shade each tile in the order of
-// its material key (0 miss, 1 + material type, PT_SORT_KEYS - 1 past the
-// end): a counting sort in shared memory (shared atomics give the ranks, one
-// thread the key offsets).  Warps then run one material's code instead of a
-// mix, which is what bounds these kernels (SIMT efficiency and instruction
-// fetch).  The order does not change any path's result.
-#ifndef PT_SORT_ITEMS
-#define PT_SORT_ITEMS 4
-#endif
-#ifndef PT_SHADE_TILE_GRID
-#define PT_SHADE_TILE_GRID 1
-#endif
-#define PT_SORT_KEYS (PT_NUM_MAT_TYPES + 2)
-#ifndef PT_SORT_FILL
-#define PT_SORT_FILL 1024u  // tiles that keep the GPU busy
-#endif
-
-struct SortTile {
-  uint16_t perm[PT_SHADE_BLOCK * PT_SORT_ITEMS];  // tile position in sorted order
-  uint32_t cnt[PT_SORT_KEYS];
-  uint32_t start[PT_SORT_KEYS];
-};
-
-__device__ __forceinline__ uint32_t shade_key(const DevScene& S0, const float4* __restrict__ hit,
-                                              uint32_t i, uint32_t n) {
-  if (i >= n) return PT_SORT_KEYS - 1;
-  uint32_t leaf = __float_as_uint(hit[i].w);
-  if (leaf == PT_NO_HIT) return 0;
-  uint32_t mid = __float_as_uint(__ldg(&S0.prims[3 * (size_t)leaf + 2].w));
-  return 1u + (uint32_t)__ldg(&S0.mats[mid].type);
+// -------------------------------------------------- material-ordered shading --
+// The trace kernel puts every extension ray on the list of its shading key
+// (miss or material type), and a warp of the sorted shade kernels takes 32
+// entries of one list: it runs one material's code, and neighbouring warps the
+// same code, which is what bounds these kernels (lanes in use, instruction
+// fetch and the latency behind both).  The order does not change any path's
+// result.  Costly materials come first, so the launch ends on cheap ones.
+// GB300, before (tiles of 1024 paths sorted in shared memory, with barriers
+// around; 7 blocks per SM) -> after: 64 frames of the 2.1 M-triangle terrain
+// 76.3 -> 64.9 ms, one 1280x720 frame 973 -> 853 us, textures 3113 -> 2284 us,
+// guided frames 22.1 -> 19.6 ms.  Scenes of cheap materials alone are faster in
+// path order: random spheres 155.8 against 167.7 ms with lists, Cornell box
+// 15.5 against 16.8 (the lists' writes and the scattered reads cost more).
+__device__ __forceinline__ uint32_t list_key(int rank) {
+  constexpr uint32_t order = 0x04123567u;  // AS, TS, ON, dielectric, metal, Lambertian, light, miss
+  return (order >> (4 * rank)) & 15u;
 }
 
-__device__ __forceinline__ void sort_tile(SortTile& t, const DevScene& S0,
-                                          const float4* __restrict__ hit, uint32_t base,
-                                          uint32_t n, int items) {
-  const uint32_t bd = blockDim.x;
-  if (threadIdx.x < PT_SORT_KEYS) t.cnt[threadIdx.x] = 0;
-  __syncthreads();
-  uint32_t key[PT_SORT_ITEMS], rank[PT_SORT_ITEMS];
+// Position of this lane's path in chunk w (32 entries) of the lists, or
+// 0xffffffff past a list's end; false past the last chunk.
+__device__ __forceinline__ bool list_entry(const WaveState& W, const WaveCounters& c, uint32_t w,
+                                           uint32_t& i) {
+  i = 0xffffffffu;
 #pragma unroll
-  for (int it = 0; it < PT_SORT_ITEMS; it++) {
-    if (it >= items) break;
-    key[it] = shade_key(S0, hit, base + it * bd + threadIdx.x, n);
-    rank[it] = atomicAdd(&t.cnt[key[it]], 1u);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t sum = 0;
-    for (int k = 0; k < PT_SORT_KEYS; k++) {
-      t.start[k] = sum;
-      sum += t.cnt[k];
+  for (int rank = 0; rank < PT_SHADE_KEYS; rank++) {
+    const uint32_t key = list_key(rank), n = c.listed[key], chunks = (n + 31) / 32;
+    if (w < chunks) {
+      const uint32_t e = 32 * w + (threadIdx.x & 31);
+      if (e < n) i = __ldcs(&W.lists[(size_t)key * (size_t)W.slots + e]);
+      return true;
     }
+    w -= chunks;
   }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < PT_SORT_ITEMS; it++) {
-    if (it >= items) break;
-    t.perm[t.start[key[it]] + rank[it]] = (uint16_t)(it * bd + threadIdx.x);
-  }
-  __syncthreads();
+  return false;
 }
 
-// Paths per thread of a tile: larger tiles sort better, but a launch of fewer
-// than PT_SORT_FILL tiles leaves SMs idle, and a block takes its paths one
-// after the other, so small launches use smaller tiles.  GB300: 33 frames of
-// 321 x 243 with textures 3467 -> 3346 us (every launch with 1024-path tiles,
-// then this rule); launches that fill the GPU keep 1024.
-__device__ __forceinline__ int sort_items(uint32_t n) {
-  return (int)min((uint32_t)PT_SORT_ITEMS, 1u + n / (PT_SORT_FILL * blockDim.x));
-}
-
-// Loop of a shade kernel over its paths: material-sorted tiles (SORT) or a
-// plain grid-stride loop.  Every lane of a warp runs every step (the queue
-// appends inside are warp-aggregated).
+// Loop of a shade kernel over its paths: by the lists (SORT) or a plain
+// grid-stride loop.  Every lane of a warp runs every step (the queue appends
+// inside are warp-aggregated).
 #define SHADE_LOOP(CALL)                                                           \
   if (SORT) {                                                                      \
-    const int items = sort_items(n);                                               \
-    const uint32_t tile_n = blockDim.x * items;                                    \
-    for (uint32_t base = blockIdx.x * tile_n; base < n; base += gridDim.x * tile_n) { \
-      sort_tile(tile, S0, W.hit, base, n, items);                                  \
-      for (int it = 0; it < items; it++) {                                         \
-        uint32_t i = base + tile.perm[it * blockDim.x + threadIdx.x];              \
-        CALL;                                                                      \
-      }                                                                            \
-      __syncthreads();                                                             \
+    uint32_t i;                                                                    \
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;                \
+         list_entry(W, c, w, i); w += (gridDim.x * blockDim.x) >> 5) {             \
+      CALL;                                                                        \
     }                                                                              \
   } else {                                                                         \
     uint32_t stride = gridDim.x * blockDim.x;                                      \
@@ -241,7 +199,6 @@ template <bool BATCH, bool SORT, bool TEX>
 __global__ void __launch_bounds__(PT_SHADE_BLOCK, PT_SHADE_MINBLOCKS) k_shade(DevScene S0, WaveState W,
                                                           const WaveCtl* __restrict__ ctlp,
                                                           BatchRefs br) {
-  __shared__ SortTile tile;
   WaveCounters c = *W.ctr;
   WaveCtl ctl = *ctlp;
   uint32_t n = c.n_cur + gen_count(c, ctl, (uint32_t)W.slots);
@@ -348,10 +305,9 @@ __device__ __forceinline__ void shade_c_path(const DevScene& S0, const WaveState
 }
 
 template <bool BATCH, bool SORT, bool GUIDE, bool TEX>
-__global__ void __launch_bounds__(PT_SHADE_BLOCK, GUIDE ? PT_SHADE_G_MINBLOCKS : PT_SHADE_C_MINBLOCKS) k_shade_c(DevScene S0, WaveState W,
+__global__ void __launch_bounds__(PT_SHADE_BLOCK, PT_SHADE_MINBLOCKS) k_shade_c(DevScene S0, WaveState W,
                                                             const WaveCtl* __restrict__ ctlp,
                                                             BatchRefs br) {
-  __shared__ SortTile tile;
   WaveCounters c = *W.ctr;
   WaveCtl ctl = *ctlp;
   uint32_t n = c.n_cur + gen_count(c, ctl, (uint32_t)W.slots);
@@ -380,6 +336,7 @@ __global__ void k_advance(WaveState W, const WaveCtl* __restrict__ ctlp, int use
   c.n_shadow = 0;
   c.ray_next[0] = 0;
   c.ray_next[1] = 0;
+  for (int k = 0; k < PT_SHADE_KEYS; k++) c.listed[k] = 0;
   c.guide_rows = 0;
   c.parity ^= 1u;
   c.iter++;
@@ -424,6 +381,7 @@ __global__ void k_batch_begin(WaveState W, WaveCtl* ctl, const BatchChunk* __res
   c.n_next = 0;
   c.n_shadow = c.n_occ = 0;
   c.n_wait = c.n_wait_next = 0;
+  for (int k = 0; k < PT_SHADE_KEYS; k++) c.listed[k] = 0;
   c.parity = 0;
   c.iter = 0;
   c.next_path = 0;
@@ -743,12 +701,15 @@ void launch_chunk_begin(const WaveState& W, WaveCtl* ctl, const WaveCtl& v, bool
   k_chunk_begin<<<1, 1, 0, st>>>(W, ctl, v, first ? 1 : 0);
 }
 
-// Blocks of a sorted shading launch: one per tile of a full buffer, or as many
-// as its smaller tiles need when it is not full (sort_items).
+// Blocks of a sorted shading launch: a warp per 32 paths of a full buffer (each
+// list may end in a part of a chunk), at most PT_SORT_BLOCKS.
+#ifndef PT_SORT_BLOCKS
+#define PT_SORT_BLOCKS 8192
+#endif
 static int sort_grid(int slots, int block) {
-  const long long full = ((long long)slots + block * PT_SORT_ITEMS - 1) / (block * PT_SORT_ITEMS);
-  const long long fine = ((long long)slots + block - 1) / block;
-  return (int)std::max<long long>(1, std::max(full, std::min<long long>(fine, PT_SORT_FILL)));
+  const long long warps = ((long long)slots + 31) / 32 + PT_SHADE_KEYS;
+  const long long blocks = (warps * 32 + block - 1) / block;
+  return (int)std::min<long long>(blocks, PT_SORT_BLOCKS);
 }
 
 template <bool BATCH>
@@ -758,13 +719,7 @@ static void launch_iteration_t(const DevScene& S, const WaveState& W, const Wave
                                unsigned long long cond, const GuideInferArgs* gi) {
   const int sb = lc.shade_block, sg = lc.shade_grid;
   const BatchRefs* brp = BATCH ? &br : nullptr;
-  // sorted shading: one block per tile of the buffer (blocks past the live
-  // paths return at once), so the block scheduler balances uneven tiles
-#if PT_SHADE_TILE_GRID
   const int tgs = sort_grid(W.slots, sb);
-#else
-  const int tgs = sg;
-#endif
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
   k_generate<BATCH><<<sg, sb, 0, st>>>(S, W, ctl, br);
   if (ev) cudaEventRecordWithFlags(ev[1], st, cudaEventRecordExternal);

@@ -68,13 +68,14 @@ struct FirstHitOut {
 #endif
 
 // BATCH: rays of several scenes; each starts at its scene's root node (the
-// scene index is in the path state word st.z).  MOTION: the scene has moving
+// scene index is in the path state word st.z).  list: extension rays are put on
+// the shading lists.  MOTION: the scene has moving
 // spheres, so each ray carries its path's time (other scenes do without).
 template <int MODE, bool COUNT, bool BATCH, bool MOTION>
 __device__ __forceinline__ void trace_rays(const DevScene& S, const WaveState& W,
                                            const WaveCtl* __restrict__ ctlp, int max_stack,
                                            const FirstHitOut& fo, const BatchRefs& br,
-                                           int refetch) {
+                                           int refetch, int list) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   WarpShared& ws = ((WarpShared*)smem)[threadIdx.x >> 5];
@@ -152,8 +153,21 @@ __device__ __forceinline__ void trace_rays(const DevScene& S, const WaveState& W
     }
   };
 
+  // puts position i on the shading list of its key (the lanes that finish
+  // together share an atomic per key)
+  auto list_hit = [&](uint32_t key) {
+    const uint32_t act = __activemask();
+    const uint32_t same = __match_any_sync(act, key);
+    const int leader = __ffs(same) - 1;
+    uint32_t at = 0;
+    if (lane == leader) at = atomicAdd(&W.ctr->listed[key], (uint32_t)__popc(same));
+    at = __shfl_sync(same, at, leader) + (uint32_t)__popc(same & ((1u << lane) - 1u));
+    W.lists[(size_t)key * (size_t)W.slots + at] = i;
+  };
+
   auto finish = [&](V3 d, float tmax) {
     if (MODE == TRACE_EXT) {
+      uint32_t key = 0;
       float4 h = make_float4(tmax, 0.f, 0.f, __uint_as_float(PT_NO_HIT));
       if (best_id != PT_NO_HIT) {
         uint32_t leaf = __ldg(S.leaf_of_id + best_id);
@@ -161,8 +175,10 @@ __device__ __forceinline__ void trace_rays(const DevScene& S, const WaveState& W
         float t = tbest, bu = 0.f, bv = 0.f;
         if (prim_type(p) == PT_PRIM_TRIANGLE) tri_candidate(p, o, wt_setup(d), tmin, tmax, t, bu, bv);
         h = make_float4(tbest, bu, bv, __uint_as_float(leaf));
+        if (list) key = 1u + (uint32_t)__ldg(&S.mats[prim_material(p)].type);
       }
       W.hit[i] = h;
+      if (list) list_hit(key);
     } else if (MODE == TRACE_OCCLUDED) {
       // anything before the light
       W.nee[parity].Wi[i].w = best_id != PT_NO_HIT ? 1.f : 0.f;
@@ -463,7 +479,7 @@ __device__ __forceinline__ void trace_rays(const DevScene& S, const WaveState& W
 template <int MODE, bool COUNT, bool BATCH, bool MOTION>
 __global__ void __maxnreg__(PT_TRACE_MAXREG)
     k_trace_t(DevScene S, WaveState W, const WaveCtl* __restrict__ ctlp, int max_stack,
-              FirstHitOut fo, BatchRefs br, int refetch) {
+              FirstHitOut fo, BatchRefs br, int refetch, int list) {
   if (MODE == TRACE_BOTH) {
     // a warp that finds no extension ray left goes on to the occlusion rays, so
     // the one kind fills the SMs while the longest rays of the other end.  Two
@@ -471,11 +487,11 @@ __global__ void __maxnreg__(PT_TRACE_MAXREG)
     // 1280x720 terrain frame and 80.0 ms per 64 frames at 1920x1080; this one,
     // with the path state passed on once instead of parked, 973 us and 76.9 ms
     // (GB300)
-    trace_rays<TRACE_EXT, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch);
+    trace_rays<TRACE_EXT, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch, list);
     __syncwarp();
-    trace_rays<TRACE_OCCLUDED, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch);
+    trace_rays<TRACE_OCCLUDED, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch, list);
   } else {
-    trace_rays<MODE, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch);
+    trace_rays<MODE, COUNT, BATCH, MOTION>(S, W, ctlp, max_stack, fo, br, refetch, list);
   }
 }
 
@@ -549,10 +565,10 @@ static void launch_mode(bool counters, const DevScene& S, const WaveState& W, co
   FirstHitOut none{};
   if (counters)
     k_trace_t<MODE, true, BATCH, MOTION><<<lc.trace_grid, lc.trace_block, smem, st>>>(
-        S, W, ctl, max_stack, none, br, lc.refetch);
+        S, W, ctl, max_stack, none, br, lc.refetch, lc.sort);
   else
     k_trace_t<MODE, false, BATCH, MOTION><<<lc.trace_grid, lc.trace_block, smem, st>>>(
-        S, W, ctl, max_stack, none, br, lc.refetch);
+        S, W, ctl, max_stack, none, br, lc.refetch, lc.sort);
 }
 
 template <bool BATCH, bool MOTION>
@@ -588,11 +604,11 @@ void launch_first_hits(const DevScene& S, int w, int h, int frame, uint32_t* pri
   if (S.has_motion)
     k_trace_t<TRACE_FIRST, false, false, true>
         <<<grid, PT_TRACE_BLOCK, trace_smem(max_stack, PT_TRACE_BLOCK), st>>>(
-            S, none, nullptr, max_stack, fo, BatchRefs{}, 32);
+            S, none, nullptr, max_stack, fo, BatchRefs{}, 32, 0);
   else
     k_trace_t<TRACE_FIRST, false, false, false>
         <<<grid, PT_TRACE_BLOCK, trace_smem(max_stack, PT_TRACE_BLOCK), st>>>(
-            S, none, nullptr, max_stack, fo, BatchRefs{}, 32);
+            S, none, nullptr, max_stack, fo, BatchRefs{}, 32, 0);
 }
 
 }  // namespace pt
