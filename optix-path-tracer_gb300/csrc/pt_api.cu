@@ -259,6 +259,7 @@ PT_API int pt_context_destroy(pt_context* ctx) {
   ctx->d_lights.release();
   ctx->d_tri_attr.release();
   ctx->d_normals.release();
+  ctx->d_normals4.release();
   ctx->d_uvs.release();
   ctx->d_leaf_of_id.release();
   ctx->d_rec_in.release();
@@ -925,6 +926,12 @@ static cudaError_t upload_tables(pt_context* ctx, size_t* bytes) {
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_tex_list, ctx->tex_list, 1, st, bytes);
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_tri_attr, ctx->tri_attr, 1, st, bytes);
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_normals, ctx->normals, 3, st, bytes);
+  const size_t nv = std::max<size_t>(1, ctx->normals.size() / 3);
+  if (e == cudaSuccess) e = ctx->d_normals4.ensure(nv);
+  if (e == cudaSuccess) {
+    pt::launch_pack_normals(ctx->d_normals.p, nv, ctx->d_normals4.p, st);
+    e = cudaGetLastError();
+  }
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_uvs, ctx->uvs, 2, st, bytes);
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_env, ctx->env, 1, st, bytes);
   ctx->env_valid = 0;
@@ -1002,7 +1009,7 @@ PT_API int pt_commit(pt_context* ctx) {
   S.mats = ctx->d_mats.p;
   S.lights = ctx->d_lights.p;
   S.tri_attr = ctx->d_tri_attr.p;
-  S.normals = ctx->d_normals.p;
+  S.normals = ctx->d_normals4.p;
   S.uvs = ctx->d_uvs.p;
   S.leaf_of_id = ctx->d_leaf_of_id.p;
   S.textures = ctx->d_textures.p;
@@ -1038,6 +1045,7 @@ PT_API int pt_commit(pt_context* ctx) {
   ctx->lc.refetch = ctx->opt.refetch_lanes ? ctx->opt.refetch_lanes : pth::auto_refetch(n);
   ctx->lc.tex = pth::uses_textures(ctx) ? 1 : 0;
   ctx->lc.motion = pth::has_motion(ctx) ? 1 : 0;
+  if (nn == 1) ctx->lc.one_grid = pt::wave_grid(3, ctx->max_stack, 0);
   ctx->lc.lights = ctx->lights.empty() ? 0 : 1;
   ctx->lc.env = ctx->env_valid ? 1 : 0;
   auto t1 = std::chrono::steady_clock::now();
@@ -1066,6 +1074,7 @@ void pth::carve_wave(WaveState& W, float4* f, uint4* u, size_t s) {
   }
   W.hit = f + 8 * s;
   W.lists = (uint32_t*)(u + 3 * s);
+  W.listed = (uint32_t*)(u + 5 * s);
   W.sh.P = f + 9 * s;
   W.sh.N = f + 10 * s;
   W.sh.Wo = f + 11 * s;
@@ -1101,7 +1110,7 @@ static int ensure_wave(pt_context* ctx, size_t results_needed) {
   if (ctx->slots != slots || !ctx->d_slot_f4.p) {
     drop_graphs(ctx);
     CK(ctx->d_slot_f4.ensure((size_t)slots * PT_SLOT_F4));
-    CK(ctx->d_slot_u4.ensure((size_t)slots * PT_SLOT_U4));
+    CK(ctx->d_slot_u4.ensure(PT_SLOTS_U4(slots)));
     CK(ctx->d_ctr.ensure(1));
     CK(ctx->d_ctl.ensure(1));
     ctx->slots = slots;
@@ -1579,7 +1588,7 @@ PT_API int pt_trace_first_hits(pt_context* ctx, int width, int height, int frame
   uint32_t* d_err = ctx->d_tmpu.p + 2 * WH;
   CK(cudaMemsetAsync(d_err, 0, 4, st));
   pt::launch_first_hits(ctx->scene, width, height, frame, ctx->d_tmpu.p, ctx->d_tmpu.p + WH,
-                        ctx->d_tmp.p, ctx->max_stack, d_err, ctx->lc.trace_grid, st);
+                        ctx->d_tmp.p, ctx->max_stack, d_err, ctx->lc, st);
   CK(cudaGetLastError());
   uint32_t herr = 0;
   CK(cudaMemcpyAsync(prim, ctx->d_tmpu.p, WH * 4, cudaMemcpyDefault, st));
@@ -1648,7 +1657,7 @@ namespace {
 constexpr size_t kNoAllocSlots = 16384;
 constexpr size_t kNoAllocMaxPixels = 262144;  // e.g. 512 x 512
 constexpr size_t kNoAllocBytes =
-    kNoAllocSlots * (PT_SLOT_F4 * sizeof(float4) + PT_SLOT_U4 * sizeof(uint4)) +
+    kNoAllocSlots * PT_SLOT_F4 * sizeof(float4) + PT_SLOTS_U4(kNoAllocSlots) * sizeof(uint4) +
     256 /* WaveCounters */ + 256 /* WaveCtl */ + kNoAllocMaxPixels * sizeof(float4);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -1680,7 +1689,7 @@ static WaveState noalloc_wave(unsigned char* base, WaveCtl** ctl) {
   float4* f = (float4*)base;
   uint4* u = (uint4*)(f + PT_SLOT_F4 * s);
   carve_wave(W, f, u, s);
-  unsigned char* tail = (unsigned char*)(u + PT_SLOT_U4 * s);
+  unsigned char* tail = (unsigned char*)(u + PT_SLOTS_U4(s));
   W.ctr = (WaveCounters*)tail;
   *ctl = (WaveCtl*)(tail + 256);
   W.results = (float4*)(tail + 512);

@@ -75,7 +75,8 @@ struct pt_batch {
   DevBuf<uint4> nodes, tri_attr;
   DevBuf<float4> prims, xforms;
   DevBuf<GpuMaterial> mats;
-  DevBuf<float> normals, uvs;
+  DevBuf<float4> normals;
+  DevBuf<float> uvs;
   DevBuf<uint32_t> leaf_of_id;
   int max_stack = 1;
   size_t total_nodes = 0;
@@ -207,7 +208,7 @@ static int ensure_geometry(pt_batch* b, const pt_batch_item* items, int n) {
   BK(b->tri_attr.ensure(std::max<size_t>(P, 1)));
   BK(b->xforms.ensure(6 * X + 1));
   BK(b->mats.ensure(std::max<size_t>(M, 1)));
-  BK(b->normals.ensure(3 * A + 3));
+  BK(b->normals.ensure(A + 1));
   BK(b->uvs.ensure(2 * A + 2));
   // the trailing empty node: root of scenes without primitives
   BK(cudaMemsetAsync(b->nodes.p + 5 * N, 0, 5 * sizeof(uint4), st));
@@ -227,7 +228,7 @@ static int ensure_geometry(pt_batch* b, const pt_batch_item* items, int n) {
     if (nx) BK(cudaMemcpyAsync(b->xforms.p + 6 * xo, c->d_xforms.p, nx * 96, cudaMemcpyDeviceToDevice, st));
     if (nm) BK(cudaMemcpyAsync(b->mats.p + mo, c->d_mats.p, nm * sizeof(GpuMaterial), cudaMemcpyDeviceToDevice, st));
     if (na) {
-      BK(cudaMemcpyAsync(b->normals.p + 3 * ao, c->d_normals.p, na * 12, cudaMemcpyDeviceToDevice, st));
+      BK(cudaMemcpyAsync(b->normals.p + ao, c->d_normals4.p, na * 16, cudaMemcpyDeviceToDevice, st));
       BK(cudaMemcpyAsync(b->uvs.p + 2 * ao, c->d_uvs.p, na * 8, cudaMemcpyDeviceToDevice, st));
     }
     pt::launch_relocate(b->nodes.p + 5 * no, nn, (uint32_t)no, (uint32_t)po, b->prims.p + 3 * po, np,
@@ -274,7 +275,7 @@ static int ensure_wave(pt_batch* b, size_t results) {
     b->slot_f4.release();
     b->slot_u4.release();
     BK(b->slot_f4.ensure(s * PT_SLOT_F4));
-    BK(b->slot_u4.ensure(s * PT_SLOT_U4));
+    BK(b->slot_u4.ensure(PT_SLOTS_U4(s)));
     BK(b->d_ctr.ensure(1));
     BK(b->d_ctl.ensure(1));
     carve_wave(b->W, b->slot_f4.p, b->slot_u4.p, s);
@@ -428,7 +429,7 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
     for (const ScenePart& p : b->parts) lc.sort = lc.sort || sort_pays(p.ctx);
   lc.tex = 0;
   lc.motion = 0;
-  lc.lights = lc.env = 0;
+  lc.lights = lc.env = lc.one_grid = 0;
   for (const ScenePart& p : b->parts) {
     lc.tex = lc.tex || uses_textures(p.ctx);
     lc.motion = lc.motion || has_motion(p.ctx);

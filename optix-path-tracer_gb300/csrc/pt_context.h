@@ -138,6 +138,7 @@ struct pt_context {
   DevBuf<int> d_tex_list;
   DevBuf<uint4> d_tri_attr;
   DevBuf<float> d_normals, d_uvs;
+  DevBuf<float4> d_normals4;  // d_normals, one 16-byte vector per vertex
   DevBuf<uint32_t> d_leaf_of_id;
   DevBuf<float4> d_rec_in;  // primitive records in call order (GPU builder input)
   PinnedBuf<float4> h_rec;  // their host staging

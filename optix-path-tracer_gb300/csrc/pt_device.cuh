@@ -199,6 +199,35 @@ PTD PrimRec load_prim(const float4* prims, uint32_t i) {
   return p;
 }
 
+// Materials and lights are read as 16-byte vectors: 3 and 4 loads where their
+// fields one by one were up to 12 and 16, each touching as many sectors when
+// the lanes' records differ.
+PTD GpuMaterial load_material(const GpuMaterial* mats, uint32_t i) {
+  static_assert(sizeof(GpuMaterial) == 48, "three float4");
+  const float4* p = (const float4*)(mats + i);
+  const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+  GpuMaterial m;
+  m.type = __float_as_int(a.x);
+  m.c0x = a.y; m.c0y = a.z; m.c0z = a.w;
+  m.c1x = b.x; m.c1y = b.y; m.c1z = b.z;
+  m.p0 = b.w; m.p1 = c.x;
+  m.tex0 = __float_as_int(c.y);
+  m.tex1 = __float_as_int(c.z);
+  return m;
+}
+PTD GpuLight load_light(const GpuLight* lights, int i) {
+  static_assert(sizeof(GpuLight) == 64, "four float4");
+  const float4* p = (const float4*)(lights + i);
+  const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
+  GpuLight L;
+  L.type = __float_as_int(a.x);
+  L.axis = __float_as_int(a.y);
+  L.a0 = a.z; L.a1 = a.w; L.b0 = b.x; L.b1 = b.y; L.k = b.z;
+  L.cx = b.w; L.cy = c.x; L.cz = c.y; L.r = c.z;
+  L.ex = c.w; L.ey = d.x; L.ez = d.y;
+  return L;
+}
+
 // Centre of a sphere at `time`: the record's centre, or for a moving sphere
 // programs/hitables/moving_sphere.cu:47-49 (linear in time, also outside
 // [time0, time1]).
@@ -415,10 +444,9 @@ PTD HitRecord hit_record(const DevScene& S, const PrimRec& p, V3 ro, V3 rd, floa
     if (!(at.w & 1u)) {
       rec.shading_normal = Ng;
     } else {
-      const float* N = S.normals;
-      V3 na = v3(N[3 * at.x], N[3 * at.x + 1], N[3 * at.x + 2]);
-      V3 nb = v3(N[3 * at.y], N[3 * at.y + 1], N[3 * at.y + 2]);
-      V3 nc = v3(N[3 * at.z], N[3 * at.z + 1], N[3 * at.z + 2]);
+      V3 na = f4xyz(__ldg(S.normals + at.x));
+      V3 nb = f4xyz(__ldg(S.normals + at.y));
+      V3 nc = f4xyz(__ldg(S.normals + at.z));
       V3 Ns = na * b0 + nb * b1 + nc * b2;
       rec.shading_normal = normalize(Ns);
     }

@@ -52,6 +52,7 @@ struct LaunchCfg {
   int tex;             /* some material takes a texture: the texture variants of shading */
   int motion;          /* some sphere moves: the trace variants that carry ray times */
   int tail_grid;       /* blocks of the tail kernel: those resident at once */
+  int one_grid;        /* the scene's tree is one node: blocks of its trace kernel, else 0 */
   int lights;          /* some scene has lights */
   int env;             /* some scene has an importance-sampled environment */
 };
@@ -62,9 +63,10 @@ struct Ray3 {
 
 /* Counters of the streaming wavefront, in device memory. */
 struct WaveCounters {
-  uint32_t n_cur;        /* live paths at the start of the current buffer (before generation) */
-  uint32_t n_next;       /* paths written to the next buffer */
+  uint32_t n_next;       /* paths written to the next buffer; with n_shadow one 64-bit word
+                            for the appends that make both (push_both) */
   uint32_t n_shadow;     /* shadow rays queued this iteration */
+  uint32_t n_cur;        /* live paths at the start of the current buffer (before generation) */
   uint32_t n_occ;        /* consistent mode: occlusion rays of the current buffer's paths */
   uint32_t n_wait, n_wait_next; /* paths of the current / next buffer that have ended but
                             for their NEE term */
@@ -77,7 +79,6 @@ struct WaveCounters {
   unsigned long long iters_total; /* iterations over all chunks (batch) */
   uint32_t chunk;        /* current chunk of a batch */
   uint32_t n_chunks;     /* chunks of the batch (set by the host) */
-  uint32_t listed[8];    /* positions in each shading list (PT_SHADE_KEYS of them) */
   uint32_t ray_next[2];  /* rays taken by trace warps this iteration (extension, shadow) */
   uint32_t guide_rows;   /* positions listed for guide inference this iteration */
   uint32_t drained;      /* iterations since the chunk's last path was generated, that one
@@ -187,6 +188,7 @@ struct WaveState {
   PathBuf path[2];            /* ping-pong: path[parity] is current */
   float4* hit;                /* t, u, v, leaf index: by position in the current buffer */
   uint32_t* lists;            /* sorted shading: `slots` positions for each shading key */
+  uint32_t* listed;           /* positions on list k: listed[k * PT_LISTED_STRIDE] */
   ShadowBuf sh;               /* reference mode */
   NeeBuf nee[2];              /* consistent mode, beside path[]; shares sh's memory */
   WaveCounters* ctr;
@@ -203,8 +205,12 @@ struct WaveState {
  * uint4 entries: 3 states and an entry in each of the 8 shading lists. */
 #define PT_SLOT_F4 16
 #define PT_SLOT_U4 5
-/* Shading key of a hit: 0 none, 1 + material type. */
+/* Shading key of a hit: 0 none, 1 + material type.  Each list's counter has a
+ * cache line of its own, at the end of the uint4 block: the trace warps append
+ * to all of them all the time. */
 #define PT_SHADE_KEYS (PT_NUM_MAT_TYPES + 1)
+#define PT_LISTED_STRIDE 32
+#define PT_SLOTS_U4(s) ((size_t)(s) * PT_SLOT_U4 + PT_SHADE_KEYS * PT_LISTED_STRIDE / 4)
 
 /* Ray kinds of the trace kernels: closest hit of extension rays; closest
  * hit of a shadow ray (reference mode: the light must be the first thing
@@ -215,9 +221,11 @@ enum { TRACE_EXT = 0, TRACE_SHADOW = 1, TRACE_FIRST = 2, TRACE_OCCLUDED = 3, TRA
 namespace pt {
 /* Dynamic shared memory of a trace block (pt_trace.cu). */
 size_t trace_smem(int max_stack, int block);
+/* Resident blocks per SM of the trace kernel for trees of one node. */
+int one_blocks_per_sm();
 /* Resident trace blocks per SM (0 if the shape does not fit). */
 int trace_blocks_per_sm(int block, size_t smem);
-static_assert(PT_SHADE_KEYS == 8, "WaveCounters::listed, WaveState::lists");
+static_assert(PT_SHADE_KEYS == 8, "PT_SLOT_U4 holds the lists");
 /* One trace launch of `mode` (TRACE_EXT, TRACE_SHADOW or TRACE_BOTH)
  * over the wavefront's rays, with the launch shape of lc. */
 void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W,
@@ -241,7 +249,8 @@ void launch_chunk_begin(const WaveState& W, WaveCtl* ctl, const WaveCtl& v, bool
  * sample there are no shadow rays to trace or finish). */
 int iteration_kernels(const LaunchCfg& lc, int mode, bool guide);
 /* Resident blocks per SM x SMs for a trace (kind 0), shade (kind 1) or tail
- * (kind 2, blocks of PT_TAIL_BLOCK) kernel of `block` threads. */
+ * (kind 2, blocks of PT_TAIL_BLOCK) kernel of `block` threads, or for the
+ * trace kernel of one-node trees (kind 3). */
 int wave_grid(int kind, int max_stack, int block);
 /* Raises the dynamic shared memory limit of the trace kernels to the
  * device maximum (once per device). */
@@ -276,15 +285,18 @@ void launch_relocate(uint4* nodes, size_t n_nodes, uint32_t node_off, uint32_t p
 void launch_env_cdf(const float4* env, int w, int h, float* marg, float* cond, double* rows,
                     double* pre, int* valid, float2* row, uint16_t* marg_idx, int marg_bits,
                     uint16_t* cond_idx, int cond_bits, cudaStream_t st);
+/* Normals of 3 floats to 16-byte vectors. */
+void launch_pack_normals(const float* n3, size_t n, float4* n4, cudaStream_t st);
 void launch_accumulate(const float4* results, float4* acc, int w, int h, int frames,
                        cudaStream_t st);
 /* acc: 4 doubles per pixel (16-byte aligned) */
 void launch_accumulate64(const float4* results, double* acc, int w, int h, int frames,
                          cudaStream_t st);
 void launch_paths_out(const float4* results, float* out, uint32_t n, cudaStream_t st);
-/* First hits of the camera rays of one frame (grid: blocks of PT_TRACE_BLOCK). */
+/* First hits of the camera rays of one frame. */
 void launch_first_hits(const DevScene& S, int w, int h, int frame, uint32_t* prim, uint32_t* mat,
-                       float* t, int max_stack, uint32_t* err, int grid, cudaStream_t st);
+                       float* t, int max_stack, uint32_t* err, const LaunchCfg& lc,
+                       cudaStream_t st);
 void launch_resolve(const float4* acc, uchar4* out, int n, int frame, cudaStream_t st);
 }  // namespace pt
 

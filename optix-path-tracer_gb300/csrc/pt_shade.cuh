@@ -162,7 +162,7 @@ __device__ __forceinline__ int nee_begin(const DevScene& S, uint32_t& seed, V3 P
   if (numLights == 0) return 0;
   index = ((int)(rnd(seed) * numLights)) % numLights;
   if (isLight && numLights == 1) return 0;
-  GpuLight L = S.lights[index];
+  GpuLight L = load_light(S.lights, index);
   Wi = light_sample(L, P, seed);
   lightPDF = light_pdf(L, P, Wi);
   if (dot(Wi, N) < 0.f) return 0;
@@ -175,7 +175,7 @@ __device__ __forceinline__ V3 nee_end(const DevScene& S, const GpuMaterial& m, u
                                       bool occluded) {
   V3 directLight = v3(0.f);
   if (occluded) return v3(0.f);
-  GpuLight L = S.lights[index];
+  GpuLight L = load_light(S.lights, index);
   V3 emission = v3(L.ex, L.ey, L.ez);
   if (lightPDF != 0.f && !isNull(emission)) {
     float matPDF = 0.f;
@@ -307,7 +307,7 @@ __device__ __forceinline__ int shade_step(const DevScene& S, float4 hit, V3 ro, 
   PrimRec p = load_prim(S.prims, leaf);
   HitRecord rec = hit_record(S, p, ro, rd, hit.x, hit.y, hit.z, false, tm);
   n.mid = rec.index;
-  GpuMaterial m = S.mats[n.mid];
+  GpuMaterial m = load_material(S.mats, n.mid);
   n.textured = TEX && (m.tex0 >= 0 || m.tex1 >= 0);
   if (n.textured) {
     apply_textures(S, m, p, ro, rd, hit.x, hit.y, hit.z, tm);
@@ -395,7 +395,7 @@ __device__ __forceinline__ void finish_step(const DevScene& S, uint4& st, V3& th
                                             const NeeCtx& n, bool occluded, Tail& tl) {
   tl.event = 1;
   tl.isSpecular = false;
-  GpuMaterial m = S.mats[n.mid];
+  GpuMaterial m = load_material(S.mats, n.mid);
   if (m.tex0 >= 0) {  // NEE materials (Lambertian, Oren-Nayar, diffuse light) read only c0
     m.c0x = n.tcol.x;
     m.c0y = n.tcol.y;
@@ -419,7 +419,7 @@ __device__ __forceinline__ void env_eval(const DevScene& S, V3 d, V3& Le, float&
 // light selection), the MIS partner of BSDF sampling at emitter hits.
 __device__ __forceinline__ float lights_pdf_c(const DevScene& S, V3 P, V3 d, int n_sel) {
   float acc = 0.f;
-  for (int k = 0; k < S.num_lights; k++) acc += light_pdf(S.lights[k], P, d);
+  for (int k = 0; k < S.num_lights; k++) acc += light_pdf(load_light(S.lights, k), P, d);
   return acc / (float)n_sel;
 }
 
@@ -509,7 +509,7 @@ __device__ __forceinline__ void shade_step_c(const DevScene& S, const PathCtl& p
   } else {
     PrimRec p = load_prim(S.prims, leaf);
     HitRecord rec = hit_record(S, p, ro, d, hit.x, hit.y, hit.z, false, tm);
-    GpuMaterial m = S.mats[rec.index];
+    GpuMaterial m = load_material(S.mats, rec.index);
     if (TEX && (m.tex0 >= 0 || m.tex1 >= 0))
       apply_textures(S, m, p, ro, d, hit.x, hit.y, hit.z, tm);
     P = rec.P;
@@ -559,7 +559,7 @@ __device__ __forceinline__ void shade_step_c(const DevScene& S, const PathCtl& p
         V3 Le;
         tmax = PT_RAY_TMAX;
         if (k < S.num_lights) {
-          GpuLight L = S.lights[k];
+          GpuLight L = load_light(S.lights, k);
           if (L.type == PT_LIGHT_RECT) {
             Wi = light_sample(L, P, st.x);
             tmax = 1.f - 1e-4f;

@@ -117,7 +117,7 @@ struct DevScene {
   const uint4* tri_attr;    /* per prim id: absolute attribute-vertex indices (x,y,z),
                                .w bit0 = has normals, bit1 = has uvs, bits 2-31 the
                                face's texture index (mesh.hpp material_buffer) */
-  const float* normals;     /* 3 floats per attribute vertex */
+  const float4* normals;    /* per attribute vertex, w unused */
   const float* uvs;         /* 2 floats per attribute vertex */
   const uint32_t* leaf_of_id; /* primitive id -> position in the leaf-ordered records */
   const float* env_marg;    /* environment sampling: marginal CDF over rows (h+1) */
