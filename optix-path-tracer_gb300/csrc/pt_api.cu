@@ -46,6 +46,8 @@ static int fail(pt_context* ctx, int code, const std::string& msg) {
   return code;
 }
 
+static const size_t kHostHits = 16384;  // rays of a first-hit query answered through host memory
+
 static const char* const kOtherDevice =
     "buffer is device memory of another GPU than the context's (pt_options.device)";
 
@@ -230,7 +232,9 @@ PT_API int pt_context_create(const pt_options* opt, pt_context** out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_ctr, 2 * sizeof(WaveCounters));
+  if (e == cudaSuccess)
+    e = cudaMallocHost((void**)&ctx->h_ctr, 2 * sizeof(WaveCounters) + (3 * kHostHits + 1) * 4);
+  if (e == cudaSuccess) ctx->h_hits = (uint32_t*)(ctx->h_ctr + 2);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->evc[0], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->evc[1], cudaEventDisableTiming);
   if (e != cudaSuccess) {
@@ -1583,6 +1587,24 @@ PT_API int pt_trace_first_hits(pt_context* ctx, int width, int height, int frame
   CK(cudaEventRecord(ctx->ev0, (cudaStream_t)stream));
   CK(cudaStreamWaitEvent(st, ctx->ev0, 0));
   size_t WH = (size_t)width * height;
+  if (WH <= kHostHits && device_ptr_kind(prim, ctx->device) == 0 &&
+      device_ptr_kind(mat, ctx->device) == 0 && device_ptr_kind(t, ctx->device) == 0) {
+    // a small query is all latency: the kernel writes its 12 bytes a ray to
+    // page-locked memory, with no clear before it and no copies behind it
+    // (96 x 64 rays of the Cornell box on a GB300: 66 -> 31 us a call)
+    uint32_t* h = ctx->h_hits;
+    h[3 * kHostHits] = 0;  // the error word
+    pt::launch_first_hits(ctx->scene, width, height, frame, h, h + kHostHits,
+                          (float*)(h + 2 * kHostHits), ctx->max_stack, h + 3 * kHostHits, ctx->lc,
+                          st);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(st));
+    if (h[3 * kHostHits]) return fail(ctx, PT_EQUEUE, "traversal stack overflow");
+    memcpy(prim, h, WH * 4);
+    memcpy(mat, h + kHostHits, WH * 4);
+    memcpy(t, h + 2 * kHostHits, WH * 4);
+    return PT_OK;
+  }
   CK(ctx->d_tmpu.ensure(2 * WH + 1));
   CK(ctx->d_tmp.ensure(WH));
   uint32_t* d_err = ctx->d_tmpu.p + 2 * WH;

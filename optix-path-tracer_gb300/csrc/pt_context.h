@@ -169,6 +169,7 @@ struct pt_context {
   DevBuf<float> d_tmp;
   DevBuf<uint32_t> d_tmpu;
   WaveCounters* h_ctr = nullptr;  // pinned, 2 (the counters after each of two graph launches)
+  uint32_t* h_hits = nullptr;     // behind h_ctr: results of small first-hit queries
   cudaGraphExec_t graph = nullptr;
   cudaGraphExec_t graph2 = nullptr;  // a second instance on its own timing events (timing)
   bool graph_loop = false;   // graph is the device loop (else iterations for the host loop)
