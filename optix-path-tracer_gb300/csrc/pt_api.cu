@@ -1144,7 +1144,7 @@ static WaveCtl chunk_ctl(const pt_context* ctx, const pt_render_params* p, int f
   ctl.mode = p->mode;
   ctl.guide = p->guide;
   ctl.guide_depth = ctx->guide.max_bounces > 0 ? (uint32_t)ctx->guide.max_bounces : 0xffffffffu;
-  ctl.tail_max = pt::tail_paths(ctx->max_stack);
+  ctl.tail_max = pt::tail_paths(ctx->max_stack, ctx->lc);
   ctl.chunk_paths = (unsigned long long)p->width * p->height * frames;
   fastdiv_magic((uint32_t)(p->width * p->height), &ctl.wh_m, &ctl.wh_l);
   fastdiv_magic((uint32_t)p->width, &ctl.w_m, &ctl.w_l);

@@ -569,7 +569,7 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
   WaveCtl hc;
   memset(&hc, 0, sizeof(hc));
   hc.mode = mode;
-  hc.tail_max = pt::tail_paths(b->max_stack);
+  hc.tail_max = pt::tail_paths(b->max_stack, b->lc);
   BK(cudaMemcpyAsync(b->d_ctl.p, &hc, sizeof(hc), cudaMemcpyHostToDevice, st));
   BatchRefs br{b->d_scenes.p, b->d_segs.p, b->d_roots.p};
   if (timing && b->tev.empty()) {

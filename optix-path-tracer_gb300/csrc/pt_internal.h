@@ -34,6 +34,15 @@
 #ifndef PT_TAIL_PATHS
 #define PT_TAIL_PATHS 16384
 #endif
+/* The same where a material has an image or noise texture: a textured bounce
+ * is several times as long a chain of dependent loads, which a warp of one
+ * path cannot hide.  GB300, us per render with 2048 / 4096 / 8192 / 16384:
+ * textures 61x82, 3 frames 799 / 822 / 910 / 1157 (consistent mode 416 / 431 /
+ * 468 / 580), 321x243 one frame 1035 / 1053 / 1176 / 1356 and 33 frames 2112 /
+ * 2121 / 2191 / 2287; 60x40 one frame 342 / 243 / 242 / 245. */
+#ifndef PT_TAIL_PATHS_TEX
+#define PT_TAIL_PATHS_TEX 4096
+#endif
 
 /* Path state word st.z: depth (bits 0-15), previous bounce specular (bit 16),
  * scene of a batch (bits 17-31). */
@@ -231,9 +240,10 @@ static_assert(PT_SHADE_KEYS == 8, "PT_SLOT_U4 holds the lists");
 void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W,
                   const WaveCtl* ctl, int max_stack, const BatchRefs* br, const LaunchCfg& lc,
                   cudaStream_t st);
-/* WaveCtl.tail_max for a BVH of this stack depth: PT_TAIL_PATHS, or 0 where
- * the tail kernel's stacks would not fit in shared memory. */
-uint32_t tail_paths(int max_stack);
+/* WaveCtl.tail_max for a BVH of this stack depth and launch shape:
+ * PT_TAIL_PATHS (PT_TAIL_PATHS_TEX where lc.tex), or 0 where the tail
+ * kernel's stacks would not fit in shared memory. */
+uint32_t tail_paths(int max_stack, const LaunchCfg& lc);
 /* Resident tail blocks per SM (pt_tail.cu). */
 int tail_blocks_per_sm(int max_stack);
 /* The chunk's last paths, each to its end, when at most tail_max are left

@@ -300,12 +300,13 @@ int tail_occupancy(K k, int max_stack) {
 
 namespace pt {
 
-uint32_t tail_paths(int max_stack) {
-  return tail_smem(max_stack) <= kMaxSmem ? PT_TAIL_PATHS : 0u;
+uint32_t tail_paths(int max_stack, const LaunchCfg& lc) {
+  if (tail_smem(max_stack) > kMaxSmem) return 0u;
+  return lc.tex ? PT_TAIL_PATHS_TEX : PT_TAIL_PATHS;
 }
 
 int tail_blocks_per_sm(int max_stack) {
-  if (!tail_paths(max_stack)) return 1;
+  if (tail_smem(max_stack) > kMaxSmem) return 1;
   int a = tail_occupancy(k_tail<0, false>, max_stack), b = tail_occupancy(k_tail<1, false>, max_stack);
   int c = tail_occupancy(k_tail<0, true>, max_stack), d = tail_occupancy(k_tail<1, true>, max_stack);
   int m = a < b ? a : b;
@@ -316,7 +317,7 @@ int tail_blocks_per_sm(int max_stack) {
 void launch_tail(const DevScene& S, const WaveState& W, const WaveCtl* ctl, int max_stack,
                  bool counters, const LaunchCfg& lc, int mode, const BatchRefs* br, bool mark,
                  cudaStream_t st) {
-  if (!tail_paths(max_stack)) return;  // the wavefront drains to the last path
+  if (tail_smem(max_stack) > kMaxSmem) return;  // the wavefront drains to the last path
   const size_t smem = tail_smem(max_stack);
   const BatchRefs b = br ? *br : BatchRefs{};
   const int cnt = counters ? 1 : 0;

@@ -33,3 +33,18 @@ def test_tail_sizes(ptgb_mod, oracle_mod, mode, w, h, spp, slots):
     assert ts["ext_rays"] == gs["ext_rays"] and ts["node_fetches"] > 0
     g.close()
     t.close()
+
+
+# with image or noise textures 4096 paths and fewer are one tail launch
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("w", [64, 65])
+def test_tail_sizes_textured(ptgb_mod, oracle_mod, mode, w):
+    s = ptgb_mod.texture_zoo(w, 64)
+    g, o = ptgb_mod.GpuRenderer(s), oracle_mod.Oracle(s)
+    acc = g.render(ptgb_mod.GpuRenderer.params(w, 64, 1, mode=mode))
+    ref, st = o.render(w, 64, 1, mode=mode)
+    assert np.array_equal(acc[..., 3], ref[..., 3])
+    assert rel_err(acc[..., :3], ref[..., :3]).max() <= REL_TOL
+    gs = g.stats()
+    assert gs["ext_rays"] == st["ext_rays"] and gs["shadow_rays"] == st["shadow_rays"]
+    g.close()
