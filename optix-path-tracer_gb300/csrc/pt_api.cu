@@ -1366,16 +1366,17 @@ static void reset_render_stats(pt_context* ctx) {
 
 }  // extern "C"
 
-// Rays through a large scene take many more steps, with a wider spread, so
-// lanes refill earlier (a quarter of the warp idle) rather than waiting for
-// the whole warp; rays through a small scene are short and alike.  (GB300,
-// 1080p: 2.1M-triangle heightfield 24 lanes +6% over 32; 488 spheres 32
-// lanes +1% over 24.)
 bool pth::has_motion(const pt_context* ctx) { return ctx->num_moving > 0; }
 
 bool pth::all_triangles(const pt_context* ctx) { return ctx->num_non_triangles == 0; }
 
-int pth::auto_refetch(size_t num_prims) { return num_prims > ((size_t)1 << 16) ? 24 : 32; }
+// Rays through a large scene take many more steps, with a wider spread, so
+// lanes refill earlier (an eighth of the warp busy) rather than waiting for
+// the whole warp; rays through a small scene are short and alike.  GB300, ms
+// with 8 / 16 / 20 / 24 / 28 / 32 idle lanes: 2.1 M triangle heightfield
+// 1080p, 64 frames 70.8 / 68.4 / 66.7 / 64.9 / 64.0 / 67.3; 488 spheres
+// 1080p, 128 frames 180 / 163 / 159.5 / 157.6 / 155.8 / 156.2.
+int pth::auto_refetch(size_t num_prims) { return num_prims > ((size_t)1 << 16) ? 28 : 32; }
 
 bool pth::sort_pays(const pt_context* ctx) {
   for (const GpuMaterial& m : ctx->mats)
