@@ -61,6 +61,31 @@ struct Bvh8Out {
 // against 76.3 ms.)  Trees of scenes with shapes other than triangles are
 // built without it, as their images have been; the clustered trees of triangle
 // meshes with it.
+//
+// box_grid: the exponent of a node's step along one axis and the grid's
+// origin p, for the node's bounds [lo, hi].
+PT_BVH_HD inline int box_grid(float lo, float hi, bool guard, float& p) {
+  p = lo;
+  const float ext = hi - lo;
+  int ex = -126;
+  if (ext > 0.f) {
+    int k;
+    frexpf(ext / 255.0f, &k);
+    ex = k;
+    while (ex > -126 && ldexpf(255.0f, ex - 1) >= ext) ex--;
+    while (ldexpf(255.0f, ex) < ext) ex++;
+    if (ex < -126) ex = -126;
+  }
+  if (guard) {  // the origin may round downward by more than a step
+    p = lo - ldexpf(1.0f, ex);
+    while (hi - p > ldexpf(254.0f, ex)) {
+      ex++;
+      p = lo - ldexpf(1.0f, ex);
+    }
+  }
+  return ex;
+}
+
 PT_BVH_HD inline void encode_node_dev(const Box& parent, const WideChild* ch, int nch,
                                       uint32_t child_base, uint32_t prim_base, uint32_t out[20],
                                       bool guard = false) {
@@ -68,24 +93,7 @@ PT_BVH_HD inline void encode_node_dev(const Box& parent, const WideChild* ch, in
   uint32_t e[3];
   float p[3], step[3];
   for (int a = 0; a < 3; a++) {
-    p[a] = parent.lo[a];
-    float ext = parent.hi[a] - parent.lo[a];
-    int ex = -126;
-    if (ext > 0.f) {
-      int k;
-      frexpf(ext / 255.0f, &k);
-      ex = k;
-      while (ex > -126 && ldexpf(255.0f, ex - 1) >= ext) ex--;
-      while (ldexpf(255.0f, ex) < ext) ex++;
-      if (ex < -126) ex = -126;
-    }
-    if (guard) {  // the origin may round downward by more than a step
-      p[a] = parent.lo[a] - ldexpf(1.0f, ex);
-      while (parent.hi[a] - p[a] > ldexpf(254.0f, ex)) {
-        ex++;
-        p[a] = parent.lo[a] - ldexpf(1.0f, ex);
-      }
-    }
+    const int ex = box_grid(parent.lo[a], parent.hi[a], guard, p[a]);
     e[a] = (uint32_t)(ex + 127);
     step[a] = ldexpf(1.0f, ex);
   }
@@ -193,11 +201,13 @@ PT_BVH_HD inline bool check_node8(const uint32_t* w, uint64_t k, uint64_t nn, ui
 }
 
 inline void encode_node(const Box& parent, const WideChild* ch, int nch, uint32_t child_base,
-                        uint32_t prim_base, uint32_t out[20]) {
-  encode_node_dev(parent, ch, nch, child_base, prim_base, out);
+                        uint32_t prim_base, uint32_t out[20], bool guard = false) {
+  encode_node_dev(parent, ch, nch, child_base, prim_base, out, guard);
 }
-/* width: most children per node, 2..8 (the node format holds 8) */
-int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width = 8);
+/* width: most children per node, 2..8 (the node format holds 8).  fit: wide
+ * nodes chosen by the cost of the quantised boxes, on guarded grids
+ * (encode_node_dev); else by the largest area, without. */
+int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width = 8, bool fit = false);
 bool validate_bvh8(const Bvh8Out& b, size_t num_prims);
 
 }  // namespace pt

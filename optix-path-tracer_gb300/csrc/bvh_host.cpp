@@ -20,7 +20,7 @@ namespace {
 struct BNode {
   Box box;
   int left = -1, right = -1;  // internal children
-  int first = 0, count = 0;   // leaf range in `order`
+  int first = 0, count = 0;   // range in `order` (count: leaves only)
   int nprims = 0;             // primitives in the subtree
 };
 
@@ -51,7 +51,9 @@ struct Bvh2 {
   std::vector<float> cx, cy, cz;
   std::vector<uint32_t>& order;
   std::vector<BNode> nodes;
-  Bvh2(const std::vector<Box>& b, std::vector<uint32_t>& o) : boxes(b), order(o) {
+  const int leaf;  // most primitives of a leaf
+  Bvh2(const std::vector<Box>& b, std::vector<uint32_t>& o, int most)
+      : boxes(b), order(o), leaf(most) {
     size_t n = b.size();
     cx.resize(n);
     cy.resize(n);
@@ -79,9 +81,23 @@ struct Bvh2 {
     int n = end - begin;
     nodes[ni].box = bb;
     nodes[ni].nprims = n;
-    if (n <= 3) {
-      nodes[ni].first = begin;
+    nodes[ni].first = begin;
+    if (n <= leaf) {
       nodes[ni].count = n;
+      return ni;
+    }
+    if (n <= 3) {  // leaf 1: the pair with the smaller box
+      if (n == 3) {
+        uint32_t* q = &order[begin];
+        const float a01 = half_area(merge(boxes[q[0]], boxes[q[1]]));
+        const float a02 = half_area(merge(boxes[q[0]], boxes[q[2]]));
+        const float a12 = half_area(merge(boxes[q[1]], boxes[q[2]]));
+        if (a12 < a01 && a12 <= a02) std::swap(q[0], q[2]);
+        else if (a02 < a01) std::swap(q[1], q[2]);
+      }
+      const int l = build(begin, end - 1), r = build(end - 1, end);
+      nodes[ni].left = l;
+      nodes[ni].right = r;
       return ni;
     }
     const int NB = 32;
@@ -146,12 +162,126 @@ struct Bvh2 {
   }
 };
 
+// Wide nodes by cost.  The cost of a subtree is that of its wide nodes (one
+// each) and of its leaves' primitives (kCostPrim each), times the area of the
+// box that a ray is tested against before it reaches them: the child's box as
+// it is quantised in its parent's grid.  That is the point of it: where a
+// scene's bounds are much larger than most of its primitives, the root's step
+// is as large as they are, and children cut small under the root would all be
+// hit by every ray that comes near them.  By this cost they go into a node of
+// their own with a fine grid (random spheres on a ground sphere of radius
+// 1000: the root's step is 8, the spheres' diameter 0.4).
+// GB300, by area -> by cost: 488 spheres 8.6 -> 3.9 node fetches a ray,
+// 1920x1080 128 frames 155.8 -> 110 ms, one frame 2.03 -> 1.48 ms; 104 moving
+// ones 1.60 -> 1.26 ms; the textures scene 2.14 -> 2.02 ms; commit of the 488
+// spheres 0.35 -> 0.53 ms.
+// A primitive test against a node step: 0.15 / 0.2 / 0.3 / 0.4 / 0.6 gave
+// 110.6 / 110.7 / 109.7 / 111.5 / 112.1 ms on the spheres.
+#ifndef PT_FIT_PRIM
+#define PT_FIT_PRIM 0.3f
+#endif
+constexpr float kCostPrim = PT_FIT_PRIM;
+
+struct Fit {
+  const std::vector<BNode>& B;
+  const int width;
+  std::vector<float> inner;   // a node's cost below itself, as a wide node
+  std::vector<uint8_t> split; // per node under the current wide node: slots of its left child by
+                              // its own slots (0: it takes one)
+  float p[3], step[3], inv[3];
+
+  Fit(const std::vector<BNode>& b, int w) : B(b), width(w), inner(w ? b.size() : 0, 0.f),
+                                         split(9 * inner.size(), 0) {
+    for (size_t k = w ? b.size() : 0; k-- > 0;)  // children come after their parents
+      if (b[k].left >= 0) inner[k] = open((int)k);
+  }
+  float area(int c) const {  // of its box in the current wide node's grid
+    float e[3];
+    for (int a = 0; a < 3; a++) {
+      const float lo = std::floor((B[c].box.lo[a] - p[a]) * inv[a] - PT_BOX_SLACK);
+      const float hi = std::ceil((B[c].box.hi[a] - p[a]) * inv[a] + PT_BOX_SLACK);
+      e[a] = (hi - lo) * step[a];
+    }
+    return e[0] * e[1] + e[1] * e[2] + e[2] * e[0];
+  }
+  // as one child of the current wide node: a leaf, or a wide node of its own
+  float slot(int c, bool* leaf = nullptr) const {
+    const float a = area(c), node = a + inner[c], prims = kCostPrim * a * (float)B[c].nprims;
+    const bool is_leaf = B[c].left < 0 || (B[c].nprims <= 3 && prims <= node);
+    if (leaf) *leaf = is_leaf;
+    return is_leaf ? prims : node;
+  }
+  // cost[k]: the subtree of c in at most k slots, k = 1..most
+  void share(int c, int most, float* cost) {
+    uint8_t* s = &split[9 * (size_t)c];
+    cost[1] = slot(c);
+    s[1] = 0;
+    if (most < 2) return;
+    for (int k = 2; k <= most; k++) {
+      cost[k] = cost[1];
+      s[k] = 0;
+    }
+    if (B[c].left < 0) return;
+    float l[9], r[9];
+    share(B[c].left, most - 1, l);
+    share(B[c].right, most - 1, r);
+    for (int k = 2; k <= most; k++) {
+      if (cost[k - 1] < cost[k]) {
+        cost[k] = cost[k - 1];
+        s[k] = s[k - 1];
+      }
+      for (int i = 1; i < k; i++)
+        if (l[i] + r[k - i] < cost[k]) {
+          cost[k] = l[i] + r[k - i];
+          s[k] = (uint8_t)(i | (k << 4));
+        }
+    }
+  }
+  // node x as a wide node: its children's cost, their shares left in `split`
+  float open(int x) {
+    for (int a = 0; a < 3; a++) {
+      const int ex = box_grid(B[x].box.lo[a], B[x].box.hi[a], true, p[a]);
+      step[a] = std::ldexp(1.0f, ex);
+      inv[a] = std::ldexp(1.0f, -ex);
+    }
+    float l[9], r[9];
+    share(B[x].left, width - 1, l);
+    share(B[x].right, width - 1, r);
+    float best = FLT_MAX;
+    uint8_t& s = split[9 * (size_t)x];
+    s = 1 | (2 << 4);  // where no cost is a number
+    for (int k = 2; k <= width; k++)
+      for (int i = 1; i < k; i++)
+        if (l[i] + r[k - i] < best) {
+          best = l[i] + r[k - i];
+          s = (uint8_t)(i | (k << 4));
+        }
+    return best;
+  }
+  void take(int c, int k, std::vector<int>& kids) const {
+    const uint8_t s = split[9 * (size_t)c + k];
+    if (s == 0) {
+      kids.push_back(c);
+      return;
+    }
+    take(B[c].left, s & 15, kids);
+    take(B[c].right, (s >> 4) - (s & 15), kids);
+  }
+  // the children of node x as a wide node
+  void children(int x, std::vector<int>& kids) {
+    open(x);
+    const uint8_t s = split[9 * (size_t)x];
+    take(B[x].left, s & 15, kids);
+    take(B[x].right, (s >> 4) - (s & 15), kids);
+  }
+};
+
 }  // namespace
 
 // The quantisation grid of encode_node extends the parent box upward by up
 // to 255 steps; the parent itself must cover the children, which the caller
 // guarantees (parent = union of children).
-int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width) {
+int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width, bool fit) {
   if (width < 2 || width > 8) width = 8;
   size_t n = boxes.size();
   out.nodes.clear();
@@ -160,10 +290,11 @@ int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width) {
   if (n == 0) return 0;
   std::vector<uint32_t> order(n);
   for (size_t i = 0; i < n; i++) order[i] = (uint32_t)i;
-  Bvh2 b2(boxes, order);
+  Bvh2 b2(boxes, order, fit ? 1 : 3);
   b2.nodes.reserve(2 * n);
   b2.build(0, (int)n);
   const std::vector<BNode>& B = b2.nodes;
+  Fit cost(B, fit ? width : 0);
 
   // breadth-first emission of wide nodes; each wide node records the binary
   // node it expands
@@ -185,6 +316,8 @@ int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width) {
     const BNode& bn = B[pd.bnode];
     if (bn.left < 0) {
       kids.push_back(pd.bnode);  // single-leaf root
+    } else if (fit) {
+      cost.children(pd.bnode, kids);
     } else {
       kids.push_back(bn.left);
       kids.push_back(bn.right);
@@ -216,22 +349,13 @@ int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width) {
       const BNode& c = B[kids[k]];
       wc[k].box = c.box;
       parent = merge(parent, c.box);
-      if (c.nprims <= 3) {
+      bool leaf = c.nprims <= 3;
+      if (fit && c.left >= 0) cost.slot(kids[k], &leaf);
+      if (leaf) {
         wc[k].internal = false;
         wc[k].count = (uint32_t)c.nprims;
         wc[k].prim_off = off;
-        // collect the subtree's primitives (a leaf, or a small internal node)
-        std::vector<int> st{kids[k]};
-        while (!st.empty()) {
-          int x = st.back();
-          st.pop_back();
-          if (B[x].left < 0) {
-            for (int q = 0; q < B[x].count; q++) out.leaf_order.push_back(order[B[x].first + q]);
-          } else {
-            st.push_back(B[x].right);
-            st.push_back(B[x].left);
-          }
-        }
+        for (int q = 0; q < c.nprims; q++) out.leaf_order.push_back(order[c.first + q]);
         off += (uint32_t)c.nprims;
       } else {
         wc[k].internal = true;
@@ -241,7 +365,7 @@ int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width) {
       }
     }
     out.nodes.resize(queue.size() * 20);
-    encode_node(parent, wc, nch, child_base, prim_base, &out.nodes[(size_t)self * 20]);
+    encode_node(parent, wc, nch, child_base, prim_base, &out.nodes[(size_t)self * 20], fit);
   }
   return 0;
 }

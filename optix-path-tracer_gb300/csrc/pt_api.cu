@@ -842,6 +842,30 @@ static void prim_record(const HostPrim& p, uint32_t id, float4* out) {
 
 }  // extern "C"
 
+// Levels whose traversal stacks fit at every trace block size: a tree chosen
+// for speed is no deeper than that, or than the one it replaces.
+constexpr int kShallow = 8;
+
+// Whether the host builder chooses wide nodes by cost on guarded grids.  Not
+// where an edge of a rectangle or a box is one of the scene's bounds (a closed
+// room): such trees stay as their images have been (encode_node_dev).
+static bool fits(const pt_context* ctx, const std::vector<pt::Box>& boxes) {
+  pt::Box all = boxes[0];
+  for (const pt::Box& b : boxes)
+    for (int a = 0; a < 3; a++) {
+      all.lo[a] = std::min(all.lo[a], b.lo[a]);
+      all.hi[a] = std::max(all.hi[a], b.hi[a]);
+    }
+  for (size_t i = 0; i < boxes.size(); i++) {
+    const int type = ctx->prims[i].type;
+    if (type == PT_PRIM_TRIANGLE || type == PT_PRIM_SPHERE) continue;
+    int on = 0;
+    for (int a = 0; a < 3; a++) on += boxes[i].lo[a] <= all.lo[a] || boxes[i].hi[a] >= all.hi[a];
+    if (on >= 2) return false;
+  }
+  return true;
+}
+
 // Builds the BVH8 of the scene's primitives (transforms already on the
 // device) into nodes / leaf-ordered records / leaf_of_id, with at most
 // `width` children per node, and checks its structure on the host.
@@ -852,7 +876,16 @@ int pth::build_bvh(pt_context* ctx, int width, DevBuf<uint4>& d_nodes, DevBuf<fl
   cudaStream_t st = ctx->stream;
   size_t n = ctx->prims.size();
   int builder = ctx->opt.bvh_builder;
-  if (builder == 0) builder = n >= 4096 ? 2 : 1;
+  // GB300, commit of a triangle mesh by the host / GPU builder, ms: 512
+  // triangles 0.53 / 0.53, 800 0.87 / 0.51, 3200 3.55 / 0.54, and the renders
+  // within 2 % (the host's trees by area: 800 0.5, 3200 2.3, renders +1..10 %).
+  // Other scenes' device trees are by Morton code and area, without guarded
+  // grids; up to 4096 primitives the host's are worth their time.
+  bool retry = false;  // the host builds it instead if the GPU's tree is deep or fails its check
+  if (builder == 0) {
+    builder = n >= (all_triangles(ctx) ? 512u : 4096u) ? 2 : 1;
+    retry = n < 4096;
+  }
   pt::Bvh8Out bvh;
   size_t nn = 0;
   if (builder == 2 && n > 0) {
@@ -882,15 +915,29 @@ int pth::build_bvh(pt_context* ctx, int width, DevBuf<uint4>& d_nodes, DevBuf<fl
                           d_prims.p, d_leaf_of_id.p, &nodes, &depth, width,
                           all_triangles(ctx),
                           ctx->cam.time0, ctx->cam.time1, &ctx->build_arena, st));
-    if (depth < 0)
+    retry = retry && (depth < 0 || depth > kShallow);
+    if (depth < 0 && !retry)
       return fail(ctx, PT_EINVAL,
                   "GPU BVH8 failed validation (check " + std::to_string(-depth) + ")");
     nn = nodes;
     bvh.depth = depth;  // the builder checked the tree's structure on the device
-  } else {
+  }
+  if (builder != 2 || n == 0 || retry) {
     std::vector<pt::Box> boxes(n);
     for (size_t i = 0; i < n; i++) boxes[i] = prim_box(ctx, ctx->prims[i]);
-    if (n) pt::build_bvh8_host(boxes, bvh, width);
+    bool fit = n > 0 && fits(ctx, boxes);
+    if (n > 0 && (!fit || n <= 24)) {
+      pt::build_bvh8_host(boxes, bvh, width);
+      fit = fit && bvh.nodes.size() > 20;  // one node stays one: it has a kernel of its own
+    }
+    if (fit) {
+      pt::build_bvh8_host(boxes, bvh, width, true);
+      if (bvh.depth > kShallow) {  // no deeper than by area
+        pt::Bvh8Out by_area;
+        pt::build_bvh8_host(boxes, by_area, width);
+        if (by_area.depth < bvh.depth) std::swap(bvh, by_area);
+      }
+    }
     if (!pt::validate_bvh8(bvh, n)) return fail(ctx, PT_EINVAL, "BVH8 failed validation");
     // primitive records in leaf order
     std::vector<float4> rec(3 * (n ? n : 1));
