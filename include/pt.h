@@ -73,7 +73,7 @@ typedef struct pt_options {
                           Oren-Nayar, Torrance-Sparrow or Ashikhmin-Shirley), 1 sorted,
                           2 path order */
   int refetch_lanes;   /* idle lanes of a trace warp that take new rays together, 1..32;
-                          0 automatic (24 for scenes of more than 2^16 primitives, else 32) */
+                          0 automatic (28) */
 } pt_options;
 
 typedef struct pt_render_params {

@@ -1093,7 +1093,7 @@ PT_API int pt_commit(pt_context* ctx) {
   CK(pt::set_trace_smem());
   ctx->lc = pt::default_launch(ctx->max_stack);
   ctx->lc.sort = ctx->opt.shade_order == 1 || (ctx->opt.shade_order == 0 && pth::sort_pays(ctx));
-  ctx->lc.refetch = ctx->opt.refetch_lanes ? ctx->opt.refetch_lanes : pth::auto_refetch(n);
+  ctx->lc.refetch = ctx->opt.refetch_lanes ? ctx->opt.refetch_lanes : pth::kAutoRefetch;
   ctx->lc.tex = pth::uses_textures(ctx) ? 1 : 0;
   ctx->lc.motion = pth::has_motion(ctx) ? 1 : 0;
   if (nn == 1) ctx->lc.one_grid = pt::wave_grid(3, ctx->max_stack, 0);
@@ -1416,14 +1416,6 @@ static void reset_render_stats(pt_context* ctx) {
 bool pth::has_motion(const pt_context* ctx) { return ctx->num_moving > 0; }
 
 bool pth::all_triangles(const pt_context* ctx) { return ctx->num_non_triangles == 0; }
-
-// Rays through a large scene take many more steps, with a wider spread, so
-// lanes refill earlier (an eighth of the warp busy) rather than waiting for
-// the whole warp; rays through a small scene are short and alike.  GB300, ms
-// with 8 / 16 / 20 / 24 / 28 / 32 idle lanes: 2.1 M triangle heightfield
-// 1080p, 64 frames 70.8 / 68.4 / 66.7 / 64.9 / 64.0 / 67.3; 488 spheres
-// 1080p, 128 frames 180 / 163 / 159.5 / 157.6 / 155.8 / 156.2.
-int pth::auto_refetch(size_t num_prims) { return num_prims > ((size_t)1 << 16) ? 28 : 32; }
 
 bool pth::sort_pays(const pt_context* ctx) {
   for (const GpuMaterial& m : ctx->mats)

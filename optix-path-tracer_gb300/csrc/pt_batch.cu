@@ -437,12 +437,7 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
     lc.env = lc.env || p.ctx->scene.env_valid;
   }
   lc.tail_grid = pt::wave_grid(2, b->max_stack, PT_TAIL_BLOCK);
-  lc.refetch = b->tune.refetch_lanes;
-  if (lc.refetch == 0) {  // automatic: by the largest scene of the batch
-    size_t most = 0;
-    for (const ScenePart& p : b->parts) most = std::max(most, p.ctx->prims.size());
-    lc.refetch = auto_refetch(most);
-  }
+  lc.refetch = b->tune.refetch_lanes ? b->tune.refetch_lanes : kAutoRefetch;
   b->lc = lc;
   // accumulators: the items' device buffers, or device copies of host ones
   std::vector<float4*> acc(n);

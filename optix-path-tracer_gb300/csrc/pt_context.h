@@ -211,7 +211,13 @@ bool has_motion(const pt_context* ctx);
  * one of the costly BRDFs (Oren-Nayar, Torrance-Sparrow, Ashikhmin-Shirley)
  * is present, whose code paths diverge most in a mixed warp. */
 bool sort_pays(const pt_context* ctx);
-int auto_refetch(size_t num_prims);
+/* Idle lanes of a trace warp that take new rays together, unless the caller
+ * says: ray lengths differ too much to wait for the whole warp, and a batch
+ * of loads should serve many lanes.  GB300, ms with 8 / 16 / 20 / 24 / 28 / 32:
+ * 2.1 M triangle heightfield 1080p, 64 frames 71.0 / 68.5 / 66.7 / 65.0 / 64.1
+ * / 67.4; 488 spheres 1080p, 128 frames 114.5 / 107.9 / 106.0 / 107.2 / 105.6 /
+ * 109.7; smaller renders within 1 % from 20 on. */
+constexpr int kAutoRefetch = 28;
 /* Padded world box of one primitive (the BVH builders' leaf box). */
 pt::Box prim_bounds(const pt_context* ctx, const HostPrim& p);
 /* Allocates the guide's buffers and finds the scene box of its position
