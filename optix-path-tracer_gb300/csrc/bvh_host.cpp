@@ -100,7 +100,7 @@ struct Bvh2 {
       nodes[ni].right = r;
       return ni;
     }
-    const int NB = 32;
+    const int NB = 32, nb = leaf == 1 ? std::min(NB, 2 * n) : NB;  // few for few
     float best = FLT_MAX;
     int best_ax = -1, best_bin = -1;
     for (int ax = 0; ax < 3; ax++) {
@@ -108,11 +108,11 @@ struct Bvh2 {
       if (!(hi - lo > 0.f)) continue;
       Box bins[NB];
       int cnt[NB] = {0};
-      for (int k = 0; k < NB; k++) bins[k] = empty_box();
-      float scale = NB / (hi - lo);
+      for (int k = 0; k < nb; k++) bins[k] = empty_box();
+      float scale = nb / (hi - lo);
       for (int k = begin; k < end; k++) {
         uint32_t p = order[k];
-        int b = std::min(NB - 1, std::max(0, (int)((cen(p, ax) - lo) * scale)));
+        int b = std::min(nb - 1, std::max(0, (int)((cen(p, ax) - lo) * scale)));
         cnt[b]++;
         bins[b] = merge(bins[b], boxes[p]);
       }
@@ -120,7 +120,7 @@ struct Bvh2 {
       int lc[NB];
       Box acc = empty_box();
       int c = 0;
-      for (int k = 0; k < NB; k++) {
+      for (int k = 0; k < nb; k++) {
         acc = merge(acc, bins[k]);
         c += cnt[k];
         la[k] = half_area(acc);
@@ -128,7 +128,7 @@ struct Bvh2 {
       }
       acc = empty_box();
       c = 0;
-      for (int k = NB - 1; k > 0; k--) {
+      for (int k = nb - 1; k > 0; k--) {
         acc = merge(acc, bins[k]);
         c += cnt[k];
         if (lc[k - 1] == 0 || c == 0) continue;
@@ -143,9 +143,9 @@ struct Bvh2 {
     int mid = begin + n / 2;
     if (best_ax >= 0) {
       float lo = cb.lo[best_ax], hi = cb.hi[best_ax];
-      float scale = NB / (hi - lo);
+      float scale = nb / (hi - lo);
       auto it = std::partition(order.begin() + begin, order.begin() + end, [&](uint32_t p) {
-        int b = std::min(NB - 1, std::max(0, (int)((cen(p, best_ax) - lo) * scale)));
+        int b = std::min(nb - 1, std::max(0, (int)((cen(p, best_ax) - lo) * scale)));
         return b <= best_bin;
       });
       mid = (int)(it - order.begin());
@@ -172,9 +172,9 @@ struct Bvh2 {
 // their own with a fine grid (random spheres on a ground sphere of radius
 // 1000: the root's step is 8, the spheres' diameter 0.4).
 // GB300, by area -> by cost: 488 spheres 8.6 -> 3.9 node fetches a ray,
-// 1920x1080 128 frames 155.8 -> 110 ms, one frame 2.03 -> 1.48 ms; 104 moving
+// 1920x1080 128 frames 155.8 -> 106 ms (28 refill lanes), one frame 2.03 -> 1.48 ms; 104 moving
 // ones 1.60 -> 1.26 ms; the textures scene 2.14 -> 2.02 ms; commit of the 488
-// spheres 0.35 -> 0.53 ms.
+// spheres within 0.1 ms of what it was.
 // A primitive test against a node step: 0.15 / 0.2 / 0.3 / 0.4 / 0.6 gave
 // 110.6 / 110.7 / 109.7 / 111.5 / 112.1 ms on the spheres.
 #ifndef PT_FIT_PRIM
@@ -211,31 +211,26 @@ struct Fit {
     if (leaf) *leaf = is_leaf;
     return is_leaf ? prims : node;
   }
-  // cost[k]: the subtree of c in at most k slots, k = 1..most
-  void share(int c, int most, float* cost) {
+  // cost[k]: the subtree of c in at most k slots, k = 1..the result, which is
+  // `most` or its primitives if they are fewer
+  int share(int c, int most, float* cost) {
     uint8_t* s = &split[9 * (size_t)c];
     cost[1] = slot(c);
     s[1] = 0;
-    if (most < 2) return;
-    for (int k = 2; k <= most; k++) {
-      cost[k] = cost[1];
-      s[k] = 0;
-    }
-    if (B[c].left < 0) return;
+    most = std::min(most, B[c].nprims);
+    if (most < 2) return 1;
     float l[9], r[9];
-    share(B[c].left, most - 1, l);
-    share(B[c].right, most - 1, r);
+    const int ml = share(B[c].left, most - 1, l), mr = share(B[c].right, most - 1, r);
     for (int k = 2; k <= most; k++) {
-      if (cost[k - 1] < cost[k]) {
-        cost[k] = cost[k - 1];
-        s[k] = s[k - 1];
-      }
-      for (int i = 1; i < k; i++)
+      cost[k] = cost[k - 1];
+      s[k] = s[k - 1];
+      for (int i = std::max(1, k - mr); i <= std::min(k - 1, ml); i++)
         if (l[i] + r[k - i] < cost[k]) {
           cost[k] = l[i] + r[k - i];
           s[k] = (uint8_t)(i | (k << 4));
         }
     }
+    return most;
   }
   // node x as a wide node: its children's cost, their shares left in `split`
   float open(int x) {
@@ -245,13 +240,13 @@ struct Fit {
       inv[a] = std::ldexp(1.0f, -ex);
     }
     float l[9], r[9];
-    share(B[x].left, width - 1, l);
-    share(B[x].right, width - 1, r);
+    const int most = std::min(width, B[x].nprims);
+    const int ml = share(B[x].left, most - 1, l), mr = share(B[x].right, most - 1, r);
     float best = FLT_MAX;
     uint8_t& s = split[9 * (size_t)x];
     s = 1 | (2 << 4);  // where no cost is a number
-    for (int k = 2; k <= width; k++)
-      for (int i = 1; i < k; i++)
+    for (int k = 2; k <= most; k++)
+      for (int i = std::max(1, k - mr); i <= std::min(k - 1, ml); i++)
         if (l[i] + r[k - i] < best) {
           best = l[i] + r[k - i];
           s = (uint8_t)(i | (k << 4));
