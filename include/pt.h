@@ -67,7 +67,8 @@ typedef struct pt_options {
                           paths per chunk rounded up to 64 Ki, at most 8 Mi) */
   int enable_counters; /* count BVH node fetches and primitive tests */
   int enable_timing;   /* per-stage device times (CUDA events in the graph) */
-  int bvh_builder;     /* 0 automatic, 1 host (binned SAH), 2 GPU (LBVH + treelets) */
+  int bvh_builder;     /* 0 automatic, 1 host (binned SAH), 2 GPU (clustering for
+                          triangles, LBVH + treelets for other scenes) */
   int bvh_width;       /* most children per BVH node, 2..8; 0 = 8 */
   int shade_order;     /* 0 automatic (material order when the scene uses
                           Oren-Nayar, Torrance-Sparrow or Ashikhmin-Shirley), 1 sorted,
@@ -101,8 +102,9 @@ typedef struct pt_stats {
   uint64_t iterations;     /* wavefront iterations of the last render, the pass over
                               each chunk's last paths included */
   uint64_t kernel_launches;/* kernels launched by the last render */
-  /* device time per stage (enable_timing): generate, trace, shade,
-     shadow trace, finish + queue advance */
+  /* device time per stage (enable_timing): generate, trace (consistent mode:
+     with the occlusion rays), shade, shadow trace, finish + queue advance + the
+     chunk's last paths */
   double stage_ms[5];
   uint64_t graph_launches; /* CUDA-graph launches of the last render */
   uint64_t guide_samples;  /* training samples of each Adam step after the last guided
@@ -281,7 +283,8 @@ PT_API int pt_set_camera(pt_context* ctx, const float lookfrom[3], const float l
 
 /* ---- build: BVH8 over all primitives (replaces Trbvh) --------------------
  * Automatic builder choice: the GPU builder (Morton codes, radix sort,
- * Karras radix tree, SAH treelet restructuring, 8-wide collapse) from 4096
+ * locally-ordered clustering for triangle meshes, a radix tree with SAH
+ * treelets for other scenes, 8-wide collapse) from 512 triangles or 4096 mixed
  * primitives up, the host binned-SAH builder below. */
 PT_API int pt_commit(pt_context* ctx);
 
