@@ -14,7 +14,7 @@
  *   while (a chunk is left)             conditional node, set on the device
  *     k_batch_begin                     load the chunk, reset the queues
  *     while (the chunk has many paths)  conditional node, set on the device
- *       generate, trace, shade, shadow trace, finish, advance
+ *       one iteration's kernels         (pt_kernels.cu)
  *     k_tail                            the last paths, each to its end
  *     k_accumulate_batch, k_batch_end
  *

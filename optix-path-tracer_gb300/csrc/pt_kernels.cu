@@ -18,8 +18,9 @@
  * the continuation before the occlusion test is known, so k_shade_c passes
  * the path on with its NEE term pending, and the next iteration traces both
  * rays in one launch (k_trace_t<BOTH>: extension rays, then occlusion rays,
- * which any hit before the light ends) and adds the term.  Trace warps take rays from a per-launch
- * counter (ray_next), so no warp sits idle while others still have rays.
+ * which any hit before the light ends) and adds the term.  Trace warps take
+ * rays from a per-launch counter (ray_next), so no warp sits idle while others
+ * still have rays.
  * Without lights (or a sampled environment) the shadow stages are not
  * launched.  The iterations of a chunk run in a conditional graph node that
  * k_advance ends; the last few paths go to the tail kernel (pt_tail.cu).
