@@ -321,6 +321,14 @@ PT_API int pt_resolve_display(pt_context* ctx, const float* accum_rgba, int widt
 
 PT_API int pt_get_stats(pt_context* ctx, pt_stats* out);
 
+/* Bound on the wavefront iterations of a chunk of frames, if lower than the
+ * automatic one (which a working render never reaches); 0: the automatic one.
+ * It exists to exercise PT_ETIMEOUT; a batch takes the lowest of its scenes'.
+ * A render that fails with PT_ETIMEOUT or PT_EQUEUE leaves a host accumulator
+ * as it was, and a device accumulator and the guide as after the last chunk of
+ * frames (with the guide: the last frame) that was complete. */
+PT_API int pt_set_iteration_limit(pt_context* ctx, uint64_t iterations);
+
 /* pt_render for callers that cannot allocate device memory while rendering
  * (a strict memory pool, or an application that allocates only at start-up).
  * No counterpart in the reference.  It calls no cudaMalloc/cudaFree: its

@@ -1258,6 +1258,11 @@ static cudaError_t capture_iterations(pt_context* ctx, int mode, bool counters, 
   return e;
 }
 
+// A chunk's iteration bound: the automatic one, or the caller's if that is lower.
+static unsigned long long iter_bound(const pt_context* ctx, unsigned long long automatic) {
+  return ctx->iter_limit ? std::min<unsigned long long>(ctx->iter_limit, automatic) : automatic;
+}
+
 // The host loop of a chunk: a graph of kItersPerGraph iterations and the tail
 // kernel, launched until the counters say that the chunk has drained.  Used
 // with per-stage timing (events cannot sit in a conditional body) and where
@@ -1270,7 +1275,8 @@ static cudaError_t capture_iterations(pt_context* ctx, int mode, bool counters, 
 // remain.
 static int host_loop(pt_context* ctx, const WaveCtl& ctl, bool timing, int iter_kernels) {
   cudaStream_t st = ctx->stream;
-  const unsigned long long max_iters = ctl.chunk_paths + (unsigned long long)ctl.max_depth + 16;
+  const unsigned long long max_iters =
+      iter_bound(ctx, ctl.chunk_paths + (unsigned long long)ctl.max_depth + 16);
   unsigned long long iters = 0;
   auto launch = [&](int slot) -> cudaError_t {
     cudaError_t e = cudaGraphLaunch(timing && slot ? ctx->graph2 : ctx->graph, st);
@@ -1325,8 +1331,8 @@ static int run_chunk(pt_context* ctx, const pt_render_params* p, int frame0, int
   cudaStream_t st = ctx->stream;
   WaveCtl ctl = chunk_ctl(ctx, p, frame0, frames);
   const unsigned long long slots = (unsigned long long)ctx->slots;
-  ctl.max_iter =
-      ((ctl.chunk_paths + slots - 1) / slots + 2) * (unsigned long long)(p->max_depth + 2) + 16;
+  ctl.max_iter = iter_bound(
+      ctx, ((ctl.chunk_paths + slots - 1) / slots + 2) * (unsigned long long)(p->max_depth + 2) + 16);
   const bool counters = ctx->opt.enable_counters != 0;
   const bool timing = ctx->opt.enable_timing != 0;
   const bool guide = p->guide != 0;
@@ -1388,8 +1394,11 @@ static cudaError_t queue_counters(pt_context* ctx) {
 }
 
 // After the render's stream is idle: the error flags and the statistics.
-static int render_done(pt_context* ctx, const pt_render_params* p) {
+// step0: the guide's Adam steps before the render; once a frame has failed, no
+// later one trained it (k_guide_adam).
+static int render_done(pt_context* ctx, const pt_render_params* p, int step0) {
   const WaveCounters& c = *ctx->h_ctr;
+  if (c.error) ctx->guide.step = step0 + (p->guide ? (int)c.chunks_done * ctx->guide.steps : 0);
   if (c.error & 1u) return fail(ctx, PT_EQUEUE, "traversal stack overflow");
   if (c.error) return fail(ctx, PT_ETIMEOUT, "wavefront did not drain");
   ctx->stats.ext_rays = c.ext_rays;
@@ -1444,9 +1453,9 @@ int pth::check_params(pt_context* ctx, const pt_render_params* p) {
 extern "C" {
 
 // Render into a device accumulator: float4 per pixel, or 4 doubles per
-// pixel when acc64.
-static int render_device(pt_context* ctx, const pt_render_params* p, void* d_acc,
-                         bool acc64 = false) {
+// pixel when acc64.  *step0: the guide's Adam steps before it.
+static int render_device(pt_context* ctx, const pt_render_params* p, void* d_acc, bool acc64,
+                         int* step0) {
   cudaStream_t st = ctx->stream;
   size_t WH = (size_t)p->width * p->height;
   const size_t results_cap = (size_t)1 << 27;  // 128 M paths = 2 GiB of results
@@ -1463,6 +1472,7 @@ static int render_device(pt_context* ctx, const pt_render_params* p, void* d_acc
     CK(ctx->guide.feat.ensure(3 * (size_t)ctx->slots));
     ctx->W.guide = ctx->guide.out.p;
   }
+  *step0 = ctx->guide.step;
   if (p->frame0 == 0) CK(cudaMemsetAsync(d_acc, 0, WH * (acc64 ? 32 : 16), st));
   for (int f = 0; f < p->spp; f += chunk) {
     int frames = std::min(chunk, p->spp - f);
@@ -1480,9 +1490,9 @@ static int render_device(pt_context* ctx, const pt_render_params* p, void* d_acc
       if (rc) return rc;
     }
     if (acc64)
-      pt::launch_accumulate64(ctx->d_results.p, (double*)d_acc, p->width, p->height, frames, st);
+      pt::launch_accumulate64(ctx->W, (double*)d_acc, p->width, p->height, frames, st);
     else
-      pt::launch_accumulate(ctx->d_results.p, (float4*)d_acc, p->width, p->height, frames, st);
+      pt::launch_accumulate(ctx->W, (float4*)d_acc, p->width, p->height, frames, st);
     ctx->stats.kernel_launches += 1;
   }
   CK(queue_counters(ctx));
@@ -1521,15 +1531,19 @@ PT_API int pt_render(pt_context* ctx, const pt_render_params* params, float* acc
       CK(cudaMemcpyAsync(d_acc, accum_rgba, WH * sizeof(float4), cudaMemcpyHostToDevice, st));
   }
   CK(cudaEventRecord(ctx->ev0, st));
-  rc = render_device(ctx, params, d_acc);
+  int step0 = 0;
+  rc = render_device(ctx, params, d_acc, false, &step0);
   if (rc) {
     cudaStreamSynchronize(st);  // queued work may still write the accumulator
     return rc;
   }
   CK(cudaEventRecord(ctx->ev1, st));
-  if (!dev) CK(cudaMemcpyAsync(accum_rgba, d_acc, WH * sizeof(float4), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  if ((rc = render_done(ctx, params)) != PT_OK) return rc;
+  if ((rc = render_done(ctx, params, step0)) != PT_OK) return rc;
+  if (!dev) {  // after a failed render the caller's array is as it was
+    CK(cudaMemcpyAsync(accum_rgba, d_acc, WH * sizeof(float4), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+  }
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   ctx->stats.render_ms = ms;
@@ -1561,15 +1575,19 @@ PT_API int pt_render_accum64(pt_context* ctx, const pt_render_params* params,
       CK(cudaMemcpyAsync(d_acc, accum_rgba, WH * 32, cudaMemcpyHostToDevice, st));
   }
   CK(cudaEventRecord(ctx->ev0, st));
-  rc = render_device(ctx, params, d_acc, true);
+  int step0 = 0;
+  rc = render_device(ctx, params, d_acc, true, &step0);
   if (rc) {
     cudaStreamSynchronize(st);  // queued work may still write the accumulator
     return rc;
   }
   CK(cudaEventRecord(ctx->ev1, st));
-  if (!dev) CK(cudaMemcpyAsync(accum_rgba, d_acc, WH * 32, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  if ((rc = render_done(ctx, params)) != PT_OK) return rc;
+  if ((rc = render_done(ctx, params, step0)) != PT_OK) return rc;
+  if (!dev) {  // after a failed render the caller's array is as it was
+    CK(cudaMemcpyAsync(accum_rgba, d_acc, WH * 32, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+  }
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   ctx->stats.render_ms = ms;
@@ -1610,10 +1628,14 @@ PT_API int pt_render_paths(pt_context* ctx, const pt_render_params* params, floa
     CK(ctx->d_tmp.ensure(3 * WH));
     d_out = ctx->d_tmp.p;
   }
-  pt::launch_paths_out(ctx->d_results.p, d_out, (uint32_t)WH, st);
-  if (!dev) CK(cudaMemcpyAsync(out_rgb, d_out, 3 * WH * sizeof(float), cudaMemcpyDeviceToHost, st));
+  pt::launch_paths_out(ctx->W, d_out, (uint32_t)WH, st);
   CK(cudaStreamSynchronize(st));
-  return render_done(ctx, &p);
+  if ((rc = render_done(ctx, &p, ctx->guide.step)) != PT_OK) return rc;
+  if (!dev) {
+    CK(cudaMemcpyAsync(out_rgb, d_out, 3 * WH * sizeof(float), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+  }
+  return PT_OK;
 }
 
 PT_API int pt_trace_first_hits(pt_context* ctx, int width, int height, int frame, uint32_t* prim,
@@ -1684,6 +1706,12 @@ PT_API int pt_resolve_display(pt_context* ctx, const float* accum_rgba, int widt
   pt::launch_resolve(d_acc, (uchar4*)ctx->d_tmpu.p, (int)WH, frame, st);
   CK(cudaMemcpyAsync(rgba8, ctx->d_tmpu.p, WH * 4, cudaMemcpyDefault, st));
   CK(cudaStreamSynchronize(st));
+  return PT_OK;
+}
+
+PT_API int pt_set_iteration_limit(pt_context* ctx, uint64_t iterations) {
+  if (!ctx) return PT_EINVAL;
+  ctx->iter_limit = iterations;
   return PT_OK;
 }
 
@@ -1795,7 +1823,8 @@ extern "C" PT_API int pt_render_noalloc(pt_context* ctx, const pt_render_params*
     int frames = std::min(chunk, p->spp - f);
     const WaveCtl ctl = chunk_ctl(ctx, p, p->frame0 + f, frames);
     pt::launch_chunk_begin(W, d_ctl, ctl, f == 0, st);
-    unsigned long long max_iters = ctl.chunk_paths + (unsigned long long)p->max_depth + 16;
+    const unsigned long long max_iters =
+        iter_bound(ctx, ctl.chunk_paths + (unsigned long long)p->max_depth + 16);
     unsigned long long iters = 0;
     while (true) {
       const int n = ctl.chunk_paths <= ctl.tail_max ? 0 : kItersPerGraph;
@@ -1815,7 +1844,7 @@ extern "C" PT_API int pt_render_noalloc(pt_context* ctx, const pt_render_params*
     }
     ctx->stats.paths += ctl.chunk_paths;
     ctx->stats.iterations += 1;
-    pt::launch_accumulate(W.results, acc, p->width, p->height, frames, st);
+    pt::launch_accumulate(W, acc, p->width, p->height, frames, st);
     ctx->stats.kernel_launches += 2;
   }
   ctx->stats.ext_rays = c.ext_rays;

@@ -500,10 +500,14 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
   size_t max_chunk = 0;
   BatchChunk cur{};
   int cur_depth = 1;
+  unsigned long long iter_limit = ~0ull;
+  for (const ScenePart& p : b->parts)
+    if (p.ctx->iter_limit) iter_limit = std::min<unsigned long long>(iter_limit, p.ctx->iter_limit);
   auto close = [&]() {
     if (!cur.paths) return;
     cur.seg_end = (uint32_t)segs.size();
-    cur.max_iter = ((cur.paths + slots - 1) / slots + 2) * (unsigned long long)(cur_depth + 2) + 16;
+    cur.max_iter = std::min(iter_limit, ((cur.paths + slots - 1) / slots + 2) *
+                                            (unsigned long long)(cur_depth + 2) + 16);
     max_chunk = std::max<size_t>(max_chunk, cur.paths);
     chunks.push_back(cur);
     cur = BatchChunk{};

@@ -174,6 +174,7 @@ struct pt_context {
   cudaGraphExec_t graph2 = nullptr;  // a second instance on its own timing events (timing)
   bool graph_loop = false;   // graph is the device loop (else iterations for the host loop)
   bool cond_ok = true;       // conditional graph nodes usable
+  uint64_t iter_limit = 0;   // pt_set_iteration_limit
   cudaEvent_t evc[2] = {nullptr, nullptr};  // the counters of a graph launch have arrived
   bool graph_counters = false;
   bool graph_timing = false;

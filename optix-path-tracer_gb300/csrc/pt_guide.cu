@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(128, 1) k_guide_grad(GuideTrainArgs A) {
 // padding entries (rows 41..47 of W5, columns past the bias column) stay 0.
 __global__ void k_guide_adam(GuideAdamArgs A) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= PTG_PARAMS) return;
+  if (p >= PTG_PARAMS || (A.error && *A.error)) return;
   int l = p / PTG_W_LAYER;
   int e = p - l * PTG_W_LAYER;
   int r = e / PTG_K, c = e % PTG_K;

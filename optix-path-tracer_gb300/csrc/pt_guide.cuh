@@ -114,6 +114,7 @@ struct GuideAdamArgs {
   float* grad_out;  // optional copy of the summed gradient
   float lr, b1, b2, eps, bc1, bc2;  // bc = 1 - beta^t
   int update;
+  const uint32_t* error;  // if not null: no step once this word is set
 };
 
 

@@ -167,6 +167,7 @@ int pth::guide_frame_train(pt_context* ctx) {
     d.eps = 1e-8f;
     d.bc1 = 1.f - powf(d.b1, (float)G.step);
     d.bc2 = 1.f - powf(d.b2, (float)G.step);
+    d.error = &ctx->W.ctr->error;  // a frame that failed trains nothing
     pt::launch_guide_adam(d, st);
   }
   GK(cudaGetLastError());

@@ -90,6 +90,7 @@ struct WaveCounters {
   uint32_t n_chunks;     /* chunks of the batch (set by the host) */
   uint32_t ray_next[2];  /* rays taken by trace warps this iteration (extension, shadow) */
   uint32_t guide_rows;   /* positions listed for guide inference this iteration */
+  uint32_t chunks_done;  /* chunks of this render that ended without an error */
   uint32_t drained;      /* iterations since the chunk's last path was generated, that one
                             included: every live path has bounced this often */
 };
@@ -297,12 +298,13 @@ void launch_env_cdf(const float4* env, int w, int h, float* marg, float* cond, d
                     uint16_t* cond_idx, int cond_bits, cudaStream_t st);
 /* Normals of 3 floats to 16-byte vectors. */
 void launch_pack_normals(const float* n3, size_t n, float4* n4, cudaStream_t st);
-void launch_accumulate(const float4* results, float4* acc, int w, int h, int frames,
-                       cudaStream_t st);
+/* The three below write nothing once W's error flags are set: the results of a
+ * chunk that failed are not complete. */
+void launch_accumulate(const WaveState& W, float4* acc, int w, int h, int frames, cudaStream_t st);
 /* acc: 4 doubles per pixel (16-byte aligned) */
-void launch_accumulate64(const float4* results, double* acc, int w, int h, int frames,
+void launch_accumulate64(const WaveState& W, double* acc, int w, int h, int frames,
                          cudaStream_t st);
-void launch_paths_out(const float4* results, float* out, uint32_t n, cudaStream_t st);
+void launch_paths_out(const WaveState& W, float* out, uint32_t n, cudaStream_t st);
 /* First hits of the camera rays of one frame. */
 void launch_first_hits(const DevScene& S, int w, int h, int frame, uint32_t* prim, uint32_t* mat,
                        float* t, int max_stack, uint32_t* err, const LaunchCfg& lc,

@@ -392,6 +392,7 @@ __global__ void k_chunk_begin(WaveState W, WaveCtl* ctl, WaveCtl v, int first) {
     c.node_fetches = o.node_fetches;
     c.prim_tests = o.prim_tests;
     c.iters_total = o.iters_total;
+    c.chunks_done = o.chunks_done + (o.error ? 0u : 1u);
   }
   *W.ctr = c;
   for (int k = 0; k < PT_SHADE_KEYS; k++) W.listed[k * PT_LISTED_STRIDE] = 0;
@@ -423,10 +424,10 @@ __global__ void k_batch_begin(WaveState W, WaveCtl* ctl, const BatchChunk* __res
 
 // acc[x, H-1-y] += (col, 1) in frame order for every pixel of every segment
 // of the chunk (the batch form of k_accumulate).
-__global__ void k_accumulate_batch(const float4* __restrict__ results, const WaveCtl* __restrict__ ctlp,
-                                   BatchRefs br) {
+__global__ void k_accumulate_batch(WaveState W, const WaveCtl* __restrict__ ctlp, BatchRefs br) {
   const WaveCtl ctl = *ctlp;
-  if (ctl.seg_end <= ctl.seg_begin) return;
+  const float4* __restrict__ results = W.results;
+  if (ctl.seg_end <= ctl.seg_begin || W.ctr->error) return;
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < ctl.pixels;
        g += gridDim.x * blockDim.x) {
     const BatchSeg& sg = br.segs[find_seg(br.segs, ctl.seg_begin, ctl.seg_end, g, true)];
@@ -494,8 +495,9 @@ __global__ void k_relocate_ids(uint32_t* leaf_of_id, uint4* tri_attr, size_t n, 
 }
 
 // acc[x, H-1-y] += (col, 1) in frame order (programs/raygen.cu:153-166)
-__global__ void k_accumulate(const float4* __restrict__ results, float4* acc, int width,
-                             int height, int frames) {
+__global__ void k_accumulate(const float4* __restrict__ results, const uint32_t* error, float4* acc,
+                             int width, int height, int frames) {
+  if (*error) return;
   uint32_t WH = (uint32_t)width * (uint32_t)height;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < WH; p += gridDim.x * blockDim.x) {
     uint32_t x = p % (uint32_t)width, y = p / (uint32_t)width;
@@ -515,8 +517,9 @@ __global__ void k_accumulate(const float4* __restrict__ results, float4* acc, in
 // The same accumulation into double sums (acc holds 4 doubles per pixel):
 // for renders beyond a few thousand frames, where float sums of per-frame
 // values lose the low bits of each new frame.
-__global__ void k_accumulate64(const float4* __restrict__ results, double2* acc, int width,
-                               int height, int frames) {
+__global__ void k_accumulate64(const float4* __restrict__ results, const uint32_t* error,
+                               double2* acc, int width, int height, int frames) {
+  if (*error) return;
   uint32_t WH = (uint32_t)width * (uint32_t)height;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < WH; p += gridDim.x * blockDim.x) {
     uint32_t x = p % (uint32_t)width, y = p / (uint32_t)width;
@@ -534,7 +537,9 @@ __global__ void k_accumulate64(const float4* __restrict__ results, double2* acc,
   }
 }
 
-__global__ void k_paths_out(const float4* __restrict__ results, float* out, uint32_t n) {
+__global__ void k_paths_out(const float4* __restrict__ results, const uint32_t* error, float* out,
+                            uint32_t n) {
+  if (*error) return;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     float4 r = results[p];
     out[3 * p] = r.x;
@@ -805,7 +810,7 @@ void launch_batch_begin(const WaveState& W, WaveCtl* ctl, const BatchChunk* chun
 
 void launch_batch_end(const WaveState& W, const WaveCtl* ctl, const BatchRefs& br,
                       bool use_cond, unsigned long long outer, cudaStream_t st) {
-  k_accumulate_batch<<<num_sms() * 8, 256, 0, st>>>(W.results, ctl, br);
+  k_accumulate_batch<<<num_sms() * 8, 256, 0, st>>>(W, ctl, br);
   k_batch_end<<<1, 1, 0, st>>>(W, use_cond ? 1 : 0, (cudaGraphConditionalHandle)outer);
 }
 
@@ -825,18 +830,18 @@ void launch_pack_normals(const float* n3, size_t n, float4* n4, cudaStream_t st)
   k_pack_normals<<<num_sms() * 4, 256, 0, st>>>(n3, n, n4);
 }
 
-void launch_accumulate(const float4* results, float4* acc, int w, int h, int frames,
-                       cudaStream_t st) {
-  k_accumulate<<<num_sms() * 8, 256, 0, st>>>(results, acc, w, h, frames);
+void launch_accumulate(const WaveState& W, float4* acc, int w, int h, int frames, cudaStream_t st) {
+  k_accumulate<<<num_sms() * 8, 256, 0, st>>>(W.results, &W.ctr->error, acc, w, h, frames);
 }
 
-void launch_accumulate64(const float4* results, double* acc, int w, int h, int frames,
+void launch_accumulate64(const WaveState& W, double* acc, int w, int h, int frames,
                          cudaStream_t st) {
-  k_accumulate64<<<num_sms() * 8, 256, 0, st>>>(results, (double2*)acc, w, h, frames);
+  k_accumulate64<<<num_sms() * 8, 256, 0, st>>>(W.results, &W.ctr->error, (double2*)acc, w, h,
+                                               frames);
 }
 
-void launch_paths_out(const float4* results, float* out, uint32_t n, cudaStream_t st) {
-  k_paths_out<<<num_sms() * 8, 256, 0, st>>>(results, out, n);
+void launch_paths_out(const WaveState& W, float* out, uint32_t n, cudaStream_t st) {
+  k_paths_out<<<num_sms() * 8, 256, 0, st>>>(W.results, &W.ctr->error, out, n);
 }
 
 void launch_env_cdf(const float4* env, int w, int h, float* marg, float* cond, double* rows,
