@@ -329,6 +329,13 @@ PT_API int pt_get_stats(pt_context* ctx, pt_stats* out);
  * frames (with the guide: the last frame) that was complete. */
 PT_API int pt_set_iteration_limit(pt_context* ctx, uint64_t iterations);
 
+/* Once at most this many paths of a chunk are left, the tail kernel traces each
+ * to its end; before, they take the wavefront's iterations.  PT_TAIL_AUTO (the
+ * default): by the scene; 0: never.  The image does not depend on it, so tests
+ * can send the same paths either way; a batch takes the lowest of its scenes'. */
+#define PT_TAIL_AUTO 0xffffffffu
+PT_API int pt_set_tail_limit(pt_context* ctx, uint32_t paths);
+
 /* pt_render for callers that cannot allocate device memory while rendering
  * (a strict memory pool, or an application that allocates only at start-up).
  * No counterpart in the reference.  It calls no cudaMalloc/cudaFree: its

@@ -1191,7 +1191,7 @@ static WaveCtl chunk_ctl(const pt_context* ctx, const pt_render_params* p, int f
   ctl.mode = p->mode;
   ctl.guide = p->guide;
   ctl.guide_depth = ctx->guide.max_bounces > 0 ? (uint32_t)ctx->guide.max_bounces : 0xffffffffu;
-  ctl.tail_max = pt::tail_paths(ctx->max_stack, ctx->lc);
+  ctl.tail_max = pt::tail_paths(ctx->max_stack, ctx->lc, ctx->tail_limit);
   ctl.chunk_paths = (unsigned long long)p->width * p->height * frames;
   fastdiv_magic((uint32_t)(p->width * p->height), &ctl.wh_m, &ctl.wh_l);
   fastdiv_magic((uint32_t)p->width, &ctl.w_m, &ctl.w_l);
@@ -1712,6 +1712,12 @@ PT_API int pt_resolve_display(pt_context* ctx, const float* accum_rgba, int widt
 PT_API int pt_set_iteration_limit(pt_context* ctx, uint64_t iterations) {
   if (!ctx) return PT_EINVAL;
   ctx->iter_limit = iterations;
+  return PT_OK;
+}
+
+PT_API int pt_set_tail_limit(pt_context* ctx, uint32_t paths) {
+  if (!ctx) return PT_EINVAL;
+  ctx->tail_limit = paths;
   return PT_OK;
 }
 

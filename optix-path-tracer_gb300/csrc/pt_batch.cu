@@ -568,7 +568,9 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
   WaveCtl hc;
   memset(&hc, 0, sizeof(hc));
   hc.mode = mode;
-  hc.tail_max = pt::tail_paths(b->max_stack, b->lc);
+  uint32_t tail_limit = PT_TAIL_AUTO;
+  for (const ScenePart& p : b->parts) tail_limit = std::min(tail_limit, p.ctx->tail_limit);
+  hc.tail_max = pt::tail_paths(b->max_stack, b->lc, tail_limit);
   BK(cudaMemcpyAsync(b->d_ctl.p, &hc, sizeof(hc), cudaMemcpyHostToDevice, st));
   BatchRefs br{b->d_scenes.p, b->d_segs.p, b->d_roots.p};
   if (timing && b->tev.empty()) {

@@ -175,6 +175,7 @@ struct pt_context {
   bool graph_loop = false;   // graph is the device loop (else iterations for the host loop)
   bool cond_ok = true;       // conditional graph nodes usable
   uint64_t iter_limit = 0;   // pt_set_iteration_limit
+  uint32_t tail_limit = PT_TAIL_AUTO;  // pt_set_tail_limit
   cudaEvent_t evc[2] = {nullptr, nullptr};  // the counters of a graph launch have arrived
   bool graph_counters = false;
   bool graph_timing = false;

@@ -241,10 +241,10 @@ static_assert(PT_SHADE_KEYS == 8, "PT_SLOT_U4 holds the lists");
 void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W,
                   const WaveCtl* ctl, int max_stack, const BatchRefs* br, const LaunchCfg& lc,
                   cudaStream_t st);
-/* WaveCtl.tail_max for a BVH of this stack depth and launch shape:
- * PT_TAIL_PATHS (PT_TAIL_PATHS_TEX where lc.tex), or 0 where the tail
- * kernel's stacks would not fit in shared memory. */
-uint32_t tail_paths(int max_stack, const LaunchCfg& lc);
+/* WaveCtl.tail_max for a BVH of this stack depth and launch shape: the limit
+ * (PT_TAIL_AUTO: PT_TAIL_PATHS, or PT_TAIL_PATHS_TEX where lc.tex), or 0 where
+ * the tail kernel's stacks would not fit in shared memory. */
+uint32_t tail_paths(int max_stack, const LaunchCfg& lc, uint32_t limit);
 /* Resident tail blocks per SM (pt_tail.cu). */
 int tail_blocks_per_sm(int max_stack);
 /* The chunk's last paths, each to its end, when at most tail_max are left

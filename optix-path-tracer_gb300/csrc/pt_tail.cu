@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "pt_bvh.cuh"
+#include "../../include/pt.h"
 #include "pt_internal.h"
 #include "pt_shade.cuh"
 #include "pt_wave.cuh"
@@ -300,8 +301,9 @@ int tail_occupancy(K k, int max_stack) {
 
 namespace pt {
 
-uint32_t tail_paths(int max_stack, const LaunchCfg& lc) {
+uint32_t tail_paths(int max_stack, const LaunchCfg& lc, uint32_t limit) {
   if (tail_smem(max_stack) > kMaxSmem) return 0u;
+  if (limit != PT_TAIL_AUTO) return limit;
   return lc.tex ? PT_TAIL_PATHS_TEX : PT_TAIL_PATHS;
 }
 
