@@ -228,6 +228,7 @@ struct Tree {
   float4* cost;             // 2 per node, of nodes that are clusters between merges: WideCost
   uint32_t* plan;           // per node: how it is cut into wide nodes (wide_cost); null: by area
   uint32_t root;
+  bool guard;               // encode_node_dev
 };
 
 // Cost of a subtree as at most i + 1 slots of a wide node, by dynamic
@@ -858,7 +859,7 @@ __device__ __forceinline__ void collapse_node(const Tree& T, const uint32_t* __r
     pb.hi[a] = parent.hi[a];
   }
   uint32_t words[20];
-  pt::encode_node_dev(pb, wc, nk, child_base, prim_base, words, T.plan != nullptr);
+  pt::encode_node_dev(pb, wc, nk, child_base, prim_base, words, T.guard);
   uint4* dst = out.nodes + 5 * (size_t)it.y;
   for (int w = 0; w < 5; w++)
     dst[w] = make_uint4(words[4 * w], words[4 * w + 1], words[4 * w + 2], words[4 * w + 3]);
@@ -955,14 +956,14 @@ namespace pt {
 // the collapse met an inconsistent tree and stopped before overrunning a
 // buffer; -depth: 1 bad count, 2 capacity, 4 leaf gather mismatch; 8: the
 // finished tree broke a structural rule; 16: incomplete or too deep).
-// triangles: every primitive is one; then the tree is clustered, else rebuilt
-// in treelets.  GB300, 2.1 M-triangle terrain: pt_commit 16.0 -> 4.3 ms (the
+// cluster: the tree is clustered, else rebuilt in treelets; guard: guarded
+// grids (encode_node_dev).  Triangle meshes take both.  GB300, 2.1 M-triangle terrain: pt_commit 16.0 -> 4.3 ms (the
 // treelet passes took 12.6), 64 frames at 1920x1080 76.9 -> 76.3 ms, a batch of
 // eight terrains 72.0 -> 71.1 ms.  Scenes with other shapes keep the treelet
 // tree and with it their images: see encode_node_dev on node boundaries.
 cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t n,
                            uint4* d_nodes, float4* d_rec_out, uint32_t* d_leaf_of_id,
-                           uint32_t* out_nodes, int* out_depth, int width, bool triangles,
+                           uint32_t* out_nodes, int* out_depth, int width, bool cluster, bool guard,
                            float cam_t0, float cam_t1, BuildArena* arena, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   if (width < 2 || width > 8) width = 8;
@@ -970,7 +971,7 @@ cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t
          *shi = nullptr, *cost = nullptr;
   uint32_t* plan = nullptr;
   uint32_t *keys = nullptr, *vals = nullptr, *keys2 = nullptr, *vals2 = nullptr, *left = nullptr,
-           *right = nullptr, *cluster = nullptr, *ends = nullptr, *counters = nullptr;
+           *right = nullptr, *entry = nullptr, *ends = nullptr, *counters = nullptr;
   uint32_t *pint = nullptr, *pleaf = nullptr, *flags = nullptr;
   unsigned int* cbox = nullptr;
   uint2 *qa = nullptr, *qb = nullptr;
@@ -1006,8 +1007,8 @@ cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t
       cv.take(&vals2, n);
       cv.take(&left, ni);
       cv.take(&right, ni);
-      if (triangles) {
-        cv.take(&cluster, n);
+      if (cluster) {
+        cv.take(&entry, n);
         cv.take(&ends, n);
         cv.take(&cost, 2 * (size_t)ni);
         cv.take(&plan, ni);
@@ -1052,12 +1053,13 @@ cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t
     T.parent_int = pint;
     T.parent_leaf = pleaf;
     T.flags = flags;
-    T.root = n == 1 ? (0u | LEAF_BIT) : (triangles ? n - 2 : 0u);
+    T.root = n == 1 ? (0u | LEAF_BIT) : (cluster ? n - 2 : 0u);
+    T.guard = guard;
     BV(cudaMemcpyAsync(counters, h_cnt, sizeof(h_cnt), cudaMemcpyHostToDevice, st));
-    k_gather_boxes<<<g, 256, 0, st>>>(lo, hi, vals2, n, slo, shi, cluster, qa, T.root);
-    if (n > 1 && triangles) {
+    k_gather_boxes<<<g, 256, 0, st>>>(lo, hi, vals2, n, slo, shi, entry, qa, T.root);
+    if (n > 1 && cluster) {
       BV(cudaMemsetAsync(ends, 0xff, (size_t)n * 4, st));
-      k_ploc<<<g, 256, 0, st>>>(T, keys2, n, cluster, ends, counters + 3, width);
+      k_ploc<<<g, 256, 0, st>>>(T, keys2, n, entry, ends, counters + 3, width);
     } else if (n > 1) {
       BV(cudaMemsetAsync(pint, 0xff, ni * 4, st));
       BV(cudaMemsetAsync(pleaf, 0xff, (size_t)n * 4, st));
@@ -1089,7 +1091,7 @@ cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t
     }
     depth = 0;
     while (depth < kLevels && h_cnt[4 + depth]) depth++;
-    if (triangles && n > 1 && !h_cnt[2] && h_cnt[3] != n - 1) h_cnt[2] = 16;
+    if (cluster && n > 1 && !h_cnt[2] && h_cnt[3] != n - 1) h_cnt[2] = 16;
     // structural check of the result (keys and vals are free by now)
     if (!h_cnt[2] && n > 0) {
       const uint32_t nn = h_cnt[0];

@@ -31,7 +31,7 @@
 namespace pt {
 cudaError_t build_bvh8_gpu(const float4* d_rec, const float4* d_xforms, uint32_t n,
                            uint4* d_nodes, float4* d_rec_out, uint32_t* d_leaf_of_id,
-                           uint32_t* out_nodes, int* out_depth, int width, bool triangles,
+                           uint32_t* out_nodes, int* out_depth, int width, bool cluster, bool guard,
                            float cam_t0, float cam_t1, BuildArena* arena, cudaStream_t st);
 }
 
@@ -846,6 +846,19 @@ static void prim_record(const HostPrim& p, uint32_t id, float4* out) {
 // for speed is no deeper than that, or than the one it replaces.
 constexpr int kShallow = 8;
 
+// A clustered tree deeper than this is odd: twice the levels of a full tree of
+// n leaves, and four.  Meshes of 5 K to 2 M triangles, regular and random, come
+// to 5..9 levels of 8 children (14..23 of 2); where cluster areas do not tell
+// pairs apart (thousands of coincident triangles, areas past the range of a
+// float) merging goes one pair at a time and chains: 65536 triangles, 33 levels
+// of 8 children and 205 of 2 (coincident), 155 of 8 (coordinates of 1e20), where
+// the treelet tree takes 15, 72 and 16.
+static int odd_depth(size_t n, int width) {
+  int levels = 0;
+  for (size_t k = 1; k < n; k *= (size_t)width) levels++;
+  return 2 * levels + 4;
+}
+
 // Whether the host builder chooses wide nodes by cost on guarded grids.  Not
 // where an edge of a rectangle or a box is one of the scene's bounds (a closed
 // room): such trees stay as their images have been (encode_node_dev).
@@ -911,11 +924,21 @@ int pth::build_bvh(pt_context* ctx, int width, DevBuf<uint4>& d_nodes, DevBuf<fl
     CK(d_leaf_of_id.ensure(n));
     uint32_t nodes = 0;
     int depth = 0;
-    CK(pt::build_bvh8_gpu(ctx->d_rec_in.p, ctx->d_xforms.p, (uint32_t)n, d_nodes.p,
-                          d_prims.p, d_leaf_of_id.p, &nodes, &depth, width,
-                          all_triangles(ctx),
-                          ctx->cam.time0, ctx->cam.time1, &ctx->build_arena, st));
+    const bool triangles = all_triangles(ctx);
+    auto gpu_tree = [&](bool cluster) {
+      return pt::build_bvh8_gpu(ctx->d_rec_in.p, ctx->d_xforms.p, (uint32_t)n, d_nodes.p,
+                                d_prims.p, d_leaf_of_id.p, &nodes, &depth, width, cluster,
+                                triangles, ctx->cam.time0, ctx->cam.time1, &ctx->build_arena, st);
+    };
+    CK(gpu_tree(triangles));
     retry = retry && (depth < 0 || depth > kShallow);
+    if (triangles && !retry && (depth < 0 || depth > odd_depth(n, width))) {
+      // the treelet tree if it is shallower: traversal stacks are as deep as the
+      // tree, and pt_commit refuses one that does not fit in shared memory
+      const int clustered = depth;
+      CK(gpu_tree(false));
+      if (clustered > 0 && (depth < 0 || depth >= clustered)) CK(gpu_tree(true));
+    }
     if (depth < 0 && !retry)
       return fail(ctx, PT_EINVAL,
                   "GPU BVH8 failed validation (check " + std::to_string(-depth) + ")");
