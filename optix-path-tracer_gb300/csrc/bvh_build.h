@@ -64,23 +64,37 @@ struct Bvh8Out {
 //
 // box_grid: the exponent of a node's step along one axis and the grid's
 // origin p, for the node's bounds [lo, hi].
+// 2^e, -126 <= e <= 127.
+PT_BVH_HD inline float exp2i(int e) {
+  const uint32_t u = (uint32_t)(e + 127) << 23;
+  float f;
+  memcpy(&f, &u, 4);
+  return f;
+}
+// floorf, without a call where the host has no instruction for it.
+PT_BVH_HD inline float round_down(float v) {
+  if (!(v > -8388608.0f && v < 8388608.0f)) return v;  // whole already, or not a number
+  const float t = (float)(int)v;
+  return t > v ? t - 1.0f : t;
+}
 PT_BVH_HD inline int box_grid(float lo, float hi, bool guard, float& p) {
   p = lo;
   const float ext = hi - lo;
   int ex = -126;
   if (ext > 0.f) {
-    int k;
-    frexpf(ext / 255.0f, &k);
-    ex = k;
-    while (ex > -126 && ldexpf(255.0f, ex - 1) >= ext) ex--;
-    while (ldexpf(255.0f, ex) < ext) ex++;
-    if (ex < -126) ex = -126;
+    const float q = ext / 255.0f;
+    uint32_t u;
+    memcpy(&u, &q, 4);
+    ex = (int)(u >> 23) - 126;  // q < 2^ex
+    if (ex > 121) ex = 121;     // 255 * 2^121 is past every float
+    while (ex > -126 && 255.0f * exp2i(ex - 1) >= ext) ex--;
+    while (255.0f * exp2i(ex) < ext) ex++;
   }
   if (guard) {  // the origin may round downward by more than a step
-    p = lo - ldexpf(1.0f, ex);
-    while (hi - p > ldexpf(254.0f, ex)) {
+    p = lo - exp2i(ex);
+    while (hi - p > 254.0f * exp2i(ex)) {
       ex++;
-      p = lo - ldexpf(1.0f, ex);
+      p = lo - exp2i(ex);
     }
   }
   return ex;
@@ -95,7 +109,7 @@ PT_BVH_HD inline void encode_node_dev(const Box& parent, const WideChild* ch, in
   for (int a = 0; a < 3; a++) {
     const int ex = box_grid(parent.lo[a], parent.hi[a], guard, p[a]);
     e[a] = (uint32_t)(ex + 127);
-    step[a] = ldexpf(1.0f, ex);
+    step[a] = exp2i(ex);
   }
   memcpy(&out[0], &p[0], 4);
   memcpy(&out[1], &p[1], 4);
@@ -125,10 +139,10 @@ PT_BVH_HD inline void encode_node_dev(const Box& parent, const WideChild* ch, in
     meta[i >> 2] |= m << (8 * (i & 3));
     for (int a = 0; a < 3; a++) {
       float lo = (c.box.lo[a] - p[a]) / step[a], hi = (c.box.hi[a] - p[a]) / step[a];
-      lo = guard ? floorf(lo - PT_BOX_SLACK) : floorf(lo) - 1.0f;
-      hi = guard ? ceilf(hi + PT_BOX_SLACK) : ceilf(hi) + 1.0f;
-      lo = fminf(fmaxf(lo, 0.0f), 255.0f);
-      hi = fminf(fmaxf(hi, 0.0f), 255.0f);
+      lo = guard ? round_down(lo - PT_BOX_SLACK) : round_down(lo) - 1.0f;
+      hi = guard ? -round_down(-(hi + PT_BOX_SLACK)) : 1.0f - round_down(-hi);
+      lo = lo > 0.0f ? (lo < 255.0f ? lo : 255.0f) : 0.0f;
+      hi = hi > 0.0f ? (hi < 255.0f ? hi : 255.0f) : 0.0f;
       qlo[a][i >> 2] = (qlo[a][i >> 2] & ~(0xffu << (8 * (i & 3)))) | ((uint32_t)lo << (8 * (i & 3)));
       qhi[a][i >> 2] |= (uint32_t)hi << (8 * (i & 3));
     }

@@ -17,148 +17,172 @@ namespace pt {
 
 namespace {
 
+// Four floats (x, y, z, unused): bounds are merged, binned and quantised a
+// vector at a time, in the scalar order of operations.
+typedef float f4 __attribute__((vector_size(16)));
+typedef int i4 __attribute__((vector_size(16)));
+
+struct VBox {
+  f4 lo, hi;
+};
 struct BNode {
-  Box box;
-  int left = -1, right = -1;  // internal children
-  int first = 0, count = 0;   // range in `order` (count: leaves only)
-  int nprims = 0;             // primitives in the subtree
+  VBox box;
+  int left, right;    // internal children; left -1: a leaf
+  int first, nprims;  // the subtree's primitives in `order`
 };
 
-inline Box merge(const Box& a, const Box& b) {
-  Box r;
-  for (int k = 0; k < 3; k++) {
-    r.lo[k] = std::min(a.lo[k], b.lo[k]);
-    r.hi[k] = std::max(a.hi[k], b.hi[k]);
-  }
-  return r;
+inline f4 splat(float v) { return f4{v, v, v, v}; }
+inline f4 vmin(f4 a, f4 b) { return b < a ? b : a; }
+inline f4 vmax(f4 a, f4 b) { return a < b ? b : a; }
+inline VBox merge(const VBox& a, const VBox& b) {
+  return {vmin(a.lo, b.lo), vmax(a.hi, b.hi)};
 }
-inline float half_area(const Box& a) {
-  float ex = a.hi[0] - a.lo[0], ey = a.hi[1] - a.lo[1], ez = a.hi[2] - a.lo[2];
-  if (ex < 0) return 0.f;
-  return ex * ey + ey * ez + ez * ex;
+inline float half_area(const VBox& a) {
+  const f4 e = a.hi - a.lo;
+  if (e[0] < 0) return 0.f;
+  return e[0] * e[1] + e[1] * e[2] + e[2] * e[0];
 }
-inline Box empty_box() {
+inline VBox empty_box() { return {splat(FLT_MAX), splat(-FLT_MAX)}; }
+inline Box to_box(const VBox& v) {
   Box b;
-  for (int k = 0; k < 3; k++) {
-    b.lo[k] = FLT_MAX;
-    b.hi[k] = -FLT_MAX;
+  for (int a = 0; a < 3; a++) {
+    b.lo[a] = v.lo[a];
+    b.hi[a] = v.hi[a];
   }
   return b;
 }
 
+// Binary tree by binned SAH.  One pass bins a node's primitives along all axes
+// and keeps their bins for the partition; the sweeps visit the bins in use (an
+// empty one repeats its neighbour's cost), of which a small node has few.
 struct Bvh2 {
-  const std::vector<Box>& boxes;
-  std::vector<float> cx, cy, cz;
+  static const int NB = 32;
+  std::vector<VBox> boxes;
+  std::vector<f4> cen;
+  std::vector<uint32_t> bin;  // per primitive: its bins in the node at hand, a byte an axis
+  std::vector<int> wrong;     // split: positions in the wrong part
   std::vector<uint32_t>& order;
   std::vector<BNode> nodes;
   const int leaf;  // most primitives of a leaf
   Bvh2(const std::vector<Box>& b, std::vector<uint32_t>& o, int most)
-      : boxes(b), order(o), leaf(most) {
-    size_t n = b.size();
-    cx.resize(n);
-    cy.resize(n);
-    cz.resize(n);
-    for (size_t i = 0; i < n; i++) {
-      cx[i] = 0.5f * (b[i].lo[0] + b[i].hi[0]);
-      cy[i] = 0.5f * (b[i].lo[1] + b[i].hi[1]);
-      cz[i] = 0.5f * (b[i].lo[2] + b[i].hi[2]);
+      : boxes(b.size()), cen(b.size()), bin(b.size()), wrong(2 * b.size() + 2), order(o), leaf(most) {
+    for (size_t i = 0; i < b.size(); i++) {
+      boxes[i] = {f4{b[i].lo[0], b[i].lo[1], b[i].lo[2], 0.f},
+                  f4{b[i].hi[0], b[i].hi[1], b[i].hi[2], 0.f}};
+      cen[i] = 0.5f * (boxes[i].lo + boxes[i].hi);
     }
+    nodes.reserve(2 * b.size());
+    build(0, (int)b.size(), bounds(0, (int)b.size()));
   }
-  float cen(uint32_t p, int ax) const { return ax == 0 ? cx[p] : (ax == 1 ? cy[p] : cz[p]); }
+  VBox bounds(int begin, int end) const {
+    VBox bb = empty_box();
+    for (int k = begin; k < end; k++) bb = merge(bb, boxes[order[k]]);
+    return bb;
+  }
 
-  int build(int begin, int end) {
-    int ni = (int)nodes.size();
-    nodes.emplace_back();
-    Box bb = empty_box(), cb = empty_box();
-    for (int k = begin; k < end; k++) {
-      uint32_t p = order[k];
-      bb = merge(bb, boxes[p]);
-      for (int a = 0; a < 3; a++) {
-        cb.lo[a] = std::min(cb.lo[a], cen(p, a));
-        cb.hi[a] = std::max(cb.hi[a], cen(p, a));
-      }
+  int build(int begin, int end, const VBox& bb) {
+    const int ni = (int)nodes.size();
+    const int n = end - begin;
+    nodes.push_back({bb, -1, -1, begin, n});
+    if (n <= leaf) return ni;
+    int mid = begin;
+    VBox lb, rb;
+    if (n > 3) {
+      mid = split(begin, end, lb, rb);
+    } else if (n == 3) {  // leaf 1: the pair with the smaller box
+      uint32_t* q = &order[begin];
+      const float a01 = half_area(merge(boxes[q[0]], boxes[q[1]]));
+      const float a02 = half_area(merge(boxes[q[0]], boxes[q[2]]));
+      const float a12 = half_area(merge(boxes[q[1]], boxes[q[2]]));
+      if (a12 < a01 && a12 <= a02) std::swap(q[0], q[2]);
+      else if (a02 < a01) std::swap(q[1], q[2]);
     }
-    int n = end - begin;
-    nodes[ni].box = bb;
-    nodes[ni].nprims = n;
-    nodes[ni].first = begin;
-    if (n <= leaf) {
-      nodes[ni].count = n;
-      return ni;
+    if (mid == begin) {  // no plane separates the centroids: in the middle, or a pair and one
+      mid = n > 3 ? begin + n / 2 : end - 1;
+      lb = bounds(begin, mid);
+      rb = bounds(mid, end);
     }
-    if (n <= 3) {  // leaf 1: the pair with the smaller box
-      if (n == 3) {
-        uint32_t* q = &order[begin];
-        const float a01 = half_area(merge(boxes[q[0]], boxes[q[1]]));
-        const float a02 = half_area(merge(boxes[q[0]], boxes[q[2]]));
-        const float a12 = half_area(merge(boxes[q[1]], boxes[q[2]]));
-        if (a12 < a01 && a12 <= a02) std::swap(q[0], q[2]);
-        else if (a02 < a01) std::swap(q[1], q[2]);
-      }
-      const int l = build(begin, end - 1), r = build(end - 1, end);
-      nodes[ni].left = l;
-      nodes[ni].right = r;
-      return ni;
-    }
-    const int NB = 32, nb = leaf == 1 ? std::min(NB, 2 * n) : NB;  // few for few
-    float best = FLT_MAX;
-    int best_ax = -1, best_bin = -1;
-    for (int ax = 0; ax < 3; ax++) {
-      float lo = cb.lo[ax], hi = cb.hi[ax];
-      if (!(hi - lo > 0.f)) continue;
-      Box bins[NB];
-      int cnt[NB] = {0};
-      for (int k = 0; k < nb; k++) bins[k] = empty_box();
-      float scale = nb / (hi - lo);
-      for (int k = begin; k < end; k++) {
-        uint32_t p = order[k];
-        int b = std::min(nb - 1, std::max(0, (int)((cen(p, ax) - lo) * scale)));
-        cnt[b]++;
-        bins[b] = merge(bins[b], boxes[p]);
-      }
-      float la[NB];
-      int lc[NB];
-      Box acc = empty_box();
-      int c = 0;
-      for (int k = 0; k < nb; k++) {
-        acc = merge(acc, bins[k]);
-        c += cnt[k];
-        la[k] = half_area(acc);
-        lc[k] = c;
-      }
-      acc = empty_box();
-      c = 0;
-      for (int k = nb - 1; k > 0; k--) {
-        acc = merge(acc, bins[k]);
-        c += cnt[k];
-        if (lc[k - 1] == 0 || c == 0) continue;
-        float cost = la[k - 1] * lc[k - 1] + half_area(acc) * c;
-        if (cost < best) {
-          best = cost;
-          best_ax = ax;
-          best_bin = k - 1;
-        }
-      }
-    }
-    int mid = begin + n / 2;
-    if (best_ax >= 0) {
-      float lo = cb.lo[best_ax], hi = cb.hi[best_ax];
-      float scale = nb / (hi - lo);
-      auto it = std::partition(order.begin() + begin, order.begin() + end, [&](uint32_t p) {
-        int b = std::min(nb - 1, std::max(0, (int)((cen(p, best_ax) - lo) * scale)));
-        return b <= best_bin;
-      });
-      mid = (int)(it - order.begin());
-      if (mid == begin || mid == end) mid = begin + n / 2;
-    } else {
-      // all centroids coincide: split by index
-      mid = begin + n / 2;
-    }
-    int l = build(begin, mid);
-    int r = build(mid, end);
+    const int l = build(begin, mid, lb), r = build(mid, end, rb);
     nodes[ni].left = l;
     nodes[ni].right = r;
     return ni;
+  }
+
+  // Partitions order[begin, end) at the cheapest plane between bins: the first
+  // of the second part and the parts' boxes (begin: there is no plane).
+  int split(int begin, int end, VBox& lb, VBox& rb) {
+    const int n = end - begin;
+    const int nb = leaf == 1 ? std::min((int)NB, 2 * n) : NB;  // few for few
+    VBox cb = empty_box();
+    for (int k = begin; k < end; k++) {
+      const f4 c = cen[order[k]];
+      cb.lo = vmin(cb.lo, c);
+      cb.hi = vmax(cb.hi, c);
+    }
+    const f4 ext = cb.hi - cb.lo, scale = splat((float)nb) / ext;
+    VBox bins[3][NB];
+    int cnt[3][NB];
+    for (int a = 0; a < 3; a++)
+      for (int q = 0; q < nb; q++) {
+        bins[a][q] = empty_box();
+        cnt[a][q] = 0;
+      }
+    const i4 zero = {0, 0, 0, 0}, top = {nb - 1, nb - 1, nb - 1, nb - 1};
+    for (int k = begin; k < end; k++) {
+      const uint32_t p = order[k];
+      i4 b = __builtin_convertvector((cen[p] - cb.lo) * scale, i4);
+      b = b < zero ? zero : b;
+      b = b > top ? top : b;
+      bin[p] = (uint32_t)b[0] | (uint32_t)b[1] << 8 | (uint32_t)b[2] << 16;
+      for (int a = 0; a < 3; a++) {
+        bins[a][b[a]] = merge(bins[a][b[a]], boxes[p]);
+        cnt[a][b[a]]++;
+      }
+    }
+    float best = FLT_MAX;
+    int best_ax = -1, best_bin = -1, best_n = 0;
+    for (int ax = 0; ax < 3; ax++) {
+      if (!(ext[ax] > 0.f)) continue;
+      int at[NB], lc[NB], m = 0, c = 0;  // the bins in use, primitives up to each
+      float la[NB];                      // and the area of their box
+      VBox acc = empty_box();
+      for (int q = 0; q < nb; q++) {
+        if (!cnt[ax][q]) continue;
+        acc = merge(acc, bins[ax][q]);
+        c += cnt[ax][q];
+        at[m] = q;
+        lc[m] = c;
+        la[m++] = half_area(acc);
+      }
+      acc = empty_box();
+      for (int k = m - 1; k > 0; k--) {
+        acc = merge(acc, bins[ax][at[k]]);
+        const float cost = la[k - 1] * lc[k - 1] + half_area(acc) * (n - lc[k - 1]);
+        if (cost < best) {
+          best = cost;
+          best_ax = ax;
+          best_bin = at[k];
+          best_n = lc[k - 1];
+        }
+      }
+    }
+    if (best_ax < 0) return begin;
+    lb = rb = empty_box();
+    for (int q = 0; q < nb; q++) (q < best_bin ? lb : rb) = merge(q < best_bin ? lb : rb, bins[best_ax][q]);
+    // what lies in the wrong part, from either end, changes places (std::partition's
+    // order, without a branch on each primitive)
+    const int mid = begin + best_n, shift = 8 * best_ax;
+    int *out = wrong.data(), *in = out + best_n + 1, no = 0, nin = 0;
+    for (int k = begin; k < mid; k++) {
+      out[no] = k;
+      no += (int)((bin[order[k]] >> shift) & 255u) >= best_bin;
+    }
+    for (int k = end - 1; k >= mid; k--) {
+      in[nin] = k;
+      nin += (int)((bin[order[k]] >> shift) & 255u) < best_bin;
+    }
+    for (int k = 0; k < no; k++) std::swap(order[out[k]], order[in[k]]);
+    return mid;
   }
 };
 
@@ -173,8 +197,7 @@ struct Bvh2 {
 // 1000: the root's step is 8, the spheres' diameter 0.4).
 // GB300, by area -> by cost: 488 spheres 8.6 -> 3.9 node fetches a ray,
 // 1920x1080 128 frames 155.8 -> 106 ms (28 refill lanes), one frame 2.03 -> 1.48 ms; 104 moving
-// ones 1.60 -> 1.26 ms; the textures scene 2.14 -> 2.02 ms; commit of the 488
-// spheres within 0.1 ms of what it was.
+// ones 1.60 -> 1.26 ms; the textures scene 2.14 -> 2.02 ms.
 // A primitive test against a node step: 0.15 / 0.2 / 0.3 / 0.4 / 0.6 gave
 // 110.6 / 110.7 / 109.7 / 111.5 / 112.1 ms on the spheres.
 #ifndef PT_FIT_PRIM
@@ -182,76 +205,119 @@ struct Bvh2 {
 #endif
 constexpr float kCostPrim = PT_FIT_PRIM;
 
+// Every node with all its descendants down to seven levels is a sub-problem, so
+// that is where the builder's time goes: loops of fixed length (a subtree of
+// fewer primitives than slots repeats its last cost), and the choices noted only
+// for the nodes that become wide nodes.  pt_commit on the GB300's host, ms, trees
+// by area with scalar loops / by cost with scalar loops / this: 488 spheres 0.31 /
+// 0.45 / 0.23, 1940 spheres 1.33 / 1.90 / 0.96, 2000 boxes 2.23 / 2.84 / 1.08.
 struct Fit {
   const std::vector<BNode>& B;
   const int width;
-  std::vector<float> inner;   // a node's cost below itself, as a wide node
+  std::vector<float> inner;   // a node's cost below itself, as a wide node (more than 3 primitives)
   std::vector<uint8_t> split; // per node under the current wide node: slots of its left child by
                               // its own slots (0: it takes one)
-  float p[3], step[3], inv[3];
+  f4 p, step, inv;            // the current wide node's grid
 
   Fit(const std::vector<BNode>& b, int w) : B(b), width(w), inner(w ? b.size() : 0, 0.f),
                                          split(9 * inner.size(), 0) {
-    for (size_t k = w ? b.size() : 0; k-- > 0;)  // children come after their parents
-      if (b[k].left >= 0) inner[k] = open((int)k);
+    for (size_t k = inner.size(); k-- > 1;)  // children come after their parents; the root is no child
+      if (b[k].nprims > 3) inner[k] = open<false>((int)k, nullptr);
   }
-  float area(int c) const {  // of its box in the current wide node's grid
-    float e[3];
+  void set_grid(const VBox& b) {
     for (int a = 0; a < 3; a++) {
-      const float lo = std::floor((B[c].box.lo[a] - p[a]) * inv[a] - PT_BOX_SLACK);
-      const float hi = std::ceil((B[c].box.hi[a] - p[a]) * inv[a] + PT_BOX_SLACK);
-      e[a] = (hi - lo) * step[a];
+      float o;
+      const int ex = box_grid(b.lo[a], b.hi[a], true, o);
+      p[a] = o;
+      step[a] = exp2i(ex);
+      inv[a] = exp2i(-ex);
     }
+  }
+  float area(int c) const {  // of its box in the current wide node's grid (at steps 0..255)
+    const VBox& b = B[c].box;
+    const f4 l = (b.lo - p) * inv - splat(PT_BOX_SLACK), h = (b.hi - p) * inv + splat(PT_BOX_SLACK);
+    const f4 top = splat(256.f), none = splat(0.f), hc = vmin(vmax(none, h), top);
+    const f4 lo = whole(vmin(vmax(none, l), top)), ht = whole(hc);
+    const f4 e = ((ht < hc ? ht + splat(1.f) : ht) - lo) * step;
     return e[0] * e[1] + e[1] * e[2] + e[2] * e[0];
   }
-  // as one child of the current wide node: a leaf, or a wide node of its own
-  float slot(int c, bool* leaf = nullptr) const {
-    const float a = area(c), node = a + inner[c], prims = kCostPrim * a * (float)B[c].nprims;
-    const bool is_leaf = B[c].left < 0 || (B[c].nprims <= 3 && prims <= node);
-    if (leaf) *leaf = is_leaf;
-    return is_leaf ? prims : node;
+  static f4 whole(f4 v) { return __builtin_convertvector(__builtin_convertvector(v, i4), f4); }
+  // as one child of the current wide node: a leaf (3 primitives cost less than
+  // one more node), or a wide node of its own
+  float slot(int c) const {
+    const float a = area(c);
+    return B[c].nprims <= 3 ? kCostPrim * a * (float)B[c].nprims : a + inner[c];
   }
-  // cost[k]: the subtree of c in at most k slots, k = 1..the result, which is
-  // `most` or its primitives if they are fewer
-  int share(int c, int most, float* cost) {
+  // cost[k]: the subtree of c in at most k slots of the current wide node, k =
+  // 1..M.  NOTE: with the choices.
+  template <int M, bool NOTE>
+  void share(int c, float* cost) {
+    const BNode& b = B[c];
     uint8_t* s = &split[9 * (size_t)c];
     cost[1] = slot(c);
-    s[1] = 0;
-    most = std::min(most, B[c].nprims);
-    if (most < 2) return 1;
-    float l[9], r[9];
-    const int ml = share(B[c].left, most - 1, l), mr = share(B[c].right, most - 1, r);
-    for (int k = 2; k <= most; k++) {
-      cost[k] = cost[k - 1];
-      s[k] = s[k - 1];
-      for (int i = std::max(1, k - mr); i <= std::min(k - 1, ml); i++)
-        if (l[i] + r[k - i] < cost[k]) {
-          cost[k] = l[i] + r[k - i];
-          s[k] = (uint8_t)(i | (k << 4));
-        }
+    if (NOTE) s[1] = 0;
+    if (M == 1) return;
+    if (b.nprims <= 2) {
+      const float two = b.nprims == 1 ? cost[1] : slot(b.left) + slot(b.right);
+      for (int k = 2; k <= M; k++) cost[k] = std::min(cost[1], two);
+      if (NOTE) {
+        for (int k = 2; k <= M; k++) s[k] = two < cost[1] ? 1 | (2 << 4) : 0;
+        if (b.nprims == 2) split[9 * (size_t)b.left + 1] = split[9 * (size_t)b.right + 1] = 0;
+      }
+      return;
     }
-    return most;
+    float l[9], r[9];
+    constexpr int N = M > 1 ? M - 1 : 1;
+    share<N, NOTE>(b.left, l);
+    share<N, NOTE>(b.right, r);
+    for (int k = 2; k <= M; k++) {
+      float best = cost[k - 1];
+      int at = NOTE ? s[k - 1] : 0;
+      for (int i = 1; i < k; i++) {
+        const float v = l[i] + r[k - i];
+        if (NOTE && v < best) at = i | (k << 4);
+        best = v < best ? v : best;
+      }
+      cost[k] = best;
+      if (NOTE) s[k] = (uint8_t)at;
+    }
   }
-  // node x as a wide node: its children's cost, their shares left in `split`
-  float open(int x) {
-    for (int a = 0; a < 3; a++) {
-      const int ex = box_grid(B[x].box.lo[a], B[x].box.hi[a], true, p[a]);
-      step[a] = std::ldexp(1.0f, ex);
-      inv[a] = std::ldexp(1.0f, -ex);
-    }
+  // the cost of node x's children where it is a wide node of at most M; NOTE:
+  // into kids
+  template <int M, bool NOTE>
+  float open_as(int x, std::vector<int>* kids) {
+    set_grid(B[x].box);
     float l[9], r[9];
-    const int most = std::min(width, B[x].nprims);
-    const int ml = share(B[x].left, most - 1, l), mr = share(B[x].right, most - 1, r);
+    share<M - 1, NOTE>(B[x].left, l);
+    share<M - 1, NOTE>(B[x].right, r);
     float best = FLT_MAX;
-    uint8_t& s = split[9 * (size_t)x];
-    s = 1 | (2 << 4);  // where no cost is a number
-    for (int k = 2; k <= most; k++)
-      for (int i = std::max(1, k - mr); i <= std::min(k - 1, ml); i++)
-        if (l[i] + r[k - i] < best) {
-          best = l[i] + r[k - i];
-          s = (uint8_t)(i | (k << 4));
+    int li = 1, ri = 1;  // where no cost is a number
+    for (int k = NOTE ? 2 : M; k <= M; k++)
+      for (int i = 1; i < k; i++) {
+        const float v = l[i] + r[k - i];
+        if (NOTE && v < best) {
+          li = i;
+          ri = k - i;
         }
+        best = v < best ? v : best;
+      }
+    if (NOTE) {
+      take(B[x].left, li, *kids);
+      take(B[x].right, ri, *kids);
+    }
     return best;
+  }
+  template <bool NOTE>
+  float open(int x, std::vector<int>* kids) {
+    switch (std::min(width, B[x].nprims)) {
+      case 2: return open_as<2, NOTE>(x, kids);
+      case 3: return open_as<3, NOTE>(x, kids);
+      case 4: return open_as<4, NOTE>(x, kids);
+      case 5: return open_as<5, NOTE>(x, kids);
+      case 6: return open_as<6, NOTE>(x, kids);
+      case 7: return open_as<7, NOTE>(x, kids);
+      default: return open_as<8, NOTE>(x, kids);
+    }
   }
   void take(int c, int k, std::vector<int>& kids) const {
     const uint8_t s = split[9 * (size_t)c + k];
@@ -261,13 +327,6 @@ struct Fit {
     }
     take(B[c].left, s & 15, kids);
     take(B[c].right, (s >> 4) - (s & 15), kids);
-  }
-  // the children of node x as a wide node
-  void children(int x, std::vector<int>& kids) {
-    open(x);
-    const uint8_t s = split[9 * (size_t)x];
-    take(B[x].left, s & 15, kids);
-    take(B[x].right, (s >> 4) - (s & 15), kids);
   }
 };
 
@@ -286,8 +345,6 @@ int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width, bool
   std::vector<uint32_t> order(n);
   for (size_t i = 0; i < n; i++) order[i] = (uint32_t)i;
   Bvh2 b2(boxes, order, fit ? 1 : 3);
-  b2.nodes.reserve(2 * n);
-  b2.build(0, (int)n);
   const std::vector<BNode>& B = b2.nodes;
   Fit cost(B, fit ? width : 0);
 
@@ -312,7 +369,7 @@ int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width, bool
     if (bn.left < 0) {
       kids.push_back(pd.bnode);  // single-leaf root
     } else if (fit) {
-      cost.children(pd.bnode, kids);
+      cost.open<true>(pd.bnode, &kids);  // the root has two primitives at least
     } else {
       kids.push_back(bn.left);
       kids.push_back(bn.right);
@@ -339,14 +396,12 @@ int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width, bool
     uint32_t child_base = (uint32_t)queue.size();
     uint32_t prim_base = (uint32_t)out.leaf_order.size();
     uint32_t off = 0;
-    Box parent = empty_box();
+    VBox parent = empty_box();
     for (int k = 0; k < nch; k++) {
       const BNode& c = B[kids[k]];
-      wc[k].box = c.box;
+      wc[k].box = to_box(c.box);
       parent = merge(parent, c.box);
-      bool leaf = c.nprims <= 3;
-      if (fit && c.left >= 0) cost.slot(kids[k], &leaf);
-      if (leaf) {
+      if (c.nprims <= 3) {
         wc[k].internal = false;
         wc[k].count = (uint32_t)c.nprims;
         wc[k].prim_off = off;
@@ -360,7 +415,7 @@ int build_bvh8_host(const std::vector<Box>& boxes, Bvh8Out& out, int width, bool
       }
     }
     out.nodes.resize(queue.size() * 20);
-    encode_node(parent, wc, nch, child_base, prim_base, &out.nodes[(size_t)self * 20], fit);
+    encode_node(to_box(parent), wc, nch, child_base, prim_base, &out.nodes[(size_t)self * 20], fit);
   }
   return 0;
 }

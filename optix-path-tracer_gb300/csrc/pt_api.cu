@@ -890,8 +890,8 @@ int pth::build_bvh(pt_context* ctx, int width, DevBuf<uint4>& d_nodes, DevBuf<fl
   size_t n = ctx->prims.size();
   int builder = ctx->opt.bvh_builder;
   // GB300, commit of a triangle mesh by the host / GPU builder, ms: 512
-  // triangles 0.53 / 0.53, 800 0.87 / 0.51, 3200 3.55 / 0.54, and the renders
-  // within 2 % (the host's trees by area: 800 0.5, 3200 2.3, renders +1..10 %).
+  // triangles 0.21 / 0.26, 800 0.36 / 0.33, 1568 0.72 / 0.35, 3200 1.50 / 0.45,
+  // and the renders within 2 %.
   // Other scenes' device trees are by Morton code and area, without guarded
   // grids; up to 4096 primitives the host's are worth their time.
   bool retry = false;  // the host builds it instead if the GPU's tree is deep or fails its check
