@@ -262,7 +262,6 @@ PT_API int pt_context_destroy(pt_context* ctx) {
   ctx->d_mats.release();
   ctx->d_lights.release();
   ctx->d_tri_attr.release();
-  ctx->d_normals.release();
   ctx->d_normals4.release();
   ctx->d_uvs.release();
   ctx->d_leaf_of_id.release();
@@ -273,12 +272,13 @@ PT_API int pt_context_destroy(pt_context* ctx) {
   ctx->d_env_marg.release();
   ctx->d_env_cond.release();
   ctx->d_env_rows.release();
-  ctx->d_env_pre.release();
+  ctx->d_table_tmp.release();
   ctx->d_env_valid.release();
   ctx->d_env_row.release();
   ctx->d_env_idx.release();
   ctx->d_slot_f4.release();
   ctx->d_slot_u4.release();
+  ctx->d_lists.release();
   ctx->d_ctr.release();
   ctx->d_ctl.release();
   ctx->d_results.release();
@@ -999,23 +999,29 @@ static cudaError_t upload_tables(pt_context* ctx, size_t* bytes) {
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_tex_data, ctx->tex_data, 1, st, bytes);
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_tex_list, ctx->tex_list, 1, st, bytes);
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_tri_attr, ctx->tri_attr, 1, st, bytes);
-  if (e == cudaSuccess) e = upload_or_zero(ctx->d_normals, ctx->normals, 3, st, bytes);
-  const size_t nv = std::max<size_t>(1, ctx->normals.size() / 3);
-  if (e == cudaSuccess) e = ctx->d_normals4.ensure(nv);
-  if (e == cudaSuccess) {
-    pt::launch_pack_normals(ctx->d_normals.p, nv, ctx->d_normals4.p, st);
-    e = cudaGetLastError();
+  const size_t nn = ctx->normals.size();
+  const bool env_tables =
+      ctx->miss.type == PT_MISS_HDR && ctx->miss.spherical && !ctx->env.empty();
+  const size_t texels = env_tables ? (size_t)ctx->miss.w * ctx->miss.h : 0;
+  if (e == cudaSuccess) e = ctx->d_table_tmp.ensure(std::max((nn + 1) / 2, texels));
+  if (e == cudaSuccess) e = ctx->d_normals4.ensure(std::max<size_t>(1, nn / 3));
+  if (e == cudaSuccess && nn > 0) {
+    float* n3 = (float*)ctx->d_table_tmp.p;
+    e = cudaMemcpyAsync(n3, ctx->normals.data(), nn * sizeof(float), cudaMemcpyHostToDevice, st);
+    *bytes += nn * sizeof(float);
+    if (e == cudaSuccess) {
+      pt::launch_pack_normals(n3, nn / 3, ctx->d_normals4.p, st);
+      e = cudaGetLastError();
+    }
   }
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_uvs, ctx->uvs, 2, st, bytes);
   if (e == cudaSuccess) e = upload_or_zero(ctx->d_env, ctx->env, 1, st, bytes);
   ctx->env_valid = 0;
-  if (e == cudaSuccess && ctx->miss.type == PT_MISS_HDR && ctx->miss.spherical &&
-      !ctx->env.empty()) {
+  if (e == cudaSuccess && env_tables) {
     const int w = ctx->miss.w, h = ctx->miss.h;
     e = ctx->d_env_marg.ensure((size_t)h + 1);
     if (e == cudaSuccess) e = ctx->d_env_cond.ensure((size_t)h * (w + 1));
     if (e == cudaSuccess) e = ctx->d_env_rows.ensure((size_t)h);
-    if (e == cudaSuccess) e = ctx->d_env_pre.ensure((size_t)w * h);
     if (e == cudaSuccess) e = ctx->d_env_valid.ensure(1);
     if (e == cudaSuccess) e = ctx->d_env_row.ensure((size_t)h);
     // search tables about as fine as the CDFs; their entries are 16-bit
@@ -1033,7 +1039,7 @@ static cudaError_t upload_tables(pt_context* ctx, size_t* bytes) {
     if (e == cudaSuccess) {
       uint16_t* mi = idx ? ctx->d_env_idx.p : nullptr;
       pt::launch_env_cdf(ctx->d_env.p, w, h, ctx->d_env_marg.p, ctx->d_env_cond.p,
-                         ctx->d_env_rows.p, ctx->d_env_pre.p, ctx->d_env_valid.p,
+                         ctx->d_env_rows.p, ctx->d_table_tmp.p, ctx->d_env_valid.p,
                          ctx->d_env_row.p, mi, mb, idx ? mi + nm : nullptr, cb, st);
       e = cudaGetLastError();
     }
@@ -1147,8 +1153,8 @@ void pth::carve_wave(WaveState& W, float4* f, uint4* u, size_t s) {
     b.st = u + k * s;
   }
   W.hit = f + 8 * s;
-  W.lists = (uint32_t*)(u + 3 * s);
-  W.listed = (uint32_t*)(u + 5 * s);
+  W.lists = nullptr;
+  W.listed = (uint32_t*)(u + PT_SLOT_U4 * s);
   W.sh.P = f + 9 * s;
   W.sh.N = f + 10 * s;
   W.sh.Wo = f + 11 * s;
@@ -1191,6 +1197,8 @@ static int ensure_wave(pt_context* ctx, size_t results_needed) {
     carve_wave(ctx->W, ctx->d_slot_f4.p, ctx->d_slot_u4.p, (size_t)slots);
     ctx->W.ctr = ctx->d_ctr.p;
   }
+  if (ctx->lc.sort) CK(ctx->d_lists.ensure(PT_SLOTS_LISTS(slots)));
+  ctx->W.lists = ctx->lc.sort ? ctx->d_lists.p : nullptr;  // the graph's W tells if it changed
   if (ctx->d_results.n < results_needed || !ctx->d_results.p) {
     drop_graphs(ctx);
     CK(ctx->d_results.ensure(results_needed));
@@ -1777,6 +1785,7 @@ constexpr size_t kNoAllocSlots = 16384;
 constexpr size_t kNoAllocMaxPixels = 262144;  // e.g. 512 x 512
 constexpr size_t kNoAllocBytes =
     kNoAllocSlots * PT_SLOT_F4 * sizeof(float4) + PT_SLOTS_U4(kNoAllocSlots) * sizeof(uint4) +
+    PT_SLOTS_LISTS(kNoAllocSlots) * sizeof(uint32_t) +
     256 /* WaveCounters */ + 256 /* WaveCtl */ + kNoAllocMaxPixels * sizeof(float4);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -1808,7 +1817,8 @@ static WaveState noalloc_wave(unsigned char* base, WaveCtl** ctl) {
   float4* f = (float4*)base;
   uint4* u = (uint4*)(f + PT_SLOT_F4 * s);
   carve_wave(W, f, u, s);
-  unsigned char* tail = (unsigned char*)(u + PT_SLOTS_U4(s));
+  W.lists = (uint32_t*)(u + PT_SLOTS_U4(s));
+  unsigned char* tail = (unsigned char*)(W.lists + PT_SLOTS_LISTS(s));
   W.ctr = (WaveCounters*)tail;
   *ctl = (WaveCtl*)(tail + 256);
   W.results = (float4*)(tail + 512);

@@ -93,6 +93,7 @@ struct pt_batch {
   WaveState W{};
   DevBuf<float4> slot_f4;
   DevBuf<uint4> slot_u4;
+  DevBuf<uint32_t> lists;
   DevBuf<WaveCounters> d_ctr;
   DevBuf<WaveCtl> d_ctl;
   DevBuf<float4> d_results;
@@ -282,6 +283,8 @@ static int ensure_wave(pt_batch* b, size_t results) {
     b->W.ctr = b->d_ctr.p;
     b->slots = (int)s;
   }
+  if (b->lc.sort) BK(b->lists.ensure(PT_SLOTS_LISTS(b->slots)));
+  b->W.lists = b->lc.sort ? b->lists.p : nullptr;  // GraphSig.W tells if it changed
   if (b->d_results.n < results || !b->d_results.p) {
     drop_graph(b);
     BK(b->d_results.ensure(results));
@@ -727,6 +730,7 @@ PT_API int pt_batch_destroy(pt_batch* b) {
   b->d_tune_acc.release();
   b->slot_f4.release();
   b->slot_u4.release();
+  b->lists.release();
   b->d_ctr.release();
   b->d_ctl.release();
   b->d_results.release();

@@ -137,15 +137,17 @@ struct pt_context {
   DevBuf<float4> d_tex_data;
   DevBuf<int> d_tex_list;
   DevBuf<uint4> d_tri_attr;
-  DevBuf<float> d_normals, d_uvs;
-  DevBuf<float4> d_normals4;  // d_normals, one 16-byte vector per vertex
+  DevBuf<float> d_uvs;
+  DevBuf<float4> d_normals4;  // one 16-byte vector per vertex
   DevBuf<uint32_t> d_leaf_of_id;
   DevBuf<float4> d_rec_in;  // primitive records in call order (GPU builder input)
   PinnedBuf<float4> h_rec;  // their host staging
   pt::BuildArena build_arena;  // GPU builder scratch, reused by every commit
   DevBuf<float> d_env_marg, d_env_cond;  // environment sampling CDFs
   DevBuf<double> d_env_rows;
-  DevBuf<double> d_env_pre;   // per texel: weights, then row prefix sums
+  // scratch of a commit's tables: the normals as the caller has them, then, per
+  // environment texel, weights and row prefix sums
+  DevBuf<double> d_table_tmp;
   DevBuf<int> d_env_valid;
   DevBuf<float2> d_env_row;
   DevBuf<uint16_t> d_env_idx; // search tables: marginal, then conditional
@@ -161,6 +163,7 @@ struct pt_context {
   WaveState W{};
   DevBuf<float4> d_slot_f4;   // PT_SLOT_F4 float4 arrays of `slots` entries
   DevBuf<uint4> d_slot_u4;    // PT_SLOT_U4 uint4 arrays
+  DevBuf<uint32_t> d_lists;   // PT_SLOTS_LISTS, where shading goes by lists
   DevBuf<WaveCounters> d_ctr;
   DevBuf<WaveCtl> d_ctl;
   DevBuf<float4> d_results;

@@ -197,7 +197,7 @@ struct GuideInferArgs;
 struct WaveState {
   PathBuf path[2];            /* ping-pong: path[parity] is current */
   float4* hit;                /* t, u, v, leaf index: by position in the current buffer */
-  uint32_t* lists;            /* sorted shading: `slots` positions for each shading key */
+  uint32_t* lists;            /* sorted shading: `slots` positions for each shading key; else null */
   uint32_t* listed;           /* positions on list k: listed[k * PT_LISTED_STRIDE] */
   ShadowBuf sh;               /* reference mode */
   NeeBuf nee[2];              /* consistent mode, beside path[]; shares sh's memory */
@@ -212,15 +212,17 @@ struct WaveState {
 };
 
 /* float4 arrays per slot: 2 x 4 (path buffers) + 1 (hit) + 7 (shadow), and
- * uint4 entries: 3 states and an entry in each of the 8 shading lists. */
+ * uint4 arrays: 3 states. */
 #define PT_SLOT_F4 16
-#define PT_SLOT_U4 5
+#define PT_SLOT_U4 3
 /* Shading key of a hit: 0 none, 1 + material type.  Each list's counter has a
  * cache line of its own, at the end of the uint4 block: the trace warps append
- * to all of them all the time. */
+ * to all of them all the time.  The lists are memory of their own (32 bytes a
+ * slot), which scenes shaded in path order do without. */
 #define PT_SHADE_KEYS (PT_NUM_MAT_TYPES + 1)
 #define PT_LISTED_STRIDE 32
 #define PT_SLOTS_U4(s) ((size_t)(s) * PT_SLOT_U4 + PT_SHADE_KEYS * PT_LISTED_STRIDE / 4)
+#define PT_SLOTS_LISTS(s) ((size_t)(s) * PT_SHADE_KEYS)
 
 /* Ray kinds of the trace kernels: closest hit of extension rays; closest
  * hit of a shadow ray (reference mode: the light must be the first thing
@@ -235,7 +237,6 @@ size_t trace_smem(int max_stack, int block);
 int one_blocks_per_sm();
 /* Resident trace blocks per SM (0 if the shape does not fit). */
 int trace_blocks_per_sm(int block, size_t smem);
-static_assert(PT_SHADE_KEYS == 8, "PT_SLOT_U4 holds the lists");
 /* One trace launch of `mode` (TRACE_EXT, TRACE_SHADOW or TRACE_BOTH)
  * over the wavefront's rays, with the launch shape of lc. */
 void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W,
