@@ -1120,6 +1120,7 @@ PT_API int pt_commit(pt_context* ctx) {
   if (pt::trace_smem(ctx->max_stack, PT_TRACE_BLOCK) > 200 * 1024)
     return fail(ctx, PT_EINVAL, "BVH too deep for the traversal stack");
   CK(pt::set_trace_smem());
+  CK(pt::set_tail_smem());
   ctx->lc = pt::default_launch(ctx->max_stack);
   ctx->lc.sort = ctx->opt.shade_order == 1 || (ctx->opt.shade_order == 0 && pth::sort_pays(ctx));
   ctx->lc.refetch = ctx->opt.refetch_lanes ? ctx->opt.refetch_lanes : pth::kAutoRefetch;

@@ -422,6 +422,7 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
   if (pt::trace_smem(b->max_stack, b->tune.trace_block) > 200 * 1024)
     return bfail(b, PT_EINVAL, "BVH too deep for the traversal stack at this trace block size");
   BK(pt::set_trace_smem());
+  BK(pt::set_tail_smem());
   LaunchCfg lc;
   lc.trace_block = b->tune.trace_block;
   lc.shade_block = b->tune.shade_block;
@@ -439,7 +440,7 @@ static int batch_render(pt_batch* b, const pt_batch_item* items, int n, float4* 
     lc.lights = lc.lights || p.ctx->scene.num_lights > 0;
     lc.env = lc.env || p.ctx->scene.env_valid;
   }
-  lc.tail_grid = pt::wave_grid(2, b->max_stack, PT_TAIL_BLOCK);
+  lc.tail_grid = pt::wave_grid(4, b->max_stack, PT_TAIL_BLOCK);
   lc.refetch = b->tune.refetch_lanes ? b->tune.refetch_lanes : kAutoRefetch;
   b->lc = lc;
   // accumulators: the items' device buffers, or device copies of host ones

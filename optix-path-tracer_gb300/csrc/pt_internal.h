@@ -246,8 +246,10 @@ void launch_trace(int mode, bool counters, const DevScene& S, const WaveState& W
  * (PT_TAIL_AUTO: PT_TAIL_PATHS, or PT_TAIL_PATHS_TEX where lc.tex), or 0 where
  * the tail kernel's stacks would not fit in shared memory. */
 uint32_t tail_paths(int max_stack, const LaunchCfg& lc, uint32_t limit);
-/* Resident tail blocks per SM (pt_tail.cu). */
-int tail_blocks_per_sm(int max_stack);
+/* Resident tail blocks per SM (pt_tail.cu); batch: of its batch form. */
+int tail_blocks_per_sm(int max_stack, bool batch);
+/* Dynamic shared memory limit of the tail kernels (once per device). */
+cudaError_t set_tail_smem();
 /* The chunk's last paths, each to its end, when at most tail_max are left
  * (pt_tail.cu); mark: the counters then say that the chunk has drained. */
 void launch_tail(const DevScene& S, const WaveState& W, const WaveCtl* ctl, int max_stack,
@@ -261,8 +263,8 @@ void launch_chunk_begin(const WaveState& W, WaveCtl* ctl, const WaveCtl& v, bool
  * sample there are no shadow rays to trace or finish). */
 int iteration_kernels(const LaunchCfg& lc, int mode, bool guide);
 /* Resident blocks per SM x SMs for a trace (kind 0), shade (kind 1) or tail
- * (kind 2, blocks of PT_TAIL_BLOCK) kernel of `block` threads, or for the
- * trace kernel of one-node trees (kind 3). */
+ * (kind 2, of a batch 4, blocks of PT_TAIL_BLOCK) kernel of `block` threads, or
+ * for the trace kernel of one-node trees (kind 3). */
 int wave_grid(int kind, int max_stack, int block);
 /* Raises the dynamic shared memory limit of the trace kernels to the
  * device maximum (once per device). */

@@ -686,8 +686,8 @@ int wave_grid(int kind, int max_stack, int block) {
   cudaError_t e = cudaSuccess;
   if (kind == 0)
     blocks = trace_blocks_per_sm(block, trace_smem(max_stack, block));
-  else if (kind == 2)
-    blocks = tail_blocks_per_sm(max_stack);
+  else if (kind == 2 || kind == 4)
+    blocks = tail_blocks_per_sm(max_stack, kind == 4);
   else if (kind == 3)
     blocks = one_blocks_per_sm();
   else

@@ -18,6 +18,7 @@
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include "pt_bvh.cuh"
 #include "../../include/pt.h"
 #include "pt_internal.h"
@@ -287,15 +288,17 @@ size_t tail_smem(int max_stack) {
 template <typename K>
 int tail_occupancy(K k, int max_stack) {
   int blocks = 0;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kMaxSmem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, PT_TAIL_BLOCK,
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, PT_TAIL_BLOCK,
                                                     tail_smem(max_stack)) != cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
   return blocks < 1 ? 1 : blocks;
 }
+
+// Once per device, with that device current.
+constexpr int kMaxDev = 64;
+std::atomic<bool> g_smem_set[kMaxDev];
 
 }  // namespace
 
@@ -307,13 +310,27 @@ uint32_t tail_paths(int max_stack, const LaunchCfg& lc, uint32_t limit) {
   return lc.tex ? PT_TAIL_PATHS_TEX : PT_TAIL_PATHS;
 }
 
-int tail_blocks_per_sm(int max_stack) {
+cudaError_t set_tail_smem() {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 0 && dev < kMaxDev && g_smem_set[dev]) return cudaSuccess;
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if ((e = cudaFuncSetAttribute(k_tail<0, false>, attr, kMaxSmem)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_tail<1, false>, attr, kMaxSmem)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_tail<0, true>, attr, kMaxSmem)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_tail<1, true>, attr, kMaxSmem)) != cudaSuccess) return e;
+  if (dev >= 0 && dev < kMaxDev) g_smem_set[dev] = true;
+  return cudaSuccess;
+}
+
+int tail_blocks_per_sm(int max_stack, bool batch) {
   if (tail_smem(max_stack) > kMaxSmem) return 1;
-  int a = tail_occupancy(k_tail<0, false>, max_stack), b = tail_occupancy(k_tail<1, false>, max_stack);
-  int c = tail_occupancy(k_tail<0, true>, max_stack), d = tail_occupancy(k_tail<1, true>, max_stack);
-  int m = a < b ? a : b;
-  if (c < m) m = c;
-  return d < m ? d : m;
+  const int a = batch ? tail_occupancy(k_tail<0, true>, max_stack)
+                      : tail_occupancy(k_tail<0, false>, max_stack);
+  const int b = batch ? tail_occupancy(k_tail<1, true>, max_stack)
+                      : tail_occupancy(k_tail<1, false>, max_stack);
+  return a < b ? a : b;
 }
 
 void launch_tail(const DevScene& S, const WaveState& W, const WaveCtl* ctl, int max_stack,
