@@ -161,8 +161,7 @@ struct pt_context {
   // ---- wavefront state
   int slots = 0;
   WaveState W{};
-  DevBuf<float4> d_slot_f4;   // PT_SLOT_F4 float4 arrays of `slots` entries
-  DevBuf<uint4> d_slot_u4;    // PT_SLOT_U4 uint4 arrays
+  DevBuf<float4> d_slots;     // PT_SLOT_F4 float4 arrays of `slots` entries, then the uint4 ones
   DevBuf<uint32_t> d_lists;   // PT_SLOTS_LISTS, where shading goes by lists
   DevBuf<WaveCounters> d_ctr;
   DevBuf<WaveCtl> d_ctl;
