@@ -6,6 +6,7 @@
 #define PT_CONTEXT_H
 
 #include <cuda_runtime.h>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -172,6 +173,7 @@ struct pt_context {
   DevBuf<uint32_t> d_tmpu;
   WaveCounters* h_ctr = nullptr;  // pinned, 2 (the counters after each of two graph launches)
   uint32_t* h_hits = nullptr;     // behind h_ctr: results of small first-hit queries
+  std::unique_ptr<unsigned char[]> keep;  // a small host array's values during a render
   cudaGraphExec_t graph = nullptr;
   cudaGraphExec_t graph2 = nullptr;  // a second instance on its own timing events (timing)
   bool graph_loop = false;   // graph is the device loop (else iterations for the host loop)

@@ -15,13 +15,17 @@ def fails(ptgb, g, call):
     assert e.value.code == -4                    # PT_ETIMEOUT
 
 
+# host arrays are copied to before or after the flags are known, by their size
+@pytest.mark.parametrize("w,h,spp", [(W, H, 2), (520, 520, 1)])
 @pytest.mark.parametrize("timing", [False, True])
 @pytest.mark.parametrize("mode", [0, 1])
-def test_accumulators_keep_their_values(ptgb_mod, mode, timing):
+def test_accumulators_keep_their_values(ptgb_mod, mode, timing, w, h, spp):
     torch = pytest.importorskip("torch")
-    g = ptgb_mod.GpuRenderer(ptgb_mod.material_zoo(W, H), path_slots=1000, timing=timing)
-    prm = ptgb_mod.GpuRenderer.params(W, H, 2, frame0=3, mode=mode)
-    start = np.random.default_rng(1).random((H, W, 4))
+    g = ptgb_mod.GpuRenderer(ptgb_mod.material_zoo(w, h), path_slots=1000, timing=timing)
+    assert g.lib.pt_set_tail_limit(g.ctx, 0) == 0
+    prm = ptgb_mod.GpuRenderer.params(w, h, spp, frame0=3, mode=mode)
+    first = ptgb_mod.GpuRenderer.params(w, h, spp, mode=mode)  # which starts from zeros
+    start = np.random.default_rng(1).random((h, w, 4))
     ref = g.render(prm, start.astype(np.float32))
     ref64 = g.render64(prm, start.copy())
     paths = g.render_paths(prm)
@@ -29,11 +33,12 @@ def test_accumulators_keep_their_values(ptgb_mod, mode, timing):
     for dtype, call in ((np.float32, g.render), (np.float64, g.render64)):
         acc = start.astype(dtype)
         fails(ptgb_mod, g, lambda: call(prm, acc))
+        fails(ptgb_mod, g, lambda: call(first, acc))
         assert np.array_equal(acc, start.astype(dtype))
         dev = torch.from_numpy(start.astype(dtype)).cuda()
         fails(ptgb_mod, g, lambda: call(prm, dev.data_ptr()))
         assert np.array_equal(dev.cpu().numpy(), start.astype(dtype))
-    out = np.full((H, W, 3), 5.0, np.float32)
+    out = np.full((h, w, 3), 5.0, np.float32)
     fails(ptgb_mod, g, lambda: g.render_paths(prm, out))
     assert np.all(out == 5.0)
     assert g.lib.pt_set_iteration_limit(g.ctx, 0) == 0
