@@ -109,8 +109,9 @@ struct Bvh2 {
   }
 
   // Partitions order[begin, end) at the cheapest plane between bins: the first
-  // of the second part and the parts' boxes (begin: there is no plane).
-  int split(int begin, int end, VBox& lb, VBox& rb) {
+  // of the second part and the parts' boxes (begin: there is no plane).  Not
+  // inlined: its bins would be part of every frame of build's recursion.
+  __attribute__((noinline)) int split(int begin, int end, VBox& lb, VBox& rb) {
     const int n = end - begin;
     const int nb = leaf == 1 ? std::min((int)NB, 2 * n) : NB;  // few for few
     VBox cb = empty_box();
