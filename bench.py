@@ -196,19 +196,19 @@ def issue_fraction(tr, ext, shadow, trace_ms, sm_mhz):
     """The trace kernels are bound by instruction issue, not by HBM (their
     BVH and records are served from L1/L2).  Warp instructions per ray come
     from a committed ncu capture (smsp__inst_executed.sum / rays of the
-    captured launches, extension and occlusion separately); the rate is the
+    captured launches, extension and occlusion rays together); the rate is the
     warp instructions this run's trace launches must have issued over their
     device time, against 152 SMs x 4 schedulers x one instruction per clock
     at the sampled SM clock (the maximum clock when no sample exists)."""
-    i_ext, i_occ = tr.get("warp_inst_per_ext_ray"), tr.get("warp_inst_per_shadow_ray")
-    if not i_ext or not i_occ:
+    per_ray = tr.get("warp_inst_per_ray")
+    if not per_ray:
         return None
     mhz = sm_mhz or 2070.0
-    inst = ext * i_ext + shadow * i_occ
+    inst = (ext + shadow) * per_ray
     achieved = inst / (trace_ms / 1e3)
     peak = SMS * SCHEDULERS_PER_SM * mhz * 1e6
     return {"warp_inst_per_s": achieved, "peak_warp_inst_per_s": peak, "frac": achieved / peak,
-            "sm_mhz": mhz, "warp_inst_per_ext_ray": i_ext, "warp_inst_per_shadow_ray": i_occ,
+            "sm_mhz": mhz, "warp_inst_per_ray": per_ray,
             "source": tr.get("_inst_source", "committed ncu capture (profiles/)")}
 
 
@@ -368,7 +368,8 @@ def run_ours(args, wl):
     b_ray = 32 + 16 + 80 * n_node + 48 * n_prim
     cnt.close()
     trace_ms = stage[1] + stage[3]
-    trace_launches = 2 * iters
+    # shadow rays of the reference mode have a launch of their own
+    trace_launches = (2 if kw.get("mode", 0) == 0 and scene.lights else 1) * iters
     achieved = (ext + shadow) * b_ray / (trace_ms / 1e3) / 1e9
     peak, peak_kind = peaks()
     traffic, issue = None, None
@@ -429,7 +430,7 @@ def run_ours(args, wl):
             "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": "k_trace + k_trace_shadow (BVH8 closest hit)",
+                         "kernel": "k_trace (BVH8: extension, shadow and occlusion rays)",
                          "peak_source": peak_kind,
                          "bytes_per_ray": b_ray, "nodes_per_ray": n_node,
                          "prims_per_ray": n_prim,
@@ -534,7 +535,7 @@ def run_batch(args):
     n_prim = cs["prim_tests"] / rays_c
     b_ray = 32 + 16 + 80 * n_node + 48 * n_prim
     trace_ms = sst["stage_ms"][1] + sst["stage_ms"][3]
-    trace_launches = 2 * sst["iterations"]
+    trace_launches = sst["iterations"]  # consistent mode: extension and occlusion rays together
     rays_t = sst["ext_rays"] + sst["shadow_rays"]
     achieved = rays_t * b_ray / (trace_ms / 1e3) / 1e9
     peak, peak_kind = peaks()
@@ -592,7 +593,7 @@ def run_batch(args):
             "graph_launches": graphs,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None,
-                         "kernel": "k_trace + k_trace_shadow (BVH8 closest hit, batch)",
+                         "kernel": "k_trace (BVH8: extension, shadow and occlusion rays, batch)",
                          "peak_source": peak_kind, "bytes_per_ray": b_ray,
                          "nodes_per_ray": n_node, "prims_per_ray": n_prim,
                          "avg_launch_ms": trace_ms / trace_launches,

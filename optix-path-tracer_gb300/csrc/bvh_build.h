@@ -46,24 +46,6 @@ struct Bvh8Out {
   int depth = 0;                     /* levels of wide nodes */
 };
 
-// Quantises the child boxes of one wide node into the 80-byte record: per
-// axis the smallest power-of-two step s with 255 s >= the parent's extent;
-// child bounds rounded outward to the step grid plus one step of slack for
-// the float decode in traversal.  Float-only, so host and device agree.
-// Without `guard` a bound on the node's own boundary has no step of slack (its
-// q is clamped to 0 or 255), and as a decoded plane is off by up to 2^-8 of a
-// step, a ray that hits the geometry within that distance of the boundary can
-// pass it by (on closed scenes of large walls about one path in 10^5).  With
-// `guard` the origin lies a step below the lower bound and a step is spare
-// above, so every bound has its slack, and PT_BOX_SLACK of a step is enough
-// of it: 64 times what the decode is off by.  (A whole step made the boxes of
-// a 2.1 M-triangle terrain larger by what costs 2.7 % of a render: 78.4
-// against 76.3 ms.)  Trees of scenes with shapes other than triangles are
-// built without it, as their images have been; the clustered trees of triangle
-// meshes with it.
-//
-// box_grid: the exponent of a node's step along one axis and the grid's
-// origin p, for the node's bounds [lo, hi].
 // 2^e, -126 <= e <= 127.
 PT_BVH_HD inline float exp2i(int e) {
   const uint32_t u = (uint32_t)(e + 127) << 23;
@@ -77,6 +59,8 @@ PT_BVH_HD inline float round_down(float v) {
   const float t = (float)(int)v;
   return t > v ? t - 1.0f : t;
 }
+// The exponent of a node's step along one axis and the grid's origin p, for the
+// node's bounds [lo, hi].
 PT_BVH_HD inline int box_grid(float lo, float hi, bool guard, float& p) {
   p = lo;
   const float ext = hi - lo;
@@ -100,6 +84,25 @@ PT_BVH_HD inline int box_grid(float lo, float hi, bool guard, float& p) {
   return ex;
 }
 
+// Quantises the child boxes of one wide node into the 80-byte record: per
+// axis the smallest power-of-two step s with 255 s >= the parent's extent;
+// child bounds rounded outward to the step grid plus one step of slack for
+// the float decode in traversal.  Float-only, so host and device agree.
+// Without `guard` a bound on the node's own boundary has no step of slack (its
+// q is clamped to 0 or 255), and as a decoded plane is off by up to 2^-8 of a
+// step, a ray that hits the geometry within that distance of the boundary can
+// pass it by (on closed scenes of large walls about one path in 10^5).  With
+// `guard` the origin lies a step below the lower bound and a step is spare
+// above, so every bound has its slack, and PT_BOX_SLACK of a step is enough
+// of it: 64 times what the decode is off by.  (Where half an ulp of the origin is
+// more than a step, the origin rounds back to the bound; there the padding of
+// the boxes themselves, 8 ulps, is the slack.)  (A whole step made the boxes of
+// a 2.1 M-triangle terrain larger by what costs 2.7 % of a render: 78.4
+// against 76.3 ms.)  Guarded are all trees of triangle meshes that the GPU
+// builds, and the host's trees except those of closed rooms of rectangles and
+// boxes, those of one node and the few by area (deep ones).  These, and the GPU's
+// trees of scenes with other shapes, are without the guard, as their images have
+// been.
 PT_BVH_HD inline void encode_node_dev(const Box& parent, const WideChild* ch, int nch,
                                       uint32_t child_base, uint32_t prim_base, uint32_t out[20],
                                       bool guard = false) {

@@ -34,12 +34,16 @@
 #ifndef PT_TAIL_PATHS
 #define PT_TAIL_PATHS 16384
 #endif
-/* The same where a material has an image or noise texture: a textured bounce
- * is several times as long a chain of dependent loads, which a warp of one
- * path cannot hide.  GB300, us per render with 2048 / 4096 / 8192 / 16384:
- * textures 61x82, 3 frames 799 / 822 / 910 / 1157 (consistent mode 416 / 431 /
- * 468 / 580), 321x243 one frame 1035 / 1053 / 1176 / 1356 and 33 frames 2112 /
- * 2121 / 2191 / 2287; 60x40 one frame 342 / 243 / 242 / 245. */
+/* The same where a material has a texture of any kind: a textured bounce can be
+ * several times as long a chain of dependent loads, which a warp of one path
+ * cannot hide.  GB300, us per render with 2048 / 4096 / 8192 / 16384: every
+ * texture callable in one scene, 61x82, 3 frames 799 / 822 / 910 / 1157
+ * (consistent mode 416 / 431 / 468 / 580), 321x243 one frame 1035 / 1053 / 1176 /
+ * 1356 and 33 frames 2112 / 2121 / 2191 / 2287; 60x40 one frame 342 / 243 / 242 /
+ * 245.  Where spheres have one simple texture the higher limit is the better one
+ * for a frame or a few: 148 spheres, 61x82, 3 frames, constant 371 / 363 / 323 /
+ * 271, checker 363 / 372 / 322 / 269, gradient 371 / 367 / 323 / 270, noise 389 /
+ * 389 / 329 / 274, image 369 / 367 / 324 / 272; 33 frames of 321x243 within 2 %. */
 #ifndef PT_TAIL_PATHS_TEX
 #define PT_TAIL_PATHS_TEX 4096
 #endif

@@ -220,7 +220,10 @@ __device__ __forceinline__ void shade_path(const DevScene& S0, const WaveState& 
 // the hit); the other variant carries no texture code at all.
 // LIGHTS: some scene has lights.  Then most warps queue shadow rays beside
 // paths, with one atomic for both; without any, the two appends stay apart
-// (random spheres, 128 frames at 1920x1080: 157.3 against 158.3 ms).
+// (random spheres, 128 frames at 1920x1080: 157.3 against 158.3 ms).  The code of
+// the shadow rays stays in that variant, although no path takes it: without it
+// the compiler's schedule is the slower one (the same render 107.7 -> 120.1 ms,
+// one frame 1505 -> 1525 us, at 80 bytes of spill stores in place of 72).
 template <bool BATCH, bool SORT, bool TEX, bool LIGHTS>
 __global__ void __launch_bounds__(PT_SHADE_BLOCK, PT_SHADE_MINBLOCKS) k_shade(DevScene S0, WaveState W,
                                                           const WaveCtl* __restrict__ ctlp,

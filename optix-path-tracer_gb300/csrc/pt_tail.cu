@@ -3,7 +3,7 @@
  * thread (one launch), in place of wavefront iterations over ever fewer
  * paths.
  *
- * A wavefront iteration costs six or seven dependent launches whatever its
+ * A wavefront iteration costs four to six dependent launches whatever its
  * size, and Russian roulette and glass leave a long, thin tail: a few hundred
  * paths live for dozens of bounces more.  Once the paths left (live ones and
  * ones not generated yet) are at most WaveCtl.tail_max, this kernel takes

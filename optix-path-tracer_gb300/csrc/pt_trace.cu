@@ -225,15 +225,14 @@ __device__ __forceinline__ void trace_rays(const DevScene& S, const WaveState& W
   };
   // loads ray i (< n) and sets up its traversal
   auto fetch = [&]() {
-    // a ray with a NaN in its origin or direction hits nothing (every
-    // primitive test fails or yields a NaN distance, which never wins the
-    // closest-hit minimum), and neither does any ray of an empty scene: both end
-    // here, without a traversal (a NaN ray would pass every box test)
+    // Some rays end here, without a traversal: one with a NaN in its origin or
+    // direction (every primitive test fails or yields a NaN distance, which never
+    // wins the closest-hit minimum, but it would pass every box test), any ray of
+    // an empty scene, and an extension ray whose path has ended (tmax 0: the path
+    // only waits for its NEE term).
     V3 d;
     float tmax;
     load_ray(d, tmax);
-    // here, and so does an extension ray whose path has ended (tmax 0: it only
-    // waits for its NEE term)
     if (nan_ray(o, d) || S.num_prims == 0 || (MODE == TRACE_EXT && tmax == 0.f)) {
       best_id = PT_NO_HIT;
       tbest = tmax;
