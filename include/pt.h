@@ -68,7 +68,8 @@ typedef struct pt_options {
   int enable_counters; /* count BVH node fetches and primitive tests */
   int enable_timing;   /* per-stage device times (CUDA events in the graph) */
   int bvh_builder;     /* 0 automatic, 1 host (binned SAH), 2 GPU (clustering for
-                          triangles, LBVH + treelets for other scenes) */
+                          triangles, LBVH + treelets for other scenes and where
+                          clustering gives an oddly deep tree) */
   int bvh_width;       /* most children per BVH node, 2..8; 0 = 8 */
   int shade_order;     /* 0 automatic (material order when the scene uses
                           Oren-Nayar, Torrance-Sparrow or Ashikhmin-Shirley), 1 sorted,
